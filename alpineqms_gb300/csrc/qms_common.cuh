@@ -26,7 +26,28 @@ struct QGrid {
     long long oY, oZ, oV, n;      // block offsets and n_dims
     long long nAx, nAy, nAz;      // block sizes
     double dx, dy, dz;
+    int okb;                      // k-planes that one CTA of a stencil kernel marches over
 };
+
+// Tiles of the stencil kernels (a CTA is 32 x 8 columns of nodes marching along k).
+#define OTX 32
+#define OTY 8
+// The k-planes a CTA marches over: 16, halved (down to 2) while the grid has fewer than 1216 tiles
+// (two waves of four CTAs on each of 152 SMs).  A march is a serial chain (one barrier and one tile
+// wait per plane, about 0.8 us each), so a grid of few tiles is bound by its length and not by
+// bandwidth; a shorter march re-reads more halo planes ((okb + 2) / okb of x), which such a grid
+// takes from L2.  Measured against marches of 16 planes, ms per run of steps: 48^3 ellipsoids
+// 277 -> 187, 96^3 370 -> 291, 64^3 in FP64 315 -> 188, 64x64x80 core 375 -> 297.  Line at 608
+// tiles: 128^3 360 instead of 333, steady state of 157x131x143 73.2 instead of 69.9; at least 4
+// planes: 48^3 198 instead of 187.
+#define QMS_CTA_TARGET 1216
+#define QMS_OKB_MIN 2
+static inline int qms_march_planes(int xs, int ys, int zs) {
+    const long long cols = (long long)((xs - 1 + OTX - 1) / OTX) * ((ys - 1 + OTY - 1) / OTY);
+    int okb = 16;
+    while (okb > QMS_OKB_MIN && cols * ((zs - 1 + okb - 1) / okb) < QMS_CTA_TARGET) okb /= 2;
+    return okb;
+}
 
 static inline QGrid qms_make_grid(int xs, int ys, int zs, double dx, double dy, double dz) {
     QGrid g;
@@ -41,6 +62,7 @@ static inline QGrid qms_make_grid(int xs, int ys, int zs, double dx, double dy, 
     g.oV = g.nAx + g.nAy + g.nAz;
     g.n = g.oV + g.Nn;
     g.dx = dx; g.dy = dy; g.dz = dz;
+    g.okb = qms_march_planes(xs, ys, zs);
     return g;
 }
 

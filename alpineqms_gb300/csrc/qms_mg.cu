@@ -491,11 +491,11 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
     __shared__ T red[KIND == 2 ? S::NQ : 1][OTY][OTX];
     constexpr bool STAGE = KIND != 0;
     const int tid = threadIdx.x + OTX * threadIdx.y;
-    const int i0 = blockIdx.x * OTX + 1, j0 = blockIdx.y * OTY + 1, k0 = blockIdx.z * OKB + 1;
+    const int i0 = blockIdx.x * OTX + 1, j0 = blockIdx.y * OTY + 1, k0 = blockIdx.z * g.okb + 1;
     const int li = threadIdx.x + 1, lj = threadIdx.y + 1;
     const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
     const bool inij = i <= g.Nx && j <= g.Ny;
-    const int kend = min(k0 + OKB - 1, g.Nz);
+    const int kend = min(k0 + g.okb - 1, g.Nz);
     const QPL L = qms_pl(g);
     const int cx = i0 - 1, cy = j0 - 2;
     auto issue_x = [&](int kk) {
@@ -847,10 +847,12 @@ int QmsMG<T>::build(const QGrid& g, const QCoef<T>& c, const QStepPar<T>& P, T v
         CKM(cudaMalloc(&L.dg, bytes)); CKM(cudaMalloc(&L.dinv, bytes)); CKM(cudaMalloc(&L.t, bytes));
         CKM(cudaMalloc(&L.mass, bytes));
         if (l > 0) { CKM(cudaMalloc(&L.x, bytes)); CKM(cudaMalloc(&L.b, bytes)); }
+        // the restriction leaves out aggregates of Dirichlet points alone: their right-hand side is zero
+        if (l == 1) CKM(cudaMemsetAsync(L.b, 0, bytes, st));
     }
     g0 = g; c0 = c; P0 = P; vshift0 = vshift;
     g0block = dim3(OTX, OTY, 1);
-    g0grid = dim3((g.Nx + OTX - 1) / OTX, (g.Ny + OTY - 1) / OTY, (g.Nz + OKB - 1) / OKB);
+    g0grid = qms_pl_tiles(g);
     const double ncut = vcut > 0.0 ? vcut : (sizeof(T) == 8 ? 1e-9 : 1e-5);
     mg_coarsen_fine<<<nblk(lv[1].total), 256, 0, st>>>(g, c, P, vshift, lv[0], lv[1], ncut);
     mg_mask_links<<<nblk(lv[1].total), 256, 0, st>>>(lv[1]);

@@ -30,7 +30,7 @@ enum QOpMode { QOP_APPLY = 0, QOP_SCALED = 1, QOP_RESID = 2 };
 
 // ---------------------------------------------------------------------------
 // A CTA of OTX x OTY threads owns a column
-// of nodes (i, j) and marches along k over OKB planes.  The six face/edge
+// of nodes (i, j) and marches along k over g.okb planes.  The six face/edge
 // coefficients of every node (1/mu_x, 1/mu_y, 1/mu_z, sigma_x, sigma_y,
 // sigma_z), which the rows of plane k need for planes k-1 and k and with a
 // -1 halo in i and j, are formed once per node into a two-plane shared-memory
@@ -53,7 +53,7 @@ qk_operator_t(QGrid g, QCoef<T> c, QStepPar<T> P, const T* __restrict__ x, const
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileCoef<T>& tc = *reinterpret_cast<TileCoef<T>*>(smem_raw);
     XTile<T>& xt = *reinterpret_cast<XTile<T>*>(smem_raw + sizeof(TileCoef<T>));
-    const int i0 = blockIdx.x * OTX + 1, j0 = blockIdx.y * OTY + 1, k0 = blockIdx.z * OKB + 1;
+    const int i0 = blockIdx.x * OTX + 1, j0 = blockIdx.y * OTY + 1, k0 = blockIdx.z * g.okb + 1;
     const int li = threadIdx.x + 1, lj = threadIdx.y + 1;   // position in the coefficient tile
     const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
     const bool inij = i <= g.Nx && j <= g.Ny;
@@ -92,7 +92,7 @@ qk_operator_t(QGrid g, QCoef<T> c, QStepPar<T> P, const T* __restrict__ x, const
     xsg.load(g, x, xt, k0 + 1);
     csg.load(c, tc, k0 - 1);
     csg.load(c, tc, k0);
-    const int kend = min(k0 + OKB - 1, g.Nz);
+    const int kend = min(k0 + g.okb - 1, g.Nz);
     // rows of this thread's four unknowns at plane k0 (32-bit: n_dims < 2^31 is checked at creation)
     int rX = (i - 1) + (j - 1) * sXj + (k0 - 1) * sXk;
     int rY = (int)g.oY + (i - 1) + (j - 1) * sYj + (k0 - 1) * sYk;
@@ -204,7 +204,7 @@ __global__ void qk_csr_spmv(long long n, const long long* __restrict__ ia, const
 static dim3 op_block() { return dim3(32, 4, 2); }
 static dim3 op_grid(const QGrid& g) { return dim3((g.Nx + 31) / 32, (g.Ny + 3) / 4, (g.Nz + 1) / 2); }
 static dim3 opt_block() { return dim3(OTX, OTY, 1); }
-static dim3 opt_grid(const QGrid& g) { return dim3((g.Nx + OTX - 1) / OTX, (g.Ny + OTY - 1) / OTY, (g.Nz + OKB - 1) / OKB); }
+static dim3 opt_grid(const QGrid& g) { return dim3((g.Nx + OTX - 1) / OTX, (g.Ny + OTY - 1) / OTY, (g.Nz + g.okb - 1) / g.okb); }
 
 // number of CTAs (= partial sums per reduction) of an operator launch
 long long qms_op_num_blocks(const QGrid& g) {

@@ -1,7 +1,7 @@
 // qms_pl.cu -- the inner solver's operator on the padded node layout (qms_tma.cuh), its
 // FP32 diagonal, and the maps between that layout and the reference's unknown order.
 //
-// qk_op_pl: one CTA of 32 x 8 threads owns a column of nodes and marches 16 k-planes.  Per
+// qk_op_pl: one CTA of 32 x 8 threads owns a column of nodes and marches g.okb k-planes.  Per
 // plane, one thread issues two cp.async.bulk.tensor copies: the four unknown blocks of
 // plane k+2 (+-1 halo, zero-filled outside the grid) into a four-slot ring, and the six node
 // coefficients of plane k+1 into a three-slot ring, each completing on its own mbarrier.
@@ -134,11 +134,11 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
     T* csm = xsm + 4 * TL::XSLOT;                             // [3 slots][6][PLCY][PLX]
     __shared__ __align__(8) uint64_t xbar[4], cbar[3];
     const int tid = threadIdx.x + OTX * threadIdx.y;
-    const int i0 = blockIdx.x * OTX + 1, j0 = blockIdx.y * OTY + 1, k0 = blockIdx.z * OKB + 1;
+    const int i0 = blockIdx.x * OTX + 1, j0 = blockIdx.y * OTY + 1, k0 = blockIdx.z * g.okb + 1;
     const int li = threadIdx.x + 1, lj = threadIdx.y + 1;
     const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
     const bool inij = i <= g.Nx && j <= g.Ny;
-    const int kend = min(k0 + OKB - 1, g.Nz);
+    const int kend = min(k0 + g.okb - 1, g.Nz);
     const QPL L = qms_pl(g);
     // tile origin in tensor coordinates: column i0 - 1 (a multiple of 32), row j0 - 2 (0-based)
     const int cx = i0 - 1, cy = j0 - 2;
@@ -878,8 +878,12 @@ static void op_pl_prepare() {
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
 
+dim3 qms_pl_tiles(const QGrid& g) {
+    return dim3((g.xs - 1 + OTX - 1) / OTX, (g.ys - 1 + OTY - 1) / OTY, (g.zs - 1 + g.okb - 1) / g.okb);
+}
 long long qms_op_pl_num_blocks(const QGrid& g) {
-    return (long long)((g.Nx + OTX - 1) / OTX) * ((g.Ny + OTY - 1) / OTY) * ((g.Nz + OKB - 1) / OKB);
+    const dim3 t = qms_pl_tiles(g);
+    return (long long)t.x * t.y * t.z;
 }
 
 template <typename T, int VM>
@@ -903,7 +907,7 @@ template <typename T>
 void qms_launch_op_pl(const QGrid& g, const QStepPar<T>& P, const CUtensorMap& xmap, const CUtensorMap& cmap, bool adv,
                       int mode, T* y, const T* w, double* partials, unsigned* err, cudaStream_t st) {
     op_pl_prepare<T>();
-    const dim3 bs(OTX, OTY, 1), gs((g.Nx + OTX - 1) / OTX, (g.Ny + OTY - 1) / OTY, (g.Nz + OKB - 1) / OKB);
+    const dim3 bs(OTX, OTY, 1), gs = qms_pl_tiles(g);
     const size_t shm = PLTiles<T>::SMEM;
     const int vm = qms_vel_mask(P, adv, sizeof(T) == 4);
     QMS_WITH_VM(vm, (op_pl_launch<T, VM>(gs, bs, shm, st, mode, g, P, xmap, cmap, y, w, partials, err)));
@@ -917,7 +921,7 @@ void qms_launch_resid_df(const QGrid& g, const QStepPar<qdf>& P, const CUtensorM
                          bool adv, float* r, const qdf* b, double* partials, unsigned* err, cudaStream_t st,
                          qdf* rfull) {
     op_pl_prepare<float>();
-    const dim3 bs(OTX, OTY, 1), gs((g.Nx + OTX - 1) / OTX, (g.Ny + OTY - 1) / OTY, (g.Nz + OKB - 1) / OKB);
+    const dim3 bs(OTX, OTY, 1), gs = qms_pl_tiles(g);
     const size_t shm = PLTiles<qdf>::SMEM;
     const int vm = qms_vel_mask(P, adv, true);
     QMS_WITH_VM(vm, (qk_op_pl<qdf, VM, QOPH_RESID, float, qdf><<<gs, bs, shm, st>>>(g, P, xmap, cmap, r, b, partials, err,

@@ -11,6 +11,10 @@
 #define QMS_NODE_BY 16
 dim3 qms_node_grid(const QGrid& g);
 dim3 qms_node_block();
+// CTAs of a kernel over tiles of the inner solver's vectors.  They cover the nodes 1..xs-1, 1..ys-1,
+// 1..zs-1: every row of a node beyond is a Dirichlet row, on which these vectors are zero and
+// stay so, and 256 cells then take 8 tiles of 32 columns instead of 9.
+dim3 qms_pl_tiles(const QGrid& g);
 long long qms_op_pl_num_blocks(const QGrid& g);
 
 // y = M x (mode QOPH_APPLY) or D^-1 M x (QOPH_SCALED) on padded vectors; x and the node

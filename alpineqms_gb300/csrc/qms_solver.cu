@@ -634,7 +634,8 @@ int QmsSolver::init(const qms_desc& d) {
     long long need = (npl + 255) / 256;
     if (need < vec_blocks) vec_blocks = need;
     nbop = qms_op_num_blocks(g);
-    long long npart = std::max(4 * nbop, (long long)(GM_MAXM + 1) * vec_blocks) + 64;
+    nbpl = qms_op_pl_num_blocks(g);
+    long long npart = std::max(4 * std::max(nbop, nbpl), (long long)(GM_MAXM + 1) * vec_blocks) + 64;
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     own_stream = true;
     const long long n = g.n, ncell = (long long)g.xs * g.ys * g.zs;
@@ -700,7 +701,7 @@ int QmsSolver::init(const qms_desc& d) {
         nwh = hx_need;
         for (int q = 0; q < nwh; q++) CK(pl_alloc((void**)&wh[q], 8));
         if (d.start_ls > 0) {
-            CK(cudaMalloc(&lsp, (size_t)QMS_LS_SUMS * nbop * 8));
+            CK(cudaMalloc(&lsp, (size_t)QMS_LS_SUMS * nbpl * 8));
             CK(cudaMalloc(&lsg, 8 * 8));
         }
         CK(pl_alloc((void**)&rfin, 8));
@@ -758,10 +759,10 @@ size_t qms_device_bytes_impl(const qms_desc& d) {
     if (ts == 4) tri += (size_t)6 * qms_pl16_pitch(g) * g.Ny * g.Nz * 2;       // bf16 node coefficients
     if (ts == 4) tri += qms_pl(g).n * (8 + 8 + 4 + 8 + 8) + 6 * qms_pl(g).comp * 8 + 5 * g.n * 8 + 2 * g.oV * 8 +
                         (hxn > 2 ? hxn - 2 : 0) * g.n * 8 + hxn * qms_pl(g).n * 8 +
-                        (lsn > 0 ? (QMS_LS_SUMS * (size_t)qms_op_num_blocks(g) + 8) * 8 : 0);
+                        (lsn > 0 ? (QMS_LS_SUMS * (size_t)qms_op_pl_num_blocks(g) + 8) * 8 : 0);
     size_t ncell = (size_t)g.xs * g.ys * g.zs;
     size_t smax = std::max({(size_t)g.ys * g.zs, (size_t)g.xs * g.zs, (size_t)g.xs * g.ys});
-    size_t nb = (size_t)qms_op_num_blocks(g);
+    size_t nb = (size_t)std::max(qms_op_num_blocks(g), qms_op_pl_num_blocks(g));
     return tri + ncell + sizeof(QMatTable<double>) + sizeof(QMatTable<float>) + 4 * g.n * 8 + 3 * ncell * 8 +
            6 * qms_pl(g).comp * 12 +
            3 * smax * 8 + (4 * nb + 64) * 8 + 2 * qms_pl(g).n * 4 + (QMS_NVEC + 1) * qms_pl(g).n * ts + 4096 +
@@ -1025,12 +1026,12 @@ int QmsSolver::inner_bicgstab(bool adv, bool transient, const double v[3], int& 
         nlaunch++;
         if (use_mg) precond<T>(p, dg, y, false, transient, false, &P, adv);
         op_pl<T>(adv, QOPH_SCALED, P, y, vv, rh, part);
-        finalize(FIN_BICG_ALPHA, 1, nbop);
+        finalize(FIN_BICG_ALPHA, 1, nbpl);
         qk_bicg_s<T><<<vb, 256, 0, st>>>(n, r, vv, s, S);
         nlaunch++;
         if (use_mg) precond<T>(s, dg, z, false, transient, false, &P, adv);
         op_pl<T>(adv, QOPH_SCALED, P, z, t, s, part);
-        finalize(FIN_BICG_OMEGA, 2, nbop);
+        finalize(FIN_BICG_OMEGA, 2, nbpl);
         qk_bicg_xr<T><<<vb, 256, 0, st>>>(n, y, z, s, t, rh, e, r, S, part);
         nlaunch++;
         finalize(FIN_BICG_RHO, 2, vec_blocks);
@@ -1118,7 +1119,7 @@ int QmsSolver::inner_pcg(bool transient, int& iters) {
     iters = 0;
     for (int it = 0; it < desc.max_inner; it++) {
         op_pl<T>(false, QOPH_APPLY, P, p, q, p, part);
-        finalize(FIN_CG_ALPHA, 1, nbop);
+        finalize(FIN_CG_ALPHA, 1, nbpl);
         qk_cg_update<T><<<vb, 256, 0, st>>>(n, p, q, S, e, r);
         nlaunch++;
         precond<T>(r, nullptr, z, true, transient, true);
@@ -1145,12 +1146,12 @@ int QmsSolver::residual_launch(bool adv, bool transient, const double v[3], bool
         // the step start (qk_step_start) formed this residual and its partials
         start_resid_ready = false;
         last_resid_df = true;
-        finalize(FIN_RESID, 4, nbop);
+        finalize(FIN_RESID, 4, nbpl);
         return 0;
     } else if (df_resid && anchor_ready && anchor_is_residual && !exact) {
         // x is the anchor state: the residual is the anchor's
         OpEv* ev = prof_begin(3, (double)g.n * 8 * 3);
-        qms_launch_anchor_resid(g, r0df, x, rpl, rfin, part, nbop, st);
+        qms_launch_anchor_resid(g, r0df, x, rpl, rfin, part, nbpl, st);
         nlaunch++;
         prof_end(ev);
         anchor_is_residual = false;
@@ -1159,7 +1160,7 @@ int QmsSolver::residual_launch(bool adv, bool transient, const double v[3], bool
         // double-float from the anchor: dx = x - x0 split into the padded layout (with the |x|^2
         // partials), then the TMA-staged stencil on the FP32 pipe
         OpEv* ev = prof_begin(3, (double)g.n * 8 * 4 + (double)g.xs * g.ys * g.zs);
-        qms_launch_delta_split(g, x, x0, xdf, part, nbop, st);
+        qms_launch_delta_split(g, x, x0, xdf, part, nbpl, st);
         qms_launch_resid_df(g, qms_step_par<qdf>(g, v[0], v[1], v[2], desc.dt, transient), xdfmap, cdfmap, adv, rpl,
                             r0df, part, status, st, rfin);
         nlaunch += 2;
@@ -1177,8 +1178,10 @@ int QmsSolver::residual_launch(bool adv, bool transient, const double v[3], bool
             anchor_ready = true;
         }
         last_resid_df = false;
+        finalize(FIN_RESID, 4, nbop);
+        return 0;
     }
-    finalize(FIN_RESID, 4, nbop);
+    finalize(FIN_RESID, 4, nbpl);
     return 0;
 }
 
@@ -1252,8 +1255,8 @@ int QmsSolver::step_graph(bool adv, const double v[3], const QStepStart& hs, boo
             capturing = true;
             cudaMemsetAsync(status, 0, 4, st);
             cudaMemcpyAsync(dptrs, hptrs, sizeof(QStepPtrs), cudaMemcpyHostToDevice, st);
-            qms_launch_step_start(g, rfin, b, bprev, dinvdf, r0df, hs, rpl, part, nbop, st, dptrs);
-            finalize(FIN_RESID, 4, nbop);
+            qms_launch_step_start(g, rfin, b, bprev, dinvdf, r0df, hs, rpl, part, nbpl, st, dptrs);
+            finalize(FIN_RESID, 4, nbpl);
             qk_cond_init<<<1, 32, 0, st>>>(S, desc.tol, hc);
             nlaunch += 2;
             ng.pro = nlaunch - n0;
@@ -1466,7 +1469,7 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
         } else {
             OpEv* ev = start_fused ? prof_begin(3, (double)g.n * (ls > 0 ? 8 * 11 + 8 * (ls - 1) + 8 * (2 * ls + 5) + 4
                                                                          : 8 * 11 + 8 * 2 * xo + 4)) : nullptr;
-            qms_launch_step_start(g, rfin, b, bprev, dinvdf, r0df, hs, start_fused ? rpl : nullptr, part, nbop, st);
+            qms_launch_step_start(g, rfin, b, bprev, dinvdf, r0df, hs, start_fused ? rpl : nullptr, part, nbpl, st);
             nlaunch++;
             prof_end(ev);
         }

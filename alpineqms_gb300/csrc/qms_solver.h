@@ -31,7 +31,8 @@ struct QmsSolver {
     bool fp64_inner = false;
     bool trace = false;         // QMS_TRACE set: one stderr line per refinement iteration
     size_t tsize = 4;
-    long long vec_blocks = 0, nbop = 0;
+    long long vec_blocks = 0;
+    long long nbop = 0, nbpl = 0;   // CTAs of the reference-layout operator / over the padded vectors' tiles
 
     uint8_t* ids = nullptr;
     QMatTable<double> htab64{};
@@ -88,7 +89,7 @@ struct QmsSolver {
     qdf* wh[4] = {nullptr, nullptr, nullptr, nullptr};
     int w_len = 0;
     int nwh = 0;                // w buffers allocated
-    double* lsp = nullptr;      // least-squares start: QMS_LS_SUMS x nbop partial sums
+    double* lsp = nullptr;      // least-squares start: QMS_LS_SUMS x nbpl partial sums
     double* lsg = nullptr;      // ... and its coefficients and diagnostics (8 doubles)
     bool last_chained = false;  // the last solve's anchor state was the solution before it
     int field_run = 0;          // consecutive solves (this one included) with the same B, G

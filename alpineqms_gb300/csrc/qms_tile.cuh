@@ -1,16 +1,13 @@
 // qms_tile.cuh -- shared-memory tiles of node coefficients for the stencil kernels.
 //
 // A CTA of OTX x OTY threads owns a column of nodes (i, j) and marches along k
-// over OKB planes.  The six face/edge coefficients of every node (1/mu_x,
+// over g.okb planes.  The six face/edge coefficients of every node (1/mu_x,
 // 1/mu_y, 1/mu_z, sigma_x, sigma_y, sigma_z) that the rows of plane k need
 // (planes k-1 and k, with a -1 halo in i and j) are staged in a three-plane ring.
 #pragma once
 #include "qms_common.cuh"
 #include "qms_tma.cuh"
 
-#define OTX 32
-#define OTY 8
-#define OKB 16
 // resident CTAs per SM the FP32 stencil kernels are compiled for (caps registers at 64)
 #ifndef QMS_STENCIL_MINB
 #define QMS_STENCIL_MINB 4

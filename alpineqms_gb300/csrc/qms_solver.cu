@@ -776,11 +776,7 @@ int QmsSolver::set_materials(const uint8_t* host_slots, const double* rows6, int
     CK(cudaSetDevice(dev));
     drop_graphs();
     gm_k_est = 0;
-    gm_k_seen = 0;
-    gm_lrate[0] = gm_lrate[1] = 0.0;
-    gm_k_fine = false;
-    gm_k_floor = 0;
-    gm_k_floor_age = 0;
+    gm_rate = 0.0;
     gm_ls_floor = 0;
     gm_ls_floor_age = 0;
     if (nmat < 0 || nmat > QMS_MAX_SLOTS - 1) { err = "nmat must be in 0..255"; return QMS_ERR_ARG; }
@@ -1056,24 +1052,26 @@ int QmsSolver::inner_bicgstab(bool adv, bool transient, const double v[3], int& 
 }
 
 
+// FGMRES in three parts: the start of a cycle, its steps j0 <= j < j1, and its end after k steps
+// (the small solve and the FP64 update of x)
 template <typename T>
-int QmsSolver::inner_gmres(bool adv, bool transient, const double v[3], int& iters, int fixed_k) {
+void QmsSolver::gmres_begin() {
+    qk_gm_reset<<<1, 128, 0, st>>>(std::min(desc.gmres_m, GM_MAXM), gm_scal);
+    resid_to_inner<T>((T*)gmV[0]);
+    nlaunch++;
+}
+
+template <typename T>
+void QmsSolver::gmres_steps(bool adv, bool transient, const double v[3], int j0, int j1) {
     const long long n = npl;
     const int m = std::min(desc.gmres_m, GM_MAXM);
-    const int kmax = fixed_k > 0 ? std::min(fixed_k, m) : m;
     const float* dg = transient ? dg_tr : dg_steady;
     QStepPar<T> P = qms_step_par<T>(g, v[0], v[1], v[2], desc.dt, transient);
     const int vb = (int)vec_blocks;
-    GmPtrs Vp{}, Zp{};
+    GmPtrs Vp{};
     for (int i = 0; i <= m; i++) Vp.p[i] = gmV[i];
-    for (int i = 0; i < m; i++) Zp.p[i] = use_mg ? gmZ[i] : gmV[i];
     T* w = (T*)vec[0];
-    qk_gm_reset<<<1, 128, 0, st>>>(m, gm_scal);
-    resid_to_inner<T>((T*)gmV[0]);
-    nlaunch++;
-    const double tol = desc.inner_rtol;
-    int k = 0;
-    for (int j = 0; j < kmax; j++) {
+    for (int j = j0; j < j1; j++) {
         T* vj = (T*)gmV[j];
         T* zj = use_mg ? (T*)gmZ[j] : vj;
         if (use_mg) precond<T>(vj, dg, zj, false, transient, false, &P, adv);
@@ -1084,16 +1082,124 @@ int QmsSolver::inner_gmres(bool adv, bool transient, const double v[3], int& ite
         qk_gm_givens<<<1, 512, 0, st>>>(part, vec_blocks, j, m, gm_H, gm_scal, status);
         qk_gm_scale<T><<<vb, 256, 0, st>>>(n, w, (T*)gmV[j + 1], gm_scal);
         nlaunch += 3;
-        k = j + 1;
-        if (fixed_k <= 0 && ((j + 1) % desc.check_every == 0 || j + 1 == m)) {
-            CK(cudaMemcpyAsync(hS, gm_scal, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
-            CK(cudaStreamSynchronize(st));
-            if (!(hS[1] > tol * hS[0])) break;       // also stops on a non-finite estimate
-        }
     }
+}
+
+template <typename T>
+void QmsSolver::gmres_end(int k) {
+    const int m = std::min(desc.gmres_m, GM_MAXM);
+    GmPtrs Zp{};
+    for (int i = 0; i < m; i++) Zp.p[i] = use_mg ? gmZ[i] : gmV[i];
     qk_gm_solve<<<1, 32, 0, st>>>(k, m, gm_H, gm_scal);
     nlaunch += 1 + gm_update<T>(k, st, g, m, Zp, gm_scal, S, x);
     last_gm_k = k;
+}
+
+int QmsSolver::gmres_estimate(double& est) {
+    CK(cudaMemcpyAsync(hS, gm_scal, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
+    est = hS[1] / hS[0];
+    return 0;
+}
+
+// a cycle of fixed_k steps, or (fixed_k = 0) with a look at the estimate every check_every steps
+template <typename T>
+int QmsSolver::inner_gmres(bool adv, bool transient, const double v[3], int& iters, int fixed_k) {
+    const int m = std::min(desc.gmres_m, GM_MAXM);
+    const int kmax = fixed_k > 0 ? std::min(fixed_k, m) : m;
+    gmres_begin<T>();
+    int k = 0;
+    while (k < kmax) {
+        const int j1 = fixed_k > 0 ? kmax : std::min(kmax, k + desc.check_every);
+        gmres_steps<T>(adv, transient, v, k, j1);
+        k = j1;
+        if (fixed_k <= 0) {
+            double est;
+            int rc = gmres_estimate(est);
+            if (rc) return rc;
+            if (!(est > desc.inner_rtol)) break;     // also stops on a non-finite estimate
+        }
+    }
+    gmres_end<T>(k);
+    iters = k;
+    CK(cudaGetLastError());
+    return 0;
+}
+
+// Steps j0 .. j0 + kSeg - 1 of a cycle as one CUDA graph, captured once per j0 for the operator of
+// this solve and replayed; the operator of another velocity starts over.
+int QmsSolver::gmres_segment(bool adv, bool transient, const double v[3], int j0, int j1, bool graph) {
+    auto steps = [&] {
+        if (fp64_inner) gmres_steps<double>(adv, transient, v, j0, j1);
+        else gmres_steps<float>(adv, transient, v, j0, j1);
+    };
+    if (!graph) {
+        steps();
+        CK(cudaGetLastError());
+        return 0;
+    }
+    if (!seg_valid || seg_tr != transient || seg_v[0] != v[0] || seg_v[1] != v[1] || seg_v[2] != v[2]) {
+        drop_segments();
+        seg_valid = true;
+        seg_tr = transient;
+        for (int q = 0; q < 3; q++) seg_v[q] = v[q];
+    }
+    const size_t at = (size_t)(j0 / kSeg);
+    if (segs.size() <= at) segs.resize(at + 1);
+    SegGraph& G = segs[at];
+    if (!G.exec) {
+        const long long n0 = nlaunch;
+        CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+        steps();
+        cudaGraph_t graph_ = nullptr;
+        cudaError_t e = cudaStreamEndCapture(st, &graph_);
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&G.exec, graph_, 0);
+        if (graph_) cudaGraphDestroy(graph_);
+        G.launches = nlaunch - n0;
+        nlaunch = n0;
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            G.exec = nullptr;
+            err = std::string("graph capture: ") + cudaGetErrorString(e);
+            return QMS_ERR_CUDA;
+        }
+    }
+    CK(cudaGraphLaunch(G.exec, st));
+    nlaunch += G.launches;
+    return 0;
+}
+
+// One cycle that ends when its residual estimate reaches `stop` (or the basis is full).  The first
+// look at the estimate comes shortly before the count that the last cycles' rate predicts, so a
+// cycle costs a host wait or two.  A cycle that ran on past the FP32 floor cost most: the counts
+// that were learned across solves before grew to 32 steps where 8 reach it (a plate in harmonic
+// motion: 84 steps per time step instead of 28).
+int QmsSolver::gmres_cycle(bool adv, bool transient, const double v[3], double stop, bool graph, int& iters) {
+    const int m = std::min(desc.gmres_m, GM_MAXM);
+    if (fp64_inner) gmres_begin<double>();
+    else gmres_begin<float>();
+    int k = 0, upto = kSeg;
+    if (gm_rate < 0.0) upto = (int)std::min((double)m, std::floor(std::log(stop) / gm_rate) - 1.0);
+    upto = std::min(m, std::max(kSeg, upto));
+    double est = 1.0;
+    for (;;) {
+        while (k < upto) {
+            const int j1 = std::min(m, k + kSeg);
+            int rc = gmres_segment(adv, transient, v, k, j1, graph);
+            if (rc) return rc;
+            k = j1;
+        }
+        int rc = gmres_estimate(est);
+        if (rc) return rc;
+        if (!(est > stop) || k >= m) break;          // also stops on a non-finite estimate
+        upto = std::min(m, k + kSeg);
+    }
+    if (est > 0.0 && est < 1.0) {
+        const double lr = std::log(est) / k;
+        gm_rate = gm_rate < 0.0 ? 0.5 * (gm_rate + lr) : lr;
+    }
+    if (fp64_inner) gmres_end<double>(k);
+    else gmres_end<float>(k);
     iters = k;
     CK(cudaGetLastError());
     return 0;
@@ -1214,14 +1320,15 @@ int QmsSolver::residual(bool adv, bool transient, const double v[3], bool exact)
     return read_scalars();
 }
 
-// One refinement iteration (FGMRES with k iterations, FP64 update, FP64 residual) as a
-// CUDA graph, captured once per (velocity, form, k) and replayed.
-void QmsSolver::drop_graphs() {
-    for (IrGraph& G : graphs) {
+void QmsSolver::drop_segments() {
+    for (SegGraph& G : segs)
         if (G.exec) cudaGraphExecDestroy(G.exec);
-        for (auto& e : G.ev) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
-    }
-    graphs.clear();
+    segs.clear();
+    seg_valid = false;
+}
+
+void QmsSolver::drop_graphs() {
+    drop_segments();
     for (StepGraph& G : sgraphs)
         if (G.exec) cudaGraphExecDestroy(G.exec);
     sgraphs.clear();
@@ -1323,77 +1430,6 @@ int QmsSolver::step_graph(bool adv, const double v[3], const QStepStart& hs, boo
     last_resid_df = true;
     start_resid_ready = false;
     return 0;
-}
-
-int QmsSolver::ir_iteration_graph(bool adv, bool transient, const double v[3], int k) {
-    const bool want_prof = prof && !graph_prof_broken;
-    IrGraph* G = nullptr;
-    for (IrGraph& e : graphs)
-        if (e.k == k && e.tr == transient && e.adv == adv && e.v[0] == v[0] && e.v[1] == v[1] && e.v[2] == v[2] &&
-            e.prof == want_prof) { G = &e; break; }
-    if (!G) {
-        // a small cache: the least recently used capture makes room
-        constexpr size_t kMaxGraphs = 6;
-        if (graphs.size() >= kMaxGraphs) {
-            size_t lru = 0;
-            for (size_t q = 1; q < graphs.size(); q++) if (graphs[q].used < graphs[lru].used) lru = q;
-            if (graphs[lru].exec) cudaGraphExecDestroy(graphs[lru].exec);
-            for (auto& e : graphs[lru].ev) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
-            graphs.erase(graphs.begin() + (long)lru);
-        }
-        graphs.emplace_back();
-        G = &graphs.back();
-        // with profiling on, the operator / V-cycle event records are captured as graph nodes
-        // on the entry's own event set and read back after every replay
-        const bool prof_was = prof;
-        const size_t ev_saved = evused;
-        prof = want_prof;
-        std::swap(evpool, G->ev);
-        evused = 0;
-        capturing = true;
-        const long long n0 = nlaunch;
-        cudaError_t e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-        int rc = 0;
-        if (e == cudaSuccess) {
-            int it = 0;
-            rc = fp64_inner ? inner_gmres<double>(adv, transient, v, it, k) : inner_gmres<float>(adv, transient, v, it, k);
-            if (rc == 0) rc = residual_launch(adv, transient, v);
-            G->resid_df = last_resid_df;
-        }
-        cudaGraph_t graph = nullptr;
-        if (e == cudaSuccess) e = cudaStreamEndCapture(st, &graph);
-        capturing = false;
-        G->evn = evused;
-        std::swap(evpool, G->ev);
-        evused = ev_saved;
-        prof = prof_was;
-        if (rc == 0 && e == cudaSuccess) e = cudaGraphInstantiate(&G->exec, graph, 0);
-        if (graph) cudaGraphDestroy(graph);
-        if (rc || e != cudaSuccess) {
-            if (G->exec) cudaGraphExecDestroy(G->exec);
-            for (auto& q : G->ev) { cudaEventDestroy(q.a); cudaEventDestroy(q.b); }
-            graphs.pop_back();
-            if (rc) return rc;
-            err = std::string("graph capture: ") + cudaGetErrorString(e);
-            return QMS_ERR_CUDA;
-        }
-        G->launches = nlaunch - n0;
-        nlaunch = n0;
-        G->k = k; G->tr = transient; G->adv = adv; G->prof = want_prof;
-        G->v[0] = v[0]; G->v[1] = v[1]; G->v[2] = v[2];
-    }
-    G->used = ++graph_clock;
-    CK(cudaGraphLaunch(G->exec, st));
-    nlaunch += G->launches;
-    // host state that the captured residual sets: a replay ends in the same kind of residual
-    last_resid_df = G->resid_df;
-    last_inner = 2;
-    last_gm_k = k;
-    int rc = read_scalars();                     // synchronises the stream
-    if (rc == 0 && G->prof && prof)
-        for (size_t q = 0; q < G->evn; q++)
-            if (!prof_accum(G->ev[q])) { graph_prof_broken = true; break; }
-    return rc;
 }
 
 int QmsSolver::solve(bool transient, const double v[3], const double B[3], const double G[9]) {
@@ -1504,10 +1540,9 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
     int outer = 0, stalled = 0;
     graph_resid_ready = false;
     const int gm_m = std::min(desc.gmres_m, GM_MAXM);
-    int graph_k_used = 0;                 // k of the graph replay that produced this residual (0: none)
-    int gm_k_last = 0;                    // FGMRES steps of the last cycle (graph or host-checked)
+    int graph_k_used = 0;                 // k of the step graph's cycle that produced this residual (0: none)
     int gm_cycles = 0;                    // FGMRES cycles run in this solve
-    int graph_cycles = 0;                 // ... of them replayed from graphs
+    int graph_cycles = 0;                 // ... of them in the step's graph
     double best_rn = INFINITY, best_rel = INFINITY;
     if (use_step_graph) {
         // the step (start and up to kStepGraphCycles cycles) in one graph; the loop below takes
@@ -1522,7 +1557,7 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
             outer = cyc;
             sref = hS[S_SREF];
             prev_rn = hS[S_PRN_LAST];
-            gm_k_last = graph_k_used = gm_k_est;
+            graph_k_used = gm_k_est;
             gm_cycles = graph_cycles = cyc;
             stats.inner_iterations = cyc * gm_k_est;
             last_inner = 2;
@@ -1551,20 +1586,9 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
         const bool v_ok = !(desc.tol_v > 0.0) || hS[S_XV] == 0.0 ||
                           std::sqrt(hS[S_RV]) <= desc.tol_v * std::sqrt(hS[S_XV]);
         if ((rel <= desc.tol && v_ok) || rn == 0.0) break;
-        // Per-step reduction rate of FGMRES from the true residuals around each cycle, kept
-        // apart for the first cycle of a solve and the later ones and smoothed in log space;
-        // it sizes the next replay.  A replay that gained less than a tenth per cycle while k
-        // can still grow is not a stall.
-        bool k_limited = false;
-        if (gm_k_last > 0 && std::isfinite(prev_rn) && prev_rn > 0 && rn > 0 && rn < prev_rn) {
-            const double rho = rn / prev_rn;
-            const double lr = std::log(rho) / gm_k_last;
-            double& slot = gm_lrate[gm_cycles == 1 ? 0 : 1];
-            slot = slot < 0.0 ? 0.5 * (slot + lr) : lr;
-            if (graph_k_used > 0 && graph_k_used < gm_m && rho > 0.1) k_limited = true;
-        }
+        // a cycle of the step's graph that gained less than a tenth with a short basis is not a stall
+        const bool k_limited = graph_k_used > 0 && graph_k_used < gm_m && rn < prev_rn && rn > 0.1 * prev_rn;
         graph_k_used = 0;
-        gm_k_last = 0;
         // Stall: near the round-off floor (within 1e3 of the tolerance) two iterations without
         // halving the residual end the solve; elsewhere only three iterations that gain less
         // than 10 % do, so that slowly but steadily converging solves continue.
@@ -1603,36 +1627,21 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
             last_inner = 1;
             rc = fp64_inner ? inner_bicgstab<double>(adv, transient, v, it)
                             : inner_bicgstab<float>(adv, transient, v, it);
-        } else if (desc.use_graphs && gm_k_est > 0) {
-            // replay a captured refinement iteration; its residual is read back with it.  The
-            // first two cycles of a solve run gm_k_est steps each (tuned across solves so that two
-            // cycles just suffice); a further cycle runs what the observed rate of the later cycles
-            // needs to reach tol / 2
-            it = gm_k_est;
-            const double lgoal = std::log(0.5 * desc.tol / rel);
-            if (graph_cycles >= 2 && gm_lrate[1] < -1e-3 && lgoal < 0.0)
-                it = std::min(gm_m, std::max(6, (int)std::ceil(lgoal / gm_lrate[1]) + 2));
-            // a start residual that the usual count would leave just above the tolerance: one
-            // cycle a few steps longer (at the observed first-cycle rate) instead of two cycles
-            if (graph_cycles == 0 && desc.gm_first_extend > 0 && gm_lrate[0] < -1e-3 && lgoal < 0.0) {
-                const int need = (int)std::ceil(lgoal / gm_lrate[0]) + 1;
-                if (need > it && need <= std::min(gm_m, gm_k_est + desc.gm_first_extend)) it = need;
-            }
-            graph_cycles++;
-            rc = ir_iteration_graph(adv, transient, v, it);
-            if (rc) return rc;
-            graph_k_used = it;
-            gm_k_last = it;
+        } else if (desc.use_graphs) {
+            // The reduction still wanted (to a tenth of the tolerance), in as few equal cycles as
+            // inner_rtol allows: the FP32 inner solve gains little past ~1e-3 per cycle (its own
+            // rounding), so deeper cycles buy less than a restart from a fresh residual
+            last_inner = 2;
+            const double want = std::log(std::min(0.1, 0.1 * desc.tol / rel));
+            const double most = std::log(std::min(0.5, std::max(desc.inner_rtol, 1e-12)));
+            const double stop = std::exp(want / std::max(1.0, std::ceil(want / most)));
+            // replayed from graphs once the operator is that of the solve before (a motion that
+            // changes it every step would pay a capture per step)
+            rc = gmres_cycle(adv, transient, v, stop, same_op && !prof, it);
             gm_cycles++;
-            stats.inner_iterations += it;
-            outer++;
-            graph_resid_ready = true;
-            continue;
         } else {
             last_inner = 2;
             rc = fp64_inner ? inner_gmres<double>(adv, transient, v, it, 0) : inner_gmres<float>(adv, transient, v, it, 0);
-            if (!rc) gm_k_seen = std::max(gm_k_seen, it);
-            gm_k_last = it;
             gm_cycles++;
         }
         if (rc) return rc;
@@ -1665,67 +1674,37 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
         rel = best_rel;
         if (rel <= desc.tol) stats.status &= ~(unsigned)QMS_ST_NO_CONVERGENCE;
     }
-    // replays start short: a solve that needs a third cycle costs less than two long cycles,
-    // and the count below adapts either way
-    if (!use_cg && desc.krylov == QMS_KRYLOV_GMRES && desc.use_graphs && gm_k_est == 0 && gm_k_seen > 0)
-        gm_k_est = std::min(std::min(desc.gmres_m, GM_MAXM), std::min(gm_k_seen + 1, 12));
-    // per-cycle count of the replays.  The FP32 inner solve gains little past ~1e-3 per cycle
-    // (its own rounding), so a longer cycle buys less than a restart from a fresh residual:
-    // probe downwards after every solve that two replays brought below tol / 3 (in steps of a
-    // fifth of k until the first solve that needed a third replay, one step after that), and
-    // step back up by two when a solve needed a third
-    // A count that needed a third replay is not probed again for 32 solves.  (One longer cycle
-    // in place of two does not pay: the FP32 inner solve stalls within a cycle, and a single
-    // cycle needed ~23 steps where two of 7 sufficed.)
-    // One-replay solves probe down to 5 steps; a probe below 6 that needed a second replay goes
-    // back to 6, which then holds for 32 solves.  (Letting any count step back up after a
-    // second replay raised it instead: one slow step pinned it at 7-8 for 32 solves.)
-    // After a least-squares start the start residual is within a few times the tolerance and
-    // falls from step to step, so the count follows the measured rate: a one-replay solve that
-    // ended below tol / 4 takes the count that this solve's reduction per FGMRES step says
-    // reaches tol / 4 from its start (at least one less); a solve that needed a second replay
-    // goes up by one (two after a third), and when its start had every direction it holds there
-    // for 4 solves (the first steps of a run know fewer directions and start worse: floors from
-    // them kept the count high well after).  Floors set by solves without this start do not apply.
+    // FGMRES steps per cycle of a step run as one graph (its count is fixed when it is captured).
+    // Solves with host-checked cycles leave the count that their reduction per FGMRES step says
+    // reaches tol / 4 from their start, at most 12.  In the graph the start residual is within a few times the tolerance
+    // and falls from step to step, so the count follows the measured rate: a one-cycle solve that
+    // ended below tol / 4 takes the count that this solve's reduction per FGMRES step says reaches
+    // tol / 4 from its start (at least one less); a solve that needed a second cycle goes up by one
+    // (two after a third), and when its start had every direction it holds there for 4 solves (the
+    // first steps of a run know fewer directions and start worse: floors from them kept the count
+    // high well after).
     // (On steps 6-25 of the moving plate at 256^3, targets of tol / 10, tol / 4 and tol / 2 ran
     // 26.80, 25.51 and 24.74 ms per step; tol / 2 left the field 1.05e-8 from the plain FP64
     // solve's at one step of 200, tol / 4 at most 9.8e-9.)
-    if (graph_cycles > 0 && rel <= desc.tol && ls > 0) {
+    auto count_for = [&](double steps) {
+        const double r0 = stats.initial_residual, goal = desc.tol / 4.0;
+        if (!(r0 > goal && rel > 0.0 && r0 > rel)) return 1;
+        return (int)std::ceil(std::log(r0 / goal) / (std::log(r0 / rel) / std::max(1.0, steps)));
+    };
+    if (graph_cycles > 0 && rel <= desc.tol) {
         if (gm_ls_floor > 0 && ++gm_ls_floor_age > 4) { gm_ls_floor = 0; gm_ls_floor_age = 0; }
-        if (graph_cycles >= 2) {
-            gm_k_est = std::min(gm_m, gm_k_est + (graph_cycles >= 3 ? 2 : 1));
+        if (gm_cycles >= 2) {
+            gm_k_est = std::min(gm_m, gm_k_est + (gm_cycles >= 3 ? 2 : 1));
             if (ls >= desc.start_ls) {
                 gm_ls_floor = gm_k_est;
                 gm_ls_floor_age = 0;
             }
         } else if (rel < desc.tol / 4.0) {
-            const double r0 = stats.initial_residual;
-            int need = 1;
-            if (r0 > desc.tol / 4.0 && rel > 0.0 && r0 > rel) {
-                const double rate = std::log(r0 / rel) / std::max(1, gm_k_est);
-                need = (int)std::ceil(std::log(r0 / (desc.tol / 4.0)) / rate);
-            }
-            gm_k_est = std::max(std::max(1, gm_ls_floor), std::min(gm_k_est - 1, need));
+            gm_k_est = std::max(std::max(1, gm_ls_floor), std::min(gm_k_est - 1, count_for(gm_k_est)));
         }
-    } else if (graph_cycles > 0 && rel <= desc.tol) {
-        if (gm_k_floor > 0 && ++gm_k_floor_age >= 32) { gm_k_floor--; gm_k_floor_age = 0; }
-        if (graph_cycles >= 3) {
-            gm_k_floor = gm_k_est + 1;
-            gm_k_floor_age = 0;
-            gm_k_est = std::min(gm_m, gm_k_est + 2);
-            gm_k_fine = true;
-        } else if (graph_cycles == 2 && gm_cycles == 2) {
-            if (gm_k_est < 6) {
-                gm_k_est = 6;
-                gm_k_floor = 6;
-                gm_k_floor_age = 0;
-            } else if (rel < desc.tol / 3.0) {
-                gm_k_est = std::max(std::max(6, gm_k_floor),
-                                    gm_k_est - (gm_k_fine ? 1 : std::max(1, gm_k_est / 5)));
-            }
-        } else if (graph_cycles == 1 && gm_cycles == 1 && rel < desc.tol / 3.0) {
-            gm_k_est = std::max(std::max(5, gm_k_floor), gm_k_est - 1);
-        }
+    } else if (transient && gm_cycles > 0 && rel <= desc.tol) {
+        gm_k_est = std::min(std::min(gm_m, 12), std::max(2, count_for(stats.inner_iterations)));
+        gm_ls_floor = 0;
     }
     unsigned stt = 0;
     double lsv[8] = {};

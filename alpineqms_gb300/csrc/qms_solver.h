@@ -134,7 +134,6 @@ struct QmsSolver {
     std::deque<OpEv> evpool;
     size_t evused = 0;
     bool capturing = false;                      // event records go into a graph being captured
-    bool graph_prof_broken = false;
     qms_profile profacc{};
     // the multigrid's timing hook (the A-block sweeps), forwarding to prof_begin / prof_end
     struct MgHook : MgProf {
@@ -189,21 +188,22 @@ struct QmsSolver {
     template <typename T> int inner_pcg(bool transient, int& iters);
     template <typename T> int inner_gmres(bool adv, bool transient, const double v[3], int& iters, int fixed_k);
     int residual_launch(bool adv, bool transient, const double v[3], bool exact = false);
-    int ir_iteration_graph(bool adv, bool transient, const double v[3], int k);
-    // captured refinement iterations, one per FGMRES count k (and step parameters); the
-    // profile event records of a capture belong to its entry
-    struct IrGraph {
+    template <typename T> void gmres_begin();
+    template <typename T> void gmres_steps(bool adv, bool transient, const double v[3], int j0, int j1);
+    template <typename T> void gmres_end(int k);
+    int gmres_estimate(double& est);
+    int gmres_segment(bool adv, bool transient, const double v[3], int j0, int j1, bool graph);
+    int gmres_cycle(bool adv, bool transient, const double v[3], double stop, bool graph, int& iters);
+    // kSeg steps of an FGMRES cycle captured as one graph, for the operator (seg_tr, seg_v)
+    static constexpr int kSeg = 2;
+    struct SegGraph {
         cudaGraphExec_t exec = nullptr;
-        int k = 0;
-        bool tr = false, adv = false, prof = false;
-        bool resid_df = false;      // the captured residual is the double-float one (rfin)
-        double v[3] = {0, 0, 0};
         long long launches = 0;
-        std::deque<OpEv> ev;
-        size_t evn = 0;
-        unsigned long long used = 0;
     };
-    std::vector<IrGraph> graphs;
+    std::vector<SegGraph> segs;
+    bool seg_valid = false, seg_tr = false;
+    double seg_v[3] = {0, 0, 0};
+    void drop_segments();
     // Whole chained transient steps as one CUDA graph each: the status reset, the step start (its
     // rotating history pointers copied from pinned host memory by a node of the graph), the start
     // residual, and a conditional WHILE node whose body is one refinement cycle (FGMRES with k
@@ -226,16 +226,10 @@ struct QmsSolver {
     unsigned long long graph_clock = 0;
     void drop_graphs();
     bool graph_resid_ready = false;
-    int gm_k_est = 0;           // FGMRES iterations replayed per refinement iteration (0: not yet known)
-    int gm_k_seen = 0;          // largest count seen while running with host checks
-    int gm_ls_floor = 0;        // lowest count for solves after a least-squares start, and its age
+    int gm_k_est = 0;           // FGMRES steps per cycle of a step run as one graph (0: not yet known)
+    int gm_ls_floor = 0;        // its lowest value for now, and that value's age in solves
     int gm_ls_floor_age = 0;
-    bool gm_k_fine = false;     // gm_k_est has overshot downwards once: tune it in single steps
-    int gm_k_floor = 0;         // smallest count not yet known to need a third replay
-    int gm_k_floor_age = 0;     // solves since gm_k_floor was set or lowered
-    // log of the per-iteration residual reduction of FGMRES, smoothed over solves: [0] the first
-    // cycle of a solve, [1] the later ones (which start from a residual rich in slow modes)
-    double gm_lrate[2] = {0, 0};
+    double gm_rate = 0.0;       // log of the residual estimate per FGMRES step, smoothed over cycles
     void* gmV[65] = {};         // FGMRES basis (m + 1) and preconditioned directions (m), m <= 64
     void* gmZ[64] = {};
     double* gm_H = nullptr;     // Hessenberg matrix (m+1) x m, row-major with stride m

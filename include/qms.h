@@ -91,8 +91,9 @@ typedef struct {
                                 potential of isolated conductors) */
     int krylov;              /* nonsymmetric inner solver: QMS_KRYLOV_GMRES (default) or _BICGSTAB */
     int gmres_m;             /* FGMRES basis size per refinement iteration (<= 64) */
-    int use_graphs;          /* replay each refinement iteration of a step as one CUDA graph, with the
-                                FGMRES iteration count learned from the first solve (1 = on) */
+    int use_graphs;          /* replay the FGMRES steps of a time step from CUDA graphs, and chained
+                                steps whole (1 = on); cycles then end by their residual estimate at
+                                equal shares of the reduction still wanted */
     double mg_region_cut;    /* conductor-region coarse space of the potential block: eigenvalues of
                                 its region-stiffness-scaled Galerkin matrix at or below this are
                                 dropped (0 = automatic: 1e-9 with FP64 inner vectors, 1e-6 with FP32;
@@ -119,11 +120,8 @@ typedef struct {
                                 diagonals it aggregates leaves the hierarchy, and the coarsest solve
                                 drops eigenvalues of its operator scaled by those sums at or below
                                 it (0 = automatic: 1e-9 with FP64 inner vectors, 1e-5 with FP32) */
-    int gm_first_extend;     /* replayed refinement iterations: the first FGMRES cycle of a solve may run
-                                up to this many steps beyond the learned count when the start residual
-                                and the observed first-cycle rate say that one cycle then reaches the
-                                tolerance (instead of two cycles); 0 = never (the default: on the
-                                moving plate it kept longer single cycles, 30.6 vs 28.0 ms per step) */
+    int gm_first_extend;     /* accepted and without effect: it lengthened a first cycle of a learned count,
+                                and cycles now end by their own residual estimate */
     double tol_v;            /* > 0: a solve also stops only when ||r_V|| <= tol_v * ||x_V|| (the potential block's
                                 scaled residual against its own size); 0 = off (the default) */
     int start_ls;            /* chained transient steps (mixed precision): the start is x_n plus the combination

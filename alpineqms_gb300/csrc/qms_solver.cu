@@ -18,6 +18,7 @@
 #include "qms_solver.h"
 #include "qms_pl.h"
 
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -45,13 +46,18 @@ enum FinOp {
 
 __global__ void qk_finalize(const double* __restrict__ part, long long nb, int nsum, double* __restrict__ S, int op,
                             unsigned* __restrict__ status) {
-    __shared__ double sh[32];
-    double sums[4];
-    for (int q = 0; q < nsum; q++) {
+    // a quarter of the block's warps per sum (16 warps, up to 4 sums), added up in a fixed order
+    __shared__ double sh[4][4];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = wid >> 2, part_w = wid & 3;
+    if (q < nsum) {
         double acc = 0.0;
-        for (long long t = threadIdx.x; t < nb; t += blockDim.x) acc += part[q * nb + t];
-        sums[q] = qBlockSum(acc, sh);
+        for (long long t = part_w * 32 + lane; t < nb; t += 128) acc += part[q * nb + t];
+        acc = qWarpSum(acc);
+        if (lane == 0) sh[q][part_w] = acc;
     }
+    __syncthreads();
+    double sums[4];
+    for (int i = 0; i < 4; i++) sums[i] = (sh[i][0] + sh[i][1]) + (sh[i][2] + sh[i][3]);
     if (threadIdx.x != 0) return;
     switch (op) {
     case FIN_RESID: {
@@ -277,16 +283,44 @@ template <> struct GmPack<double> {
     static __device__ __forceinline__ double at(const V& v, int q) { return q == 0 ? v.x : v.y; }
 };
 
-// h_ij = V_i . w for i < NV, and w . w (partials at NV nb + block)
+// True in every thread of the block that arrives last (its threads then see what the others wrote
+// before); the counter is zero again for the next launch.
+__device__ __forceinline__ bool gm_last_block(unsigned* counter) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(counter, 1u) == gridDim.x - 1;
+        if (last) *counter = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// h_ij = V_i . w for i < NV, and w . w, as block partials (row i of `part`, rows of gridDim.x); in
+// the last pass over the basis (final) the last block adds them up in a fixed order into column j
+// of H and forms the norm of the orthogonalised w from Pythagoras, |w'|^2 = |w|^2 - sum_i h_ij^2:
+// when that keeps at least a hundredth of |w|^2 (no severe cancellation), Gm[4] = |w'| and Gm[3]
+// = 1, and the orthogonalisation writes V_{j+1} = w' / |w'| directly (no norm pass over w', no
+// scaling pass); otherwise Gm[3] = 0.  row0: the basis vectors of the passes before; part0: row 0.
+// On large grids the basis vectors' bandwidth bounds this (256^3: 85-90 % of the copy rate); on
+// small ones the tail did: a block sum with two barriers per vector and a one-block kernel that
+// added up one vector after the other.  Now the warps leave their sums in shared memory behind one
+// barrier, and each warp of the last block adds up vectors of its own (48^3: 240 ms per run of 8
+// steps instead of 299, 64x64x80 core 261 instead of 303).  The grid is one resident wave: with
+// eight blocks per SM whatever the registers, a second wave of a few blocks followed (256^3, 8
+// vectors: 367 us instead of 405).
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) qk_gm_dots(long long n, GmPtrs V, const T* __restrict__ w,
-                                                  double* __restrict__ part) {
+                                                  double* __restrict__ part0, int row0, int final, int j, int m,
+                                                  double* __restrict__ Hm, double* __restrict__ Gm,
+                                                  unsigned* __restrict__ counter) {
     using PK = GmPack<T>;
     using PV = typename PK::V;
-    float acc[NV];
-    float accw = 0.f;
+    float acc[NV + 1];
 #pragma unroll
-    for (int i = 0; i < NV; i++) acc[i] = 0.f;
+    for (int i = 0; i <= NV; i++) acc[i] = 0.f;
     const PV* vp[NV];
 #pragma unroll
     for (int i = 0; i < NV; i++) vp[i] = (const PV*)V.p[i];
@@ -302,57 +336,59 @@ __global__ void __launch_bounds__(256) qk_gm_dots(long long n, GmPtrs V, const T
 #pragma unroll
             for (int q = 0; q < PK::W; q++) acc[i] += (float)(PK::at(vv[i], q) * PK::at(wv, q));
 #pragma unroll
-        for (int q = 0; q < PK::W; q++) accw += (float)(PK::at(wv, q) * PK::at(wv, q));
+        for (int q = 0; q < PK::W; q++) acc[NV] += (float)(PK::at(wv, q) * PK::at(wv, q));
     }
-    __shared__ double sh[32];
+    __shared__ double sums[GM_MAXM + 2];
+    __shared__ float sh[NV + 1][8];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
 #pragma unroll
-    for (int i = 0; i < NV; i++) {
-        double sum = qBlockSum(acc[i], sh);
-        if (threadIdx.x == 0) part[(long long)i * gridDim.x + blockIdx.x] = sum;
+    for (int i = 0; i <= NV; i++) {
+        const float s = qWarpSum(acc[i]);
+        if (lane == 0) sh[i][wid] = s;
     }
-    const double sw = qBlockSum(accw, sh);
-    if (threadIdx.x == 0) part[(long long)NV * gridDim.x + blockIdx.x] = sw;
-}
-
-// column j of H from the partials (h_ij = V_i . w), and the norm of the orthogonalised w from
-// Pythagoras, |w'|^2 = |w|^2 - sum_i h_ij^2: when that keeps at least a hundredth of |w|^2 (no
-// severe cancellation), Gm[4] = |w'| and Gm[3] = 1, and the orthogonalisation writes V_{j+1}
-// = w' / |w'| directly (no norm pass over w', no scaling pass); otherwise Gm[3] = 0
-__global__ void qk_gm_hcol(const double* __restrict__ part, long long nb, int j, int m, double* __restrict__ Hm,
-                           double* __restrict__ Gm) {
-    __shared__ double sh[32];
-    double hh = 0.0;
-    for (int i = 0; i <= j + 1; i++) {
-        double acc = 0.0;
-        for (long long t = threadIdx.x; t < nb; t += blockDim.x) acc += part[(long long)i * nb + t];
-        double s = qBlockSum(acc, sh);
-        if (threadIdx.x == 0) {
-            if (i <= j) {
-                Hm[i * m + j] = s;
-                hh += s * s;
-            } else {
-                const double est = s - hh;
-                const bool ok = isfinite(est) && est > 1e-2 * s;
-                Gm[3] = ok ? 1.0 : 0.0;
-                Gm[4] = ok ? sqrt(est) : 0.0;
-            }
-        }
+    __syncthreads();
+    if (threadIdx.x <= NV) {
+        double s = 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) s += (double)sh[threadIdx.x][q];
+        part0[(long long)(row0 + threadIdx.x) * gridDim.x + blockIdx.x] = s;
+    }
+    if (!final || !gm_last_block(counter)) return;
+    for (int i = wid; i <= j + 1; i += 8) {
+        double s = 0.0;
+        for (int t = lane; t < (int)gridDim.x; t += 32) s += __ldcg(part0 + (long long)i * gridDim.x + t);
+        s = qWarpSum(s);
+        if (lane == 0) sums[i] = s;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x <= j) Hm[threadIdx.x * m + j] = sums[threadIdx.x];
+    if (threadIdx.x == 0) {
+        double hh = 0.0;
+        for (int i = 0; i <= j; i++) hh += sums[i] * sums[i];
+        const double s = sums[j + 1], est = s - hh;
+        const bool ok = isfinite(est) && est > 1e-2 * s;
+        Gm[3] = ok ? 1.0 : 0.0;
+        Gm[4] = ok ? sqrt(est) : 0.0;
     }
 }
 
-// w' = w - sum_i h_ij V_i (NV = j + 1, compile-time; 16-byte packets): with Gm[3] set, V_{j+1} =
-// w' / Gm[4] goes to vout; otherwise w' back into w with the partials of |w'|^2
+// w' = w - sum_i h_ij V_i (NV basis vectors, compile-time; 16-byte packets): with Gm[3] set, V_{j+1}
+// = w' / Gm[4] goes to vout; otherwise w' back into w with the partials of |w'|^2.
+// final = 0: a first pass over part of the basis (w' back into w, no norm partials, no direct write).
+// In the last pass the last block (every block has read column j of H by then) takes h_{j+1,j} = |w'|,
+// applies the Givens rotations and forms the residual estimate; Gm layout: [0]: beta,
+// [1]: |g_{j+1}|, [2]: 1/h_{j+1,j}, cs[m] at 8, sn[m] at 8+m, g[m+1] at 8+2m
 template <typename T, int NV>
-// final = 0: a first pass over part of the basis (w' back into w, no norm partials, no direct write)
-__global__ void __launch_bounds__(256) qk_gm_orth(long long n, int j, int m, GmPtrs V, const double* __restrict__ Hm,
-                                                  T* __restrict__ w, double* __restrict__ part,
-                                                  const double* __restrict__ Gm, T* __restrict__ vout, int final) {
+__global__ void __launch_bounds__(256) qk_gm_orth(long long n, int j, int m, GmPtrs V, double* __restrict__ Hcol0,
+                                                  int row0, T* __restrict__ w, double* __restrict__ part,
+                                                  double* __restrict__ Gm, T* __restrict__ vout, int final,
+                                                  unsigned* __restrict__ counter, unsigned* __restrict__ status) {
     using PK = GmPack<T>;
     using PV = typename PK::V;
     T h[NV];
     const PV* vp[NV];
 #pragma unroll
-    for (int i = 0; i < NV; i++) { h[i] = (T)Hm[i * m + j]; vp[i] = (const PV*)V.p[i]; }
+    for (int i = 0; i < NV; i++) { h[i] = (T)Hcol0[(row0 + i) * m + j]; vp[i] = (const PV*)V.p[i]; }
     const bool direct = final && Gm[3] != 0.0;
     const T inv = direct ? (T)(1.0 / Gm[4]) : T(1);
     PV* wp = (PV*)w;
@@ -375,42 +411,49 @@ __global__ void __launch_bounds__(256) qk_gm_orth(long long n, int j, int m, GmP
         }
         op[t] = wv;
     }
-    if (direct || !final) return;
+    if (!final) return;
     __shared__ double sh[32];
-    double s0 = qBlockSum(acc, sh);
-    if (threadIdx.x == 0) part[blockIdx.x] = s0;
-}
-
-// h_{j+1,j} = |w|, Givens rotations, residual estimate; Gm layout:
-// [0]: beta, [1]: |g_{j+1}|, [2]: 1/h_{j+1,j}, cs[m] at 8, sn[m] at 8+m, g[m+1] at 8+2m
-__global__ void qk_gm_givens(const double* __restrict__ part, long long nb, int j, int m, double* __restrict__ Hm,
-                             double* __restrict__ Gm, unsigned* __restrict__ status) {
-    __shared__ double sh[32];
-    const bool direct = Gm[3] != 0.0;
-    double acc = 0.0;
-    if (!direct)
-        for (long long t = threadIdx.x; t < nb; t += blockDim.x) acc += part[t];
-    double nw = qBlockSum(acc, sh);
-    if (threadIdx.x != 0) return;
-    double hn = direct ? Gm[4] : sqrt(nw);
-    double* cs = Gm + 8;
-    double* sn = Gm + 8 + m;
-    double* gv = Gm + 8 + 2 * m;
-    Gm[2] = hn > 0.0 ? 1.0 / hn : 0.0;
-    for (int i = 0; i < j; i++) {                // previous rotations on column j
-        double a = Hm[i * m + j], b = Hm[(i + 1) * m + j];
-        Hm[i * m + j] = cs[i] * a + sn[i] * b;
-        Hm[(i + 1) * m + j] = -sn[i] * a + cs[i] * b;
+    if (!direct) {
+        const double s0 = qBlockSum(acc, sh);
+        if (threadIdx.x == 0) part[blockIdx.x] = s0;
     }
-    double a = Hm[j * m + j], b = hn;
-    double r = sqrt(a * a + b * b);
-    double c = r > 0.0 ? a / r : 1.0, s = r > 0.0 ? b / r : 0.0;
-    cs[j] = c; sn[j] = s;
-    Hm[j * m + j] = r;
-    gv[j + 1] = -s * gv[j];
-    gv[j] = c * gv[j];
-    Gm[1] = fabs(gv[j + 1]);
-    if (!(r > 0.0) || !isfinite(r)) atomicOr(status, (unsigned)QMS_ST_BREAKDOWN);
+    if (!gm_last_block(counter)) return;
+    double nw = 0.0;
+    if (!direct) {
+        for (int t = threadIdx.x; t < (int)gridDim.x; t += blockDim.x) nw += __ldcg(part + t);
+        nw = qBlockSum(nw, sh);
+    }
+    // column j of H and the rotations in shared memory: the chain of rotations is one thread's
+    __shared__ double hc[GM_MAXM + 1], rc[GM_MAXM], rs[GM_MAXM];
+    if ((int)threadIdx.x <= j) hc[threadIdx.x] = __ldcg(Hcol0 + threadIdx.x * m + j);
+    if ((int)threadIdx.x < j) {
+        rc[threadIdx.x] = Gm[8 + threadIdx.x];
+        rs[threadIdx.x] = Gm[8 + m + threadIdx.x];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double hn = direct ? Gm[4] : sqrt(nw);
+        double* gv = Gm + 8 + 2 * m;
+        Gm[2] = hn > 0.0 ? 1.0 / hn : 0.0;
+        double b = hc[0];
+        for (int i = 0; i < j; i++) {                // previous rotations on column j
+            const double a = b, c = hc[i + 1];
+            hc[i] = rc[i] * a + rs[i] * c;
+            b = -rs[i] * a + rc[i] * c;
+        }
+        const double r = sqrt(b * b + hn * hn);
+        const double c = r > 0.0 ? b / r : 1.0, s = r > 0.0 ? hn / r : 0.0;
+        Gm[8 + j] = c;
+        Gm[8 + m + j] = s;
+        hc[j] = r;
+        const double gj = gv[j];
+        gv[j + 1] = -s * gj;
+        gv[j] = c * gj;
+        Gm[1] = fabs(s * gj);
+        if (!(r > 0.0) || !isfinite(r)) atomicOr(status, (unsigned)QMS_ST_BREAKDOWN);
+    }
+    __syncthreads();
+    if ((int)threadIdx.x <= j) Hcol0[threadIdx.x * m + j] = hc[threadIdx.x];
 }
 
 // V_{j+1} = w / h_{j+1,j} (nothing to do when the orthogonalisation wrote it, Gm[3])
@@ -429,16 +472,25 @@ __global__ void qk_gm_reset(int m, double* __restrict__ Gm) {
     if (threadIdx.x == 0) { Gm[0] = 1.0; Gm[8 + 2 * m] = 1.0; Gm[1] = 1.0; }
 }
 
-// back substitution H(0:k,0:k) y = g(0:k); y stored at Gm + 8 + 3m + 1
-__global__ void qk_gm_solve(int k, int m, const double* __restrict__ Hm, double* __restrict__ Gm) {
-    if (threadIdx.x != 0) return;
+// back substitution H(0:k,0:k) y = g(0:k), column by column in one warp (lane l holds the right-hand
+// sides of rows l and l + 32); y stored at Gm + 8 + 3m + 1
+__global__ void __launch_bounds__(256) qk_gm_solve(int k, int m, const double* __restrict__ Hm,
+                                                  double* __restrict__ Gm) {
+    __shared__ double hs[GM_MAXM * GM_MAXM];
+    for (int q = threadIdx.x; q < k * k; q += blockDim.x) hs[q] = Hm[(q / k) * m + q % k];
+    __syncthreads();
+    if (threadIdx.x >= 32) return;
+    const int lane = threadIdx.x;
     const double* gv = Gm + 8 + 2 * m;
     double* y = Gm + 8 + 3 * m + 1;
+    double a0 = lane < k ? gv[lane] : 0.0, a1 = lane + 32 < k ? gv[lane + 32] : 0.0;
     for (int i = k - 1; i >= 0; i--) {
-        double acc = gv[i];
-        for (int q = i + 1; q < k; q++) acc -= Hm[i * m + q] * y[q];
-        const double d = Hm[i * m + i];
-        y[i] = d != 0.0 ? acc / d : 0.0;
+        const double d = hs[i * k + i];
+        const double acc = __shfl_sync(0xffffffffu, i >= 32 ? a1 : a0, i & 31);
+        const double yi = d != 0.0 ? acc / d : 0.0;
+        if (lane == 0) y[i] = yi;
+        if (lane < i) a0 -= hs[lane * k + i] * yi;
+        if (lane + 32 < i) a1 -= hs[(lane + 32) * k + i] * yi;
     }
 }
 
@@ -479,35 +531,44 @@ static GmPtrs gm_shift(const GmPtrs& V, int off) {
     for (int i = 0; i + off <= GM_MAXM; i++) r.p[i] = V.p[i + off];
     return r;
 }
-// returns the kernel launches
-template <typename T>
-static int gm_dots(int nv, int vb, cudaStream_t st, long long n, const GmPtrs& V, const T* w, double* part) {
-    if (nv > GM_PASS) {
-        // the first GM_PASS projections, then the rest (whose |w|^2 partials land at nv * vb)
-        gm_dots<T>(GM_PASS, vb, st, n, V, w, part);
-        return 1 + gm_dots<T>(nv - GM_PASS, vb, st, n, gm_shift(V, GM_PASS), w, part + (long long)GM_PASS * vb);
+// One resident wave of blocks (at most vb): each walks the vectors with the same stride, so blocks of a
+// second, partial wave would run while most SMs have nothing left
+static int gm_blocks(const void* kernel, std::atomic<int>& per, int vb) {
+    int p = per.load(std::memory_order_relaxed);
+    if (p == 0) {
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, kernel, 256, 0);
+        p = std::max(1, p);
+        per.store(p, std::memory_order_relaxed);
     }
-    switch (nv) {
-#define C(N) case N: qk_gm_dots<T, N><<<vb, 256, 0, st>>>(n, V, w, part); break;
+    return std::min(vb, 152 * p);
+}
+// return the kernel launches
+template <typename T>
+static int gm_dots(int nv, int vb, cudaStream_t st, long long n, const GmPtrs& V, const T* w, double* part, int row0,
+                   int j, int m, double* Hm, double* Gm, unsigned* counter) {
+    const int now = std::min(nv, GM_PASS), final = now == nv ? 1 : 0;
+    int nb = vb;                                // later passes: as many blocks (partials) as the first
+    switch (now) {
+#define C(N) case N: { static std::atomic<int> per{0}; \
+        if (row0 == 0) nb = gm_blocks((const void*)qk_gm_dots<T, N>, per, vb); \
+        qk_gm_dots<T, N><<<nb, 256, 0, st>>>(n, V, w, part, row0, final, j, m, Hm, Gm, counter); } break;
         GM_CASES(C)
 #undef C
     }
-    return 1;
+    return final ? 1 : 1 + gm_dots<T>(nv - now, nb, st, n, gm_shift(V, now), w, part, row0 + now, j, m, Hm, Gm, counter);
 }
 template <typename T>
-static int gm_orth(int nv, int vb, cudaStream_t st, long long n, int j, int m, const GmPtrs& V, const double* Hm, T* w,
-                   double* part, const double* Gm, T* vout, int final = 1) {
-    if (nv > GM_PASS) {
-        gm_orth<T>(GM_PASS, vb, st, n, j, m, V, Hm, w, part, Gm, vout, 0);
-        return 1 + gm_orth<T>(nv - GM_PASS, vb, st, n, j, m, gm_shift(V, GM_PASS), Hm + (long long)GM_PASS * m, w,
-                              part, Gm, vout, final);
-    }
-    switch (nv) {
-#define C(N) case N: qk_gm_orth<T, N><<<vb, 256, 0, st>>>(n, j, m, V, Hm, w, part, Gm, vout, final); break;
+static int gm_orth(int nv, int vb, cudaStream_t st, long long n, int j, int m, const GmPtrs& V, double* Hm, int row0,
+                   T* w, double* part, double* Gm, T* vout, unsigned* counter, unsigned* status) {
+    const int now = std::min(nv, GM_PASS), final = now == nv ? 1 : 0;
+    switch (now) {
+#define C(N) case N: { static std::atomic<int> per{0}; \
+        qk_gm_orth<T, N><<<gm_blocks((const void*)qk_gm_orth<T, N>, per, vb), 256, 0, st>>>(n, j, m, V, Hm, row0, w, part, Gm, vout, final, counter, status); } break;
         GM_CASES(C)
 #undef C
     }
-    return 1;
+    return final ? 1 : 1 + gm_orth<T>(nv - now, vb, st, n, j, m, gm_shift(V, now), Hm, row0 + now, w, part, Gm, vout,
+                                      counter, status);
 }
 template <typename T>
 static int gm_update(int nv, cudaStream_t st, const QGrid& g, int m, const GmPtrs& Z, const double* Gm,
@@ -569,7 +630,9 @@ void QmsSolver::release() {
     for (auto& p : gmZ) { if (p) cudaFree(p); p = nullptr; }
     if (gm_H) cudaFree(gm_H);
     if (gm_scal) cudaFree(gm_scal);
+    if (gm_count) cudaFree(gm_count);
     gm_H = gm_scal = nullptr;
+    gm_count = nullptr;
     if (nc16) cudaFree(nc16);
     nc16 = nullptr;
     void* ptrs[] = {ids,   dtab64, dtab32,    x,     b,      r64,    xbest, H,   slicebuf, part,   S,
@@ -676,6 +739,8 @@ int QmsSolver::init(const qms_desc& d) {
         if (use_mg) for (int i = 0; i < m; i++) CK(pl_alloc(&gmZ[i], tsize));
         CK(cudaMalloc(&gm_H, (size_t)m * (m + 1) * 8));
         CK(cudaMalloc(&gm_scal, (size_t)(8 + 4 * m + 8) * 8));
+        CK(cudaMalloc(&gm_count, sizeof(unsigned)));
+        CK(cudaMemsetAsync(gm_count, 0, sizeof(unsigned), st));
     }
     CK(cudaMallocHost(&hS, S_COUNT * 8));
     CK(cudaMemsetAsync(x, 0, n * 8, st));
@@ -1067,7 +1132,8 @@ void QmsSolver::gmres_steps(bool adv, bool transient, const double v[3], int j0,
     const int m = std::min(desc.gmres_m, GM_MAXM);
     const float* dg = transient ? dg_tr : dg_steady;
     QStepPar<T> P = qms_step_par<T>(g, v[0], v[1], v[2], desc.dt, transient);
-    const int vb = (int)vec_blocks;
+    // two packets per thread at least: fewer partial sums to add up on small grids
+    const int vb = (int)std::max(1LL, std::min(vec_blocks, (n * (long long)sizeof(T) / 16 + 511) / 512));
     GmPtrs Vp{};
     for (int i = 0; i <= m; i++) Vp.p[i] = gmV[i];
     T* w = (T*)vec[0];
@@ -1076,12 +1142,10 @@ void QmsSolver::gmres_steps(bool adv, bool transient, const double v[3], int j0,
         T* zj = use_mg ? (T*)gmZ[j] : vj;
         if (use_mg) precond<T>(vj, dg, zj, false, transient, false, &P, adv);
         op_pl<T>(adv, QOPH_SCALED, P, zj, w, nullptr, nullptr);
-        nlaunch += gm_dots<T>(j + 1, vb, st, n, Vp, w, part);
-        qk_gm_hcol<<<1, 512, 0, st>>>(part, vec_blocks, j, m, gm_H, gm_scal);
-        nlaunch += gm_orth<T>(j + 1, vb, st, n, j, m, Vp, gm_H, w, part, gm_scal, (T*)gmV[j + 1]);
-        qk_gm_givens<<<1, 512, 0, st>>>(part, vec_blocks, j, m, gm_H, gm_scal, status);
-        qk_gm_scale<T><<<vb, 256, 0, st>>>(n, w, (T*)gmV[j + 1], gm_scal);
-        nlaunch += 3;
+        nlaunch += gm_dots<T>(j + 1, vb, st, n, Vp, w, part, 0, j, m, gm_H, gm_scal, gm_count);
+        nlaunch += gm_orth<T>(j + 1, vb, st, n, j, m, Vp, gm_H, 0, w, part, gm_scal, (T*)gmV[j + 1], gm_count, status);
+        qk_gm_scale<T><<<std::min(vb, 152), 256, 0, st>>>(n, w, (T*)gmV[j + 1], gm_scal);
+        nlaunch++;
     }
 }
 
@@ -1090,7 +1154,7 @@ void QmsSolver::gmres_end(int k) {
     const int m = std::min(desc.gmres_m, GM_MAXM);
     GmPtrs Zp{};
     for (int i = 0; i < m; i++) Zp.p[i] = use_mg ? gmZ[i] : gmV[i];
-    qk_gm_solve<<<1, 32, 0, st>>>(k, m, gm_H, gm_scal);
+    qk_gm_solve<<<1, 256, 0, st>>>(k, m, gm_H, gm_scal);
     nlaunch += 1 + gm_update<T>(k, st, g, m, Zp, gm_scal, S, x);
     last_gm_k = k;
 }
@@ -1170,8 +1234,8 @@ int QmsSolver::gmres_segment(bool adv, bool transient, const double v[3], int j0
 }
 
 // One cycle that ends when its residual estimate reaches `stop` (or the basis is full).  The first
-// look at the estimate comes shortly before the count that the last cycles' rate predicts, so a
-// cycle costs a host wait or two.  A cycle that ran on past the FP32 floor cost most: the counts
+// look at the estimate comes at 0.6 of the count that the last cycles' rate predicts (a look costs a
+// host wait of some 15 us, a step too many 0.2 to 5 ms).  A cycle that ran on past the FP32 floor cost most: the counts
 // that were learned across solves before grew to 32 steps where 8 reach it (a plate in harmonic
 // motion: 84 steps per time step instead of 28).
 int QmsSolver::gmres_cycle(bool adv, bool transient, const double v[3], double stop, bool graph, int& iters) {
@@ -1179,7 +1243,7 @@ int QmsSolver::gmres_cycle(bool adv, bool transient, const double v[3], double s
     if (fp64_inner) gmres_begin<double>();
     else gmres_begin<float>();
     int k = 0, upto = kSeg;
-    if (gm_rate < 0.0) upto = (int)std::min((double)m, std::floor(std::log(stop) / gm_rate) - 1.0);
+    if (gm_rate < 0.0) upto = (int)std::min((double)m, 0.6 * std::log(stop) / gm_rate);
     upto = std::min(m, std::max(kSeg, upto));
     double est = 1.0;
     for (;;) {

@@ -233,6 +233,7 @@ struct QmsSolver {
     void* gmV[65] = {};         // FGMRES basis (m + 1) and preconditioned directions (m), m <= 64
     void* gmZ[64] = {};
     double* gm_H = nullptr;     // Hessenberg matrix (m+1) x m, row-major with stride m
+    unsigned* gm_count = nullptr;   // blocks of a Gram-Schmidt kernel that are done
     double* gm_scal = nullptr;  // beta, |g_{j+1}|, 1/h, rotations, g, y
     int last_gm_k = 0;
     int last_inner = 0;         // 0 PCG, 1 BiCGSTAB, 2 FGMRES

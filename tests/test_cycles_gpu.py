@@ -4,7 +4,8 @@ A velocity that repeats replays the cycle's steps from graphs, a new one launche
 drops the graphs of the one before; bases of odd and of the largest length end a cycle in the middle
 of a graph's steps.  Whatever the route, every step meets the tolerance in the exact FP64 residual
 (1.5 tol: the double-float residual's rounding stays below tol / 10), also after a state that was
-set from outside.
+set from outside.  The solver's tolerance is relative to the larger of |x| before and after the solve
+(a frame that stops loses its potential, and |x| shrinks), qms_residual_norm's to |x| after it.
 """
 import numpy as np
 import pytest
@@ -35,6 +36,8 @@ def test_steps_meet_the_tolerance_on_every_route(precision, m, krylov_graphs):
         for again in range(2):
             s.set_state(start)
             for n, v in enumerate(moves):
+                before = np.linalg.norm(s.get_state())
                 st = s.step(v, (1.0 - 0.05 * n) * B, G)
+                after = np.linalg.norm(s.get_state())
                 assert st["status"] == 0 and st["r"] <= s.desc.tol, (again, n, st)
-                assert s.residual_norm(True, v) <= 1.5 * s.desc.tol, (again, n)
+                assert s.residual_norm(True, v) * after <= 1.5 * s.desc.tol * max(before, after), (again, n)

@@ -26,6 +26,7 @@
 #include "qms_pl.h"
 #include "qms_tile.cuh"
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include <atomic>
@@ -33,6 +34,8 @@
 #include <cstring>
 #include <map>
 #include <vector>
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -294,139 +297,270 @@ __global__ void mg_prolong(MGLevelDev<T> F, const T* xin, T* xf, MGLevelDev<T> C
     xf[t] = xin[t] + alpha * xc[cb.off + (i >> 1) + (long long)(j >> 1) * cb.n1 + (long long)(k >> 1) * cb.n1 * cb.n2];
 }
 
-// coarsest level: x = Minv b per block, dense FP64 (one CTA per block)
+// ------------------------------------------------------------------ coarse sub-cycle
+// The last levels of a cycle in one launch: one cluster of CTAs (16, or 8 where the chip cannot place 16)
+// per block runs their whole V-cycle for that block.  A level's planes are dealt out to the CTAs in slabs (a level of at most
+// MGC_LOCAL points is the first CTA's alone); links, right-hand side and x live in shared memory, x
+// with a halo plane on each side, the boundary planes are written to the neighbours' halos through
+// distributed shared memory, and a pass ends with a cluster barrier.
+// These levels are bound by latency, not by bytes (33^3 points of a block are 0.1 MB per array): a
+// launch per sweep cost 2.8-4 us each, and the smallest levels in one CTA with their data in L2 20-36 us.
+// So the links are copied to shared memory once per cycle (the lower levels' while the first one runs);
+// the passes are short loops that every level shares (unrolled by the points of a thread, with the links
+// in registers, a level's first pass waited for its instructions: 15,000 clocks for a sweep of 4,000);
+// and levels whose cluster barriers (600 clocks) would outweigh their work stay in one CTA.
+// Per cycle on the A blocks, levels 25^3 to 4^3: 63 us as nine launches before, 24 us now; 33^3 to 5^3:
+// 76 us as seventeen, 36 us now.  Measured and not taken: 8 CTAs (3 % slower on the runs), 1024 or 256
+// threads (7 %, 2-5 %), one-CTA levels of up to 2500 points (3 %).
+#define MGC_THREADS 512
+#define MGC_LEVELS 8
+#define MGC_LOCAL 1024
+#define MGC_SMEM (216 * 1024)
 template <typename T>
-__global__ void mg_dense(MGLevelDev<T> L, const double* __restrict__ minv, const long long* __restrict__ moff,
-                         const T* __restrict__ b, T* __restrict__ x, int mask_v) {
-    const int blk = blockIdx.x;
-    const MGBlockDesc& B = L.blk[blk];
-    const int m = B.n1 * B.n2 * B.n3;
-    const double* M = minv + moff[blk];
-    for (int r = threadIdx.x; r < m; r += blockDim.x) {
-        double acc = 0.0;
-        if (!(mask_v && blk == L.nb - 1))
-            for (int c = 0; c < m; c++) acc += M[(long long)r * m + c] * (double)b[B.off + c];
-        x[B.off + r] = (T)acc;
-    }
+struct MGSub {
+    int nl;                                     // levels; the last is the coarsest
+    int lg;                                     // 2^lg CTAs in the cluster
+    MGLevelDev<T> L[MGC_LEVELS];
+};
+// planes of a level that one CTA of 2^lg holds, and the shared memory (elements) of a level: two copies of x
+// with halo planes and an element on either side, the right-hand side, and (not the last level) dinv,
+// w1, w2, w3 with the plane before
+__host__ __device__ __forceinline__ int mgc_planes(const MGBlockDesc& B, int lg) {
+    return (long long)B.n1 * B.n2 * B.n3 <= MGC_LOCAL ? B.n3 : (B.n3 + (1 << lg) - 1) >> lg;
+}
+__host__ __device__ __forceinline__ long long mgc_xlen(const MGBlockDesc& B, int lg) {
+    return (long long)(mgc_planes(B, lg) + 2) * B.n1 * B.n2 + 2;
+}
+__host__ __device__ __forceinline__ long long mgc_len(const MGBlockDesc& B, int lg, bool links) {
+    const int P = mgc_planes(B, lg);
+    return 2 * mgc_xlen(B, lg) + (long long)(P + (links ? 4 * (P + 1) : 0)) * B.n1 * B.n2;
+}
+// fast reciprocal in FP32 (a preconditioner needs no correctly rounded divide)
+template <typename T>
+__device__ __forceinline__ T mgc_rcp(T d) {
+    if constexpr (sizeof(T) == 4) return __fdividef(1.0f, d);
+    else return T(1) / d;
 }
 
+extern __shared__ __align__(16) unsigned char mgc_raw[];
 
-// ------------------------------------------------------------------ coarse tail
-// The last levels of a cycle (a few thousand points per block at most) in one launch: one CTA
-// per block runs their whole V-cycle for that block, passes separated by __syncthreads, the
-// data L2-resident.  These levels otherwise cost a launch per sweep, most of it latency.
-#define MG_TAIL_MAX_LEVELS 8
-template <typename T>
-struct MGTail {
-    int nl;                                     // tail levels; the last is the coarsest
-    MGLevelDev<T> L[MG_TAIL_MAX_LEVELS];
+// one CTA's slab of a level; x, b, w: indexes in the CTA's shared memory (of T): own point q of x at
+// x + which * xlen + s3 + q, its dinv and links at w + s3 + q + (0..3) * P4
+struct MGSlab {
+    int n1, n2, n3, s3, P, P3, P4, z0, np, rank;    // P: planes of a full slab, np: points of this one
+    int x, xlen, b, w;
+    bool dn, up, spread;                        // a neighbour holds the plane before / after; more than one CTA
+    __device__ __forceinline__ MGSlab(const MGBlockDesc& B, int lg, int c, int at) {
+        n1 = B.n1;
+        n2 = B.n2;
+        n3 = B.n3;
+        s3 = B.n1 * B.n2;
+        P = mgc_planes(B, lg);
+        P3 = P * s3;
+        P4 = P3 + s3;
+        rank = c;
+        z0 = min(c * P, B.n3);
+        np = (min(z0 + P, B.n3) - z0) * s3;
+        dn = c > 0 && np > 0;
+        up = z0 + P < B.n3;
+        spread = P < B.n3;
+        x = at + 1;
+        xlen = (int)mgc_xlen(B, lg);
+        b = at + 2 * xlen;
+        w = b + P3;
+    }
 };
 
 template <typename T>
-__global__ void __launch_bounds__(1024) mg_tail(MGTail<T> tl, const double* __restrict__ minv,
-                                                const long long* __restrict__ moff, T omega, T alpha, int nu1,
-                                                int nu2, int mask_v) {
-    const int b = blockIdx.x;
-    const int nb = tl.L[0].nb;
-    const bool masked = mask_v && b == nb - 1;
-    T* xcur[MG_TAIL_MAX_LEVELS];
-    T* tcur[MG_TAIL_MAX_LEVELS];
-    auto npts = [&](const MGBlockDesc& B) { return (long long)B.n1 * B.n2 * B.n3; };
-    // x_out = x_in + omega D^-1 (b - A x_in) over the block's points
-    auto sweep = [&](const MGLevelDev<T>& L, const T* xin, T* xout) {
-        const MGBlockDesc& B = L.blk[b];
-        const long long n = npts(B);
-        for (long long q = threadIdx.x; q < n; q += blockDim.x) {
-            const long long t = B.off + q;
-            const T di = masked ? T(0) : L.dinv[t];
-            if (di == T(0)) { xout[t] = T(0); continue; }
-            int i, j, k;
-            mg_ijk(q, B.n1, B.n2, i, j, k);
-            xout[t] = xin[t] + omega * di * (L.b[t] - apply7(L, B, t, i, j, k, xin));
+struct MGCluster {
+    cg::cluster_group cl;
+    T* sm;                                      // mgc_raw's part of T, the same place in every CTA
+    __device__ __forceinline__ void sync(bool all) {
+        if (all) cl.sync();
+        else __syncthreads();
+    }
+    __device__ __forceinline__ T* remote(int at, int rank) { return cl.map_shared_rank(sm + at, rank); }
+    // a value of the slab, and into the neighbours' halos from its outer planes
+    __device__ __forceinline__ void put(const MGSlab& S, int x, int q, T v) {
+        sm[x + S.s3 + q] = v;
+        if (S.dn && q < S.s3) *remote(x + S.s3 + S.P3 + q, S.rank - 1) = v;
+        if (S.up && q >= S.np - S.s3) *remote(x + (q - (S.np - S.s3)), S.rank + 1) = v;
+    }
+    // b + sum w x_n at own point q.  The links of the last point of a row, a column or the block are
+    // zero, so the ones "before" the first point are too (zeros in the plane before the block).
+    __device__ __forceinline__ T rest(const MGSlab& S, int x, int q) const {
+        const T* y = sm + x + S.s3 + q;
+        const T* w = sm + S.w + S.s3 + q;
+        return sm[S.b + q] + w[S.P4] * y[1] + w[S.P4 - 1] * y[-1] + w[2 * S.P4] * y[S.n1] +
+               w[2 * S.P4 - S.n1] * y[-S.n1] + w[3 * S.P4] * y[S.s3] + w[3 * S.P4 - S.s3] * y[-S.s3];
+    }
+    // x' = (1 - omega) x + omega D^-1 (b + sum w x_n) from copy cur into the other
+    __device__ __forceinline__ void sweep(const MGSlab& S, int& cur, T omega) {
+        const int x = S.x + cur * S.xlen;
+        cur ^= 1;
+#pragma unroll 2
+        for (int q = threadIdx.x; q < S.np; q += MGC_THREADS)
+            put(S, S.x + cur * S.xlen, q, (T(1) - omega) * sm[x + S.s3 + q] + omega * sm[S.w + S.s3 + q] * rest(S, x, q));
+        sync(S.spread);
+    }
+};
+
+template <typename T>
+__global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__ MGSub<T> sub,
+                                                       const double* __restrict__ minv,
+                                                       const long long* __restrict__ moff, T omega, T alpha, int nu1,
+                                                       int nu2, int mask_v) {
+    const int lg = sub.lg, size = 1 << lg, b = blockIdx.x >> lg, last = sub.nl - 1, tid = threadIdx.x;
+    const int m = sub.L[last].blk[b].n1 * sub.L[last].blk[b].n2 * sub.L[last].blk[b].n3;
+    double* db = reinterpret_cast<double*>(mgc_raw);
+    MGCluster<T> G{cg::this_cluster(), reinterpret_cast<T*>(mgc_raw) + m * (int)(sizeof(double) / sizeof(T))};
+    const int c = (int)G.cl.block_rank();
+    __shared__ int at[MGC_LEVELS + 1];
+    if (mask_v && b == sub.L[0].nb - 1) {        // the whole cluster: V frozen at zero
+        const MGBlockDesc& B = sub.L[0].blk[b];
+        const long long n = (long long)B.n1 * B.n2 * B.n3;
+        for (long long q = c * MGC_THREADS + tid; q < n; q += size * MGC_THREADS) sub.L[0].x[B.off + q] = T(0);
+        return;
+    }
+    if (tid == 0) {
+        int o = 0;
+        for (int l = 0; l <= last; l++) { at[l] = o; o += (int)mgc_len(sub.L[l].blk[b], lg, l < last); }
+    }
+    __syncthreads();
+    auto slab = [&](int l) { return MGSlab(sub.L[l].blk[b], lg, c, at[l]); };
+    // the links of every level (and the first one's right-hand side) on their way; x's copies start at
+    // zero: the halos beyond the grid are never written, zero like the links that point there
+#pragma unroll 1
+    for (int l = 0; l <= last; l++) {
+        const MGSlab S = slab(l);
+        if (l < last && S.np > 0) {
+            const MGLevelDev<T>& L = sub.L[l];
+            const long long first = L.blk[b].off + (long long)(S.z0 - 1) * S.s3;
+#pragma unroll 1
+            for (int q = tid; q < S.np + S.s3; q += MGC_THREADS) {
+                const bool in = S.z0 > 0 || q >= S.s3;
+                const long long t = in ? first + q : L.blk[b].off;
+                T* d = G.sm + S.w + q;
+                cp_async_elem(d, L.dinv + t, in);
+                cp_async_elem(d + S.P4, L.w1 + t, in);
+                cp_async_elem(d + 2 * S.P4, L.w2 + t, in);
+                cp_async_elem(d + 3 * S.P4, L.w3 + t, in);
+                if (l == 0 && q >= S.s3) cp_async_elem(G.sm + S.b + q - S.s3, L.b + t, true);
+            }
         }
-        __syncthreads();
-    };
-    const int last = tl.nl - 1;
+        if (l == 0) cp_async_commit();
+    }
+    cp_async_commit();
+#pragma unroll 1
+    for (int l = 0; l <= last; l++)
+        for (int q = tid; q < 2 * (int)mgc_xlen(sub.L[l].blk[b], lg); q += MGC_THREADS) G.sm[at[l] + q] = T(0);
+    // this warp's first row of the coarsest inverse: its loads are out of the way when the row is needed
+    const double* M = minv + moff[b];
+    const int lane = tid & 31, r0 = c * (MGC_THREADS / 32) + (tid >> 5);
+    double mrow[4];
+#pragma unroll
+    for (int e = 0; e < 4; e++) mrow[e] = r0 < m && lane + 32 * e < m ? M[(long long)r0 * m + lane + 32 * e] : 0.0;
+    asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    G.cl.sync();
+    // down: pre-smoothing from zero, and the residual summed over each 2x2x2 aggregate into the
+    // right-hand side of the CTA that holds the coarse point
+#pragma unroll 1
     for (int l = 0; l < last; l++) {
-        const MGLevelDev<T>& L = tl.L[l];
-        const MGBlockDesc& B = L.blk[b];
-        const long long n = npts(B);
-        T* x = L.x;
-        T* t = L.t;
-        for (long long q = threadIdx.x; q < n; q += blockDim.x) {
-            const long long p = B.off + q;
-            x[p] = masked ? T(0) : omega * L.dinv[p] * L.b[p];
+        if (l == 1) {                            // the copies of every thread
+            cp_async_wait_all();
+            __syncthreads();
         }
-        __syncthreads();
-        for (int s = 1; s < nu1; s++) {
-            sweep(L, x, t);
-            T* w = x; x = t; t = w;
+        const MGSlab S = slab(l), SC = slab(l + 1);
+        if (!S.spread && c != 0) break;
+#pragma unroll 2
+        for (int q = tid; q < S.np; q += MGC_THREADS) G.put(S, S.x, q, omega * G.sm[S.w + S.s3 + q] * G.sm[S.b + q]);
+        G.sync(S.spread);
+        int cur = 0;
+#pragma unroll 1
+        for (int s = 1; s < nu1; s++) G.sweep(S, cur, omega);
+        const int X = S.x + cur * S.xlen, R = S.x + (cur ^ 1) * S.xlen;   // the residual into the other copy
+#pragma unroll 2
+        for (int q = tid; q < S.np; q += MGC_THREADS) {
+            const T di = G.sm[S.w + S.s3 + q];
+            G.put(S, R, q, di != T(0) ? G.rest(S, X, q) - G.sm[X + S.s3 + q] * mgc_rcp(di) : T(0));
         }
-        xcur[l] = x;
-        tcur[l] = t;
-        // residual summed over each 2x2x2 aggregate -> the next level's right-hand side
-        const MGLevelDev<T>& C = tl.L[l + 1];
-        const MGBlockDesc& cb = C.blk[b];
-        const long long nc = npts(cb);
-        for (long long q = threadIdx.x; q < nc; q += blockDim.x) {
+        G.sync(S.spread);
+        const int n1 = S.n1, s3 = S.s3;
+        const int K0 = (S.z0 + 1) >> 1, K1 = (S.z0 + S.np / s3 + 1) >> 1;   // coarse planes whose first fine plane is here
+#pragma unroll 1
+        for (int q = tid; q < (K1 - K0) * SC.s3; q += MGC_THREADS) {
             int I, J, K;
-            mg_ijk(q, cb.n1, cb.n2, I, J, K);
-            T acc = T(0);
-            if (!masked)
-                for (int dk = 0; dk < 2; dk++) for (int dj = 0; dj < 2; dj++) for (int dd = 0; dd < 2; dd++) {
-                    const int i = 2 * I + dd, j = 2 * J + dj, k = 2 * K + dk;
-                    if (i >= B.n1 || j >= B.n2 || k >= B.n3) continue;
-                    const long long f = B.off + i + (long long)j * B.n1 + (long long)k * B.n1 * B.n2;
-                    if (L.dinv[f] == T(0)) continue;
-                    acc += L.b[f] - apply7(L, B, f, i, j, k, x);
-                }
-            C.b[cb.off + q] = acc;
+            mg_ijk(q, SC.n1, SC.n2, I, J, K);
+            K += K0;
+            const T* r = G.sm + R + s3 + (2 * K - S.z0) * s3 + 2 * J * n1 + 2 * I;
+            const bool i2 = 2 * I + 1 < S.n1, j2 = 2 * J + 1 < S.n2, k2 = 2 * K + 1 < S.n3;
+            T a = r[0];
+            if (i2) a += r[1];
+            if (j2) a += r[n1];
+            if (i2 && j2) a += r[n1 + 1];
+            if (k2) {
+                a += r[s3];
+                if (i2) a += r[s3 + 1];
+                if (j2) a += r[s3 + n1];
+                if (i2 && j2) a += r[s3 + n1 + 1];
+            }
+            const int owner = K / SC.P;
+            *G.remote(SC.b + (K - owner * SC.P) * SC.s3 + J * SC.n1 + I, owner) = a;
         }
-        __syncthreads();
+        G.sync(S.spread);
     }
-    {   // coarsest: x = Minv b (FP64 dense; pseudo-inverse for V)
-        const MGLevelDev<T>& C = tl.L[last];
-        const MGBlockDesc& B = C.blk[b];
-        const int m = (int)npts(B);
-        const double* M = minv + moff[b];
-        for (int r = threadIdx.x; r < m; r += blockDim.x) {
+    cp_async_wait_all();
+    G.cl.sync();
+    {   // coarsest: x = Minv b (FP64 dense; pseudo-inverse for V), b and x in the first CTA, a warp per row
+        // over the cluster: one SM's FP64 rate (2 FMA per clock) would take 4 us for 125 rows
+        const MGSlab S = slab(last);
+        const long long off = sub.L[last].blk[b].off;
+        const T* rb = G.remote(S.b, 0);
+        for (int q = tid; q < m; q += MGC_THREADS) db[q] = (double)(last == 0 ? sub.L[0].b[off + q] : rb[q]);
+        __syncthreads();
+        T* rx = last == 0 ? sub.L[0].x + off : G.remote(S.x + S.s3, 0);
+#pragma unroll 1
+        for (int r = r0; r < m; r += size * (MGC_THREADS / 32)) {
             double acc = 0.0;
-            if (!masked)
-                for (int c = 0; c < m; c++) acc += M[(long long)r * m + c] * (double)C.b[B.off + c];
-            C.x[B.off + r] = (T)acc;
+            int q = lane;
+            if (r == r0) {
+#pragma unroll
+                for (int e = 0; e < 4; e++, q += 32) acc += mrow[e] * (q < m ? db[q] : 0.0);
+            }
+#pragma unroll 1
+            for (; q < m; q += 32) acc += M[(long long)r * m + q] * db[q];
+            acc = qWarpSum(acc);
+            if (lane == 0) rx[r] = (T)acc;
         }
-        xcur[last] = C.x;
-        __syncthreads();
+        G.cl.sync();
     }
+    // up: the coarse correction and the post-smoothing.  Where the last sweep of a level left x: the copy
+    // alternates with every sweep after the first
+    const int down = (nu1 - 1) & 1, done = (nu1 - 1 + nu2) & 1;
+#pragma unroll 1
     for (int l = last - 1; l >= 0; l--) {
-        const MGLevelDev<T>& L = tl.L[l];
-        const MGLevelDev<T>& C = tl.L[l + 1];
-        const MGBlockDesc& B = L.blk[b];
-        const MGBlockDesc& cb = C.blk[b];
-        const long long n = npts(B);
-        T* x = xcur[l];
-        T* t = tcur[l];
-        const T* xc = xcur[l + 1];
-        for (long long q = threadIdx.x; q < n; q += blockDim.x) {
-            const long long p = B.off + q;
-            if (L.dinv[p] == T(0) || masked) { x[p] = T(0); continue; }
+        const MGSlab S = slab(l), SC = slab(l + 1);
+        if (!S.spread && c != 0) continue;
+        if (S.spread && !SC.spread && l + 1 < last) G.cl.sync();   // the first CTA has the coarse correction
+        const int X = S.x + down * S.xlen, XC = SC.x + (l + 1 == last ? 0 : done * SC.xlen) + SC.s3;
+#pragma unroll 2
+        for (int q = tid; q < S.np; q += MGC_THREADS) {
             int i, j, k;
-            mg_ijk(q, B.n1, B.n2, i, j, k);
-            x[p] += alpha * xc[cb.off + (i >> 1) + (long long)(j >> 1) * cb.n1 + (long long)(k >> 1) * cb.n1 * cb.n2];
+            mg_ijk(q, S.n1, S.n2, i, j, k);
+            const int K = (S.z0 + k) >> 1, owner = K / SC.P;
+            const T xc = *G.remote(XC + (K - owner * SC.P) * SC.s3 + (j >> 1) * SC.n1 + (i >> 1), owner);
+            G.put(S, X, q, G.sm[S.w + S.s3 + q] != T(0) ? G.sm[X + S.s3 + q] + alpha * xc : T(0));
         }
-        __syncthreads();
-        for (int s = 0; s < nu2; s++) {
-            sweep(L, x, t);
-            T* w = x; x = t; t = w;
-        }
-        xcur[l] = x;
+        G.sync(S.spread);
+        int cur = down;
+#pragma unroll 1
+        for (int s = 0; s < nu2; s++) G.sweep(S, cur, omega);
     }
-    // the level above reads the tail's top level from its x array
-    const MGLevelDev<T>& L0 = tl.L[0];
-    if (xcur[0] != L0.x) {
-        const MGBlockDesc& B = L0.blk[b];
-        const long long n = npts(B);
-        for (long long q = threadIdx.x; q < n; q += blockDim.x) L0.x[B.off + q] = xcur[0][B.off + q];
+    if (last > 0) {
+        const MGSlab S = slab(0);
+        const int x = S.x + done * S.xlen + S.s3;
+        const long long off = sub.L[0].blk[b].off + (long long)S.z0 * S.s3;
+        for (int q = tid; q < S.np; q += MGC_THREADS) sub.L[0].x[off + q] = G.sm[x + q];
     }
 }
 
@@ -697,7 +831,29 @@ static void mg0_prepare() {
     ATTR(0, 1); ATTR(1, 1); ATTR(2, 1); ATTR(3, 1);
     ATTR(0, 2); ATTR(1, 2); ATTR(2, 2); ATTR(3, 2);
 #undef ATTR
+    cudaFuncSetAttribute(mg_sub<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, MGC_SMEM);
+    cudaFuncSetAttribute(mg_sub<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     done.fetch_or(bit, std::memory_order_acq_rel);
+}
+
+// log2 of the CTAs of the coarse sub-cycle's clusters: 16 where the device can place such a cluster with the most
+// shared memory it may take, else 8
+template <typename T>
+static int mgc_size() {
+    mg0_prepare<T>();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(MGC_THREADS);
+    cfg.dynamicSmemBytes = MGC_SMEM;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {16, 1, 1};
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, mg_sub<T>, &cfg) == cudaSuccess && n >= 1) return 4;
+    cudaGetLastError();
+    return 3;
 }
 
 }  // namespace
@@ -981,6 +1137,38 @@ int QmsMG<T>::build(const QGrid& g, const QCoef<T>& c, const QStepPar<T>& P, T v
         for (T** q : ps)
             if (*q) *q += o;
     }
+    // the first level of each view's sub-cycle in one launch: as many levels as fit shared memory (and
+    // tail_points allows)
+    sub_lg = mgc_size<T>();
+    for (int qs = 0; qs < 3; qs++) {
+        const std::vector<MGLevelDev<T>>& v = qs == 0 ? lv : views[qs];
+        auto smem = [&](int lt) {
+            size_t most = 0;
+            for (int b = 0; b < v[lt].nb; b++) {
+                const MGBlockDesc& c = v.back().blk[b];
+                size_t bytes = (size_t)c.n1 * c.n2 * c.n3 * sizeof(double);
+                for (size_t l = lt; l < v.size(); l++)
+                    bytes += (size_t)mgc_len(v[l].blk[b], sub_lg, l + 1 < v.size()) * sizeof(T);
+                most = std::max(most, bytes);
+            }
+            return most;
+        };
+        auto fits = [&](int lt) {
+            for (int b = 0; b < v[lt].nb; b++) {
+                const MGBlockDesc& B = v[lt].blk[b];
+                const long long pts = (long long)B.n1 * B.n2 * B.n3;
+                if (tail_points < 0 || (tail_points > 0 && pts > tail_points)) return false;
+            }
+            return smem(lt) <= MGC_SMEM;
+        };
+        int lt = (int)v.size() - 1;
+        bool small = true;                       // the coarsest level is one CTA's
+        for (int b = 0; b < v[lt].nb; b++)
+            small = small && (long long)v[lt].blk[b].n1 * v[lt].blk[b].n2 * v[lt].blk[b].n3 <= MGC_LOCAL;
+        while (small && lt > 1 && (int)v.size() - (lt - 1) <= MGC_LEVELS && fits(lt - 1)) lt--;
+        sub_first[qs] = lt;
+        sub_smem[qs] = smem(lt);
+    }
     return 0;
 }
 
@@ -1051,28 +1239,26 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     // levels >= 1: nu_coarse sweeps on each side when set
     const int nuc1 = (QS == 2 && nu_v > 0) ? nu_v : (nu_coarse > 0 ? nu_coarse : nu1);
     const int nuc2 = (QS == 2 && nu_v > 0) ? nu_v : (nu_coarse > 0 ? nu_coarse : nu2);
-    // coarse tail: from level lt on, every level has at most tail_points points per block and
-    // the whole sub-cycle runs as one launch (one CTA per block)
-    auto maxpts = [](const MGLevelDev<T>& L) {
-        long long m = 0;
-        for (int q = 0; q < L.nb; q++) m = std::max(m, (long long)L.blk[q].n1 * L.blk[q].n2 * L.blk[q].n3);
-        return m;
-    };
-    int lt = nl - 1;
-    if (tail_points > 0)
-        while (lt > 1 && maxpts(lv[lt - 1]) <= tail_points && nl - (lt - 1) <= MG_TAIL_MAX_LEVELS) lt--;
+    // from level lt on the whole sub-cycle is one launch
+    const int lt = sub_first[QS];
     for (int l = 1; l < nl; l++) {
         MGLevelDev<T>& L = lv[l];
-        if (l == lt && tail_points > 0) {
-            MGTail<T> tl{};
-            tl.nl = nl - lt;
-            for (int q = 0; q < tl.nl; q++) tl.L[q] = lv[lt + q];
-            mg_tail<T><<<L.nb, 1024, 0, st>>>(tl, dminv, dmo, omega, alpha, nuc1, nuc2, mv);
-            launches++;
-            break;
-        }
-        if (l == nl - 1) {
-            mg_dense<<<L.nb, 256, 0, st>>>(L, dminv, dmo, L.b, L.x, mv);
+        if (l == lt) {
+            MGSub<T> sub{};
+            sub.nl = nl - lt;
+            sub.lg = sub_lg;
+            for (int q = 0; q < sub.nl; q++) sub.L[q] = lv[lt + q];
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(L.nb << sub_lg);
+            cfg.blockDim = dim3(MGC_THREADS);
+            cfg.dynamicSmemBytes = sub_smem[QS];
+            cfg.stream = st;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim = {1u << sub_lg, 1, 1};
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            cudaLaunchKernelEx(&cfg, mg_sub<T>, sub, (const double*)dminv, dmo, omega, alpha, nuc1, nuc2, mv);
             launches++;
             break;
         }

@@ -49,7 +49,11 @@ struct QmsMG {
     int nu1 = 2, nu2 = 2;
     int nu_coarse = 0;             // sweeps on each side on levels >= 1 (0: nu1 / nu2)
     int nu_v = 0;                  // sweeps on each side, every level, of a V-block cycle (0: as above)
-    long long tail_points = 4096;  // levels of at most this many points per block run as one launch (0: off)
+    long long tail_points = 0;     // most points per block of a level in the one-launch sub-cycle (0: as many as
+                                   // fit, < 0: the coarsest level alone)
+    int sub_first[3] = {};         // per view, that sub-cycle's first level and its shared memory
+    size_t sub_smem[3] = {};
+    int sub_lg = 3;                // log2 of the CTAs of its clusters
     T omega = T(0.8);
     T alpha = T(1);
     int min_coarse = 5;

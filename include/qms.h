@@ -107,8 +107,9 @@ typedef struct {
                                 (0: mg_sweeps) */
     int mg_v_sweeps;         /* sweeps on each side, on every level, of the block-triangular
                                 preconditioner's V-block cycle (0: as the A blocks) */
-    int mg_tail_points;      /* the coarse levels with at most this many points per block run their
-                                sub-cycle as one launch, one CTA per block (0: 4096; < 0: off) */
+    int mg_tail_points;      /* the last coarse levels run their sub-cycle as one launch, a cluster of CTAs per
+                                block: at most this many points per block of a level (0: as many as
+                                fit the chip; < 0: the coarsest level alone) */
     int extrapolate;         /* a transient step that follows steps with the same operator starts
                                 from an extrapolation of the last solutions instead of x_n, of
                                 this order at most (lower while fewer solutions are known):

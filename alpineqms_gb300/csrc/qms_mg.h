@@ -107,12 +107,15 @@ struct QmsMG {
 struct QmsRegions {
     int K = 0;                    // regions carrying a coarse degree of freedom (0: disabled)
     int total_entries = 0;        // V rows in all regions
-    int* ptr = nullptr;           // K+1 offsets into rows
+    int nchunk = 0;               // chunks of rows, each of one region
+    int* cptr = nullptr;          // nchunk+1 offsets into rows
+    int* rchunk = nullptr;        // K+1: first chunk of each region
     int* rows = nullptr;          // V rows (global unknown index) of each region, region by region
     int* rid = nullptr;           // region of each entry of rows
     double* Kp = nullptr;         // K x K pseudo-inverse, row-major
-    double* s = nullptr;          // K region sums / coarse solution
-    double* y = nullptr;
+    double* part = nullptr;       // chunk sums
+    double* y = nullptr;          // K coarse values
+    unsigned* counter = nullptr;  // chunks done
     std::string err;
     ~QmsRegions();
     void release();

@@ -585,12 +585,21 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
 //           shared memory, in k in registers -- no atomics, fixed order)
 // b is scaled pointwise by the row scaling of the outer system when bscale is
 // given; that scaling is the operator diagonal, formed here from the coefficients.
-// x_in is staged in shared memory by cp.async two planes ahead (four
-// components, +-1 halo in i and j); b is fetched into registers one plane ahead.
-// The kernels are instruction-bound at this arithmetic intensity, so the
-// Dirichlet tests are split into a per-thread (i, j) part and a per-plane k
-// part, row indices advance by one add per plane, and D^-1 is a fast
-// reciprocal in FP32 (a preconditioner needs no correctly rounded divide).
+// A stage of a march is x's plane k + 1 (all components, +-1 halo in i and j) and
+// the coefficients' plane k, two TMA copies on one mbarrier, issued two planes
+// ahead; b is fetched into registers one plane ahead.
+// The kernels are bound by instruction issue, not by bytes, so: what plane k - 1
+// contributes (x and three coefficients at the thread's own node) stays in
+// registers; the sweeps use x' = (1 - omega) x + omega D^-1 (b + sum w x_n) (the
+// restriction keeps the difference form, whose rounding scales with the variation
+// of x); on cubic cells (UNI) the links are the coefficients themselves, the factor
+// 1/h^2 left out where it cancels; the Dirichlet tests are split into a per-thread
+// (i, j) part and a per-plane k part, and Dirichlet points, zero in every vector
+// here, are not written; D^-1 is a fast reciprocal in FP32 (a preconditioner needs
+// no correctly rounded divide).
+// Before these (coefficients and x of three planes read from shared memory, links multiplied by 1/h^2,
+// two mbarriers per plane, one plane ahead), ms per run of steps: 96^3 202 -> 191, 128^3 244 -> 229,
+// moving plate 256^3 780 -> 717, 64^3 in FP64 411 -> 337.
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T mg_rcp(T d) {
@@ -616,7 +625,7 @@ template <> struct MG0Coef<float> { using type = __nv_bfloat16; };
 __device__ __forceinline__ float mg_cf(__nv_bfloat16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ double mg_cf(double v) { return v; }
 
-template <typename T, int KIND, int QS>
+template <typename T, int KIND, int QS, bool UNI>
 __global__ void __launch_bounds__(OTX * OTY, sizeof(T) == 4 ? QMS_STENCIL_MINB : 2)
 mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __restrict__ b, int scaled,
           const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap, T* __restrict__ xout,
@@ -627,9 +636,10 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* xsm = reinterpret_cast<T*>(smem_raw);                  // [4 slots][NQ][PLXY][PLX]
     CT* csm = reinterpret_cast<CT*>(smem_raw + 4 * TL::XSLOT * sizeof(T));   // [3 slots][NC][PLCY][CX]
-    __shared__ __align__(8) uint64_t xbar[4], cbar[3];
+    __shared__ __align__(8) uint64_t bar[4], pbar;
     __shared__ T red[KIND == 2 ? S::NQ : 1][OTY][OTX];
     constexpr bool STAGE = KIND != 0;
+    constexpr int NQ = S::NQ;
     const int tid = threadIdx.x + OTX * threadIdx.y;
     const int i0 = blockIdx.x * OTX + 1, j0 = blockIdx.y * OTY + 1, k0 = blockIdx.z * g.okb + 1;
     const int li = threadIdx.x + 1, lj = threadIdx.y + 1;
@@ -638,149 +648,162 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
     const int kend = min(k0 + g.okb - 1, g.Nz);
     const QPL L = qms_pl(g);
     const int cx = i0 - 1, cy = j0 - 2;
-    auto issue_x = [&](int kk) {
-        const int sl = kk & 3;
-        mbar_expect_tx(&xbar[sl], TL::XBYTES);
-        tma_load_4d(xsm + sl * TL::XSLOT, &xmap, cx, cy, kk - 1, 0, &xbar[sl]);
+    auto load_x = [&](int kk, uint64_t* on) { tma_load_4d(xsm + (kk & 3) * TL::XSLOT, &xmap, cx, cy, kk - 1, 0, on); };
+    auto load_c = [&](int kk, uint64_t* on) { tma_load_4d(csm + (kk % 3) * TL::CSLOT, &cmap, cx, cy, kk - 1, 0, on); };
+    // what plane k needs beyond the planes before it: x's plane k + 1 and the coefficients' plane k
+    auto issue = [&](int k) {
+        uint64_t* on = &bar[(k - k0) & 3];
+        mbar_expect_tx(on, (STAGE ? TL::XBYTES : 0u) + TL::CBYTES);
+        if (STAGE) load_x(k + 1, on);
+        load_c(k, on);
     };
-    auto issue_c = [&](int kk) {
-        const int sl = kk % 3;
-        mbar_expect_tx(&cbar[sl], TL::CBYTES);
-        tma_load_4d(csm + sl * TL::CSLOT, &cmap, cx, cy, kk - 1, 0, &cbar[sl]);
-    };
-    auto xpar = [&](int kk) { return (unsigned)(((kk - (k0 - 1)) >> 2) & 1); };
-    auto cpar = [&](int kk) { return (unsigned)(((kk - (k0 - 1)) / 3) & 1); };
     if (tid == 0) {
-        for (int q = 0; q < 4; q++) mbar_init(&xbar[q], 1);
-        for (int q = 0; q < 3; q++) mbar_init(&cbar[q], 1);
+        for (int q = 0; q < 4; q++) mbar_init(&bar[q], 1);
+        mbar_init(&pbar, 1);
         fence_mbar_init();
+        mbar_expect_tx(&pbar, (STAGE ? 2 * TL::XBYTES : 0u) + TL::CBYTES);
+        load_c(k0 - 1, &pbar);
         if (STAGE) {
-            issue_x(k0 - 1);
-            issue_x(k0);
-            issue_x(k0 + 1);
+            load_x(k0 - 1, &pbar);
+            load_x(k0, &pbar);
         }
-        issue_c(k0 - 1);
-        issue_c(k0);
+        issue(k0);
+        if (k0 + 1 <= kend) issue(k0 + 1);
     }
     __syncthreads();
-    bool ok = mbar_wait(&cbar[(k0 - 1) % 3], cpar(k0 - 1), err);
-    if (STAGE) ok = ok && mbar_wait(&xbar[(k0 - 1) & 3], xpar(k0 - 1), err) && mbar_wait(&xbar[k0 & 3], xpar(k0), err);
-    // per-thread parts of the component predicates (qFixX/Y/Z/V without their k terms)
-    const bool exX = inij && i <= g.xs, exY = inij && j <= g.ys;
+    bool ok = mbar_wait(&pbar, 0, err);
+    // the rows this thread solves: inside the grid and no Dirichlet row but for its k terms
     const bool fxA = i <= 2 || i >= g.Nx - 1, fyA = j <= 2 || j >= g.Ny - 1;
-    const bool fijX = fyA || i == 1 || i == g.xs;
-    const bool fijY = fxA || j == 1 || j == g.ys;
-    const bool fijZ = fxA || fyA;
-    const bool fijV = fxA || fyA || mask_v;
+    const bool aX = inij && !(fyA || i == 1 || i >= g.xs), aY = inij && !(fxA || j == 1 || j >= g.ys);
+    const bool aZ = inij && !(fxA || fyA), aV = aZ && !mask_v;
     // node offset at plane k0 (padded layout); block q's row is q * comp + node
     long long nd = inij ? qms_pl_node(g, L, i, j, k0) : 0;
     const long long plane = (long long)g.Ny * L.P;
     const T iscV = scaled ? T(1) / (T(1) + vshift) : T(1);
+    // 1/h^2 of the links, and the mass and b in their units
+    const T wx = UNI ? T(1) : P.idx2, wy = UNI ? T(1) : P.idy2, wz = UNI ? T(1) : P.idz2;
+    const T unit = UNI ? P.idx2 : T(1), iunit = UNI ? T(1) / P.idx2 : T(1), wm = P.idt * iunit;
     T acc[4] = {T(0), T(0), T(0), T(0)};
     // right-hand side of this thread's four rows, fetched one plane ahead so that the loads
-    // are in flight while the previous plane is computed.  The row scaling of the outer
-    // system is the operator's diagonal, which is this level's diagonal d divided by dscale
-    // (1 + vshift on V, 1 on A): it is formed from the staged coefficients, not read.
-    T bn0 = T(0), bn1 = T(0), bn2 = T(0), bn3 = T(0);
+    // are in flight while the previous plane is computed (KIND 3 has it in its tiles).  The row
+    // scaling of the outer system is the operator's diagonal, which is this level's diagonal d divided
+    // by dscale (1 + vshift on V, 1 on A): it is formed from the staged coefficients, not read.
+    T bn[4] = {T(0), T(0), T(0), T(0)};
     auto fetch_b = [&](int kk, long long n) {
+        if (KIND == 3) return;
         if (S::A) {
-            bn0 = exX ? __ldg(b + n) : T(0);
-            bn1 = exY ? __ldg(b + L.comp + n) : T(0);
-            bn2 = inij && kk <= g.zs ? __ldg(b + 2 * L.comp + n) : T(0);
+            bn[0] = aX ? __ldg(b + n) : T(0);
+            bn[1] = aY ? __ldg(b + L.comp + n) : T(0);
+            bn[2] = aZ && kk <= g.zs ? __ldg(b + 2 * L.comp + n) : T(0);
         }
-        if (S::V) bn3 = inij && !mask_v ? __ldg(b + 3 * L.comp + n) : T(0);
+        if (S::V) bn[3] = aV ? __ldg(b + 3 * L.comp + n) : T(0);
     };
     fetch_b(k0, nd);
-    for (int k = k0; k <= kend; k++) {
-        const T b0 = bn0, b1 = bn1, b2 = bn2, b3 = bn3;
-        if (k < kend) fetch_b(k + 1, nd + plane);
-        if (!__syncthreads_and(ok)) break;         // slots of plane k-2 free; uniform stop on a lost copy
-        if (tid == 0) {
-            fence_proxy_async();
-            if (STAGE && k + 2 <= kend + 1) issue_x(k + 2);
-            if (k < kend) issue_c(k + 1);
+#define CF(s, q, dj, di) ((T)mg_cf((s)[((q) - S::C0) * PLCY * TL::CX + (lj + (dj)) * TL::CX + li + (di)]))
+#define XS(s, q, dj, di) (s)[((q) - S::Q0) * PLXY * PLX + (lj + (dj)) * PLX + li + (di)]
+    // plane k - 1 at this node: x of every component and the coefficients of the links along k
+    T xm[4], xc[4], cm0 = T(0), cm1 = T(0), cm2 = T(0), sm2 = T(0);
+    if (ok) {
+        const T* p0 = xsm + ((k0 - 1) & 3) * TL::XSLOT;
+        const T* p1 = xsm + (k0 & 3) * TL::XSLOT;
+        const CT* cp = csm + ((k0 - 1) % 3) * TL::CSLOT;
+#pragma unroll
+        for (int q = S::Q0; q < S::Q0 + NQ; q++) {
+            xm[q] = STAGE ? XS(p0, q, 0, 0) : T(0);
+            xc[q] = STAGE ? XS(p1, q, 0, 0) : T(0);
         }
-        ok = mbar_wait(&cbar[k % 3], cpar(k), err);
-        if (STAGE) ok = ok && mbar_wait(&xbar[(k + 1) & 3], xpar(k + 1), err);
-        const T* xm = xsm + ((k - 1) & 3) * TL::XSLOT;
+        if (S::A) { cm0 = CF(cp, 0, 0, 0); cm1 = CF(cp, 1, 0, 0); cm2 = CF(cp, 2, 0, 0); }
+        if (S::V) sm2 = CF(cp, 5, 0, 0);
+    }
+    for (int k = k0; k <= kend; k++) {
+        T bv[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) bv[q] = bn[q];
+        if (k < kend) fetch_b(k + 1, nd + plane);
+        if (!__syncthreads_and(ok)) break;         // plane k-1's slots free; uniform stop on a lost copy
+        if (tid == 0 && k + 2 <= kend) {
+            fence_proxy_async();
+            issue(k + 2);
+        }
+        ok = mbar_wait(&bar[(k - k0) & 3], (unsigned)(((k - k0) >> 2) & 1), err);
         const T* x0 = xsm + (k & 3) * TL::XSLOT;
-        const T* xp = xsm + ((k + 1) & 3) * TL::XSLOT;
-        const CT* cprv = csm + ((k - 1) % 3) * TL::CSLOT;
-        const CT* ccur = csm + (k % 3) * TL::CSLOT;
+        const T* xq = xsm + ((k + 1) & 3) * TL::XSLOT;
+        const CT* cc = csm + (k % 3) * TL::CSLOT;
         const bool kfA = k <= 2 || k >= g.Nz - 1;       // k terms of qFixX / qFixY / qFixV
-        const bool kfZ = k == 1 || k == g.zs;           // k term of qFixZ
-#define CF(q, dk, dj, di) \
-    ((T)mg_cf((dk < 0 ? cprv : ccur)[((q) - S::C0) * PLCY * TL::CX + (lj + (dj)) * TL::CX + li + (di)]))
-#define XS(q, sl, dj, di) (sl)[((q) - S::Q0) * PLXY * PLX + (lj + (dj)) * PLX + li + (di)]
+        const bool kfZ = k == 1 || k >= g.zs;           // k term of qFixZ
         T r[4] = {T(0), T(0), T(0), T(0)};
         // one component: links (wxp, wxm, wyp, wym, wzp, wzm), extra diagonal
-        auto point = [&](int q, bool exists, bool fixed, long long row, T bq, T wxp, T wxm, T wyp, T wym, T wzp,
-                         T wzm, T dextra, T dscale, T isc) {
-            if (!exists) return;
-            if (fixed) {
-                if (KIND != 2) xout[row] = T(0);
-                return;
+        auto point = [&](int q, bool active, T wxp, T wxm, T wyp, T wym, T wzp, T wzm, T mass, T dscale, T isc) {
+            const T xp = STAGE ? XS(xq, q, 0, 0) : T(0);
+            if (active) {
+                const T wsum = ((wxp + wxm) + (wyp + wym)) + (wzp + wzm);
+                const T d = (wsum + mass) * dscale;
+                const long long row = q * L.comp + nd;
+                if (KIND == 0) {
+                    xout[row] = scaled ? omega * isc * bv[q] : omega * bv[q] * iunit * mg_rcp(d);
+                } else if (KIND == 2) {
+                    const T xs = xc[q];
+                    // difference form: d - sum(w) is the mass term, or the diagonal shift of V
+                    const T Ax = wxp * (xs - XS(x0, q, 0, 1)) + wxm * (xs - XS(x0, q, 0, -1)) +
+                                 wyp * (xs - XS(x0, q, 1, 0)) + wym * (xs - XS(x0, q, -1, 0)) + wzp * (xs - xp) +
+                                 wzm * (xs - xm[q]) + (d - wsum) * xs;
+                    r[q] = scaled ? unit * (bv[q] * d * isc - Ax) : bv[q] - unit * Ax;
+                } else {
+                    const T nb = wxp * XS(x0, q, 0, 1) + wxm * XS(x0, q, 0, -1) + wyp * XS(x0, q, 1, 0) +
+                                 wym * XS(x0, q, -1, 0) + wzp * xp + wzm * xm[q];
+                    // KIND 3: the staged values are b; x_1 = c b with c = omega isc, and the neighbours' sum
+                    // scales with it
+                    if (KIND == 3) {
+                        const T cq = omega * isc;
+                        xout[row] = cq * ((T(2) - omega) * xc[q] + omega * nb * mg_rcp(d));
+                    } else if (scaled) {
+                        xout[row] = (T(1) - omega) * xc[q] + omega * (isc * bv[q] + nb * mg_rcp(d));
+                    } else {
+                        xout[row] = (T(1) - omega) * xc[q] + omega * (iunit * bv[q] + nb) * mg_rcp(d);
+                    }
+                }
             }
-            const T d = (wxp + wxm + wyp + wym + wzp + wzm + dextra) * dscale;
-            const T bv = scaled ? bq * d * isc : bq;
-            if (KIND == 0) {
-                xout[row] = omega * bv * mg_rcp(d);
-                return;
-            }
-            const T xs = XS(q, x0, 0, 0);
-            // difference form (rounding scales with the variation of x): d - sum(w) is the mass
-            // term, or the diagonal shift of V
-            const T Axs = wxp * (xs - XS(q, x0, 0, 1)) + wxm * (xs - XS(q, x0, 0, -1)) + wyp * (xs - XS(q, x0, 1, 0)) +
-                          wym * (xs - XS(q, x0, -1, 0)) + wzp * (xs - XS(q, xp, 0, 0)) + wzm * (xs - XS(q, xm, 0, 0)) +
-                          (dextra * dscale + (wxp + wxm + wyp + wym + wzp + wzm) * (dscale - T(1))) * xs;
-            // KIND 3: the staged values are b; x_1 = c b with c = omega isc, and A x_1 = c A b
-            const T cq = KIND == 3 ? omega * isc : T(1);
-            const T xc = cq * xs, Ax = cq * Axs;
-            if (KIND == 2) r[q - S::Q0] = bv - Ax;
-            else xout[row] = xc + omega * (bv - Ax) * mg_rcp(d);
+            xm[q] = xc[q];
+            xc[q] = xp;
         };
         if constexpr (S::A) {
-        point(0, exX, fijX || kfA, nd, b0,
-              CF(0, 0, 0, 0) * P.idx2, CF(0, 0, 0, -1) * P.idx2, CF(2, 0, 0, 0) * P.idy2,
-              CF(2, 0, -1, 0) * P.idy2, CF(1, 0, 0, 0) * P.idz2, CF(1, -1, 0, 0) * P.idz2,
-              CF(3, 0, 0, 0) * P.idt, T(1), T(1));
-        point(1, exY, fijY || kfA, L.comp + nd, b1,
-              CF(2, 0, 0, 0) * P.idx2, CF(2, 0, 0, -1) * P.idx2, CF(1, 0, 0, 0) * P.idy2,
-              CF(1, 0, -1, 0) * P.idy2, CF(0, 0, 0, 0) * P.idz2, CF(0, -1, 0, 0) * P.idz2,
-              CF(4, 0, 0, 0) * P.idt, T(1), T(1));
-        point(2, inij && k <= g.zs, fijZ || kfZ, 2 * L.comp + nd, b2,
-              CF(1, 0, 0, 0) * P.idx2, CF(1, 0, 0, -1) * P.idx2, CF(0, 0, 0, 0) * P.idy2,
-              CF(0, 0, -1, 0) * P.idy2, CF(2, 0, 0, 0) * P.idz2, CF(2, -1, 0, 0) * P.idz2,
-              CF(5, 0, 0, 0) * P.idt, T(1), T(1));
+            const T c0 = CF(cc, 0, 0, 0), c1 = CF(cc, 1, 0, 0), c2 = CF(cc, 2, 0, 0);
+            const T c0i = CF(cc, 0, 0, -1), c1i = CF(cc, 1, 0, -1), c2i = CF(cc, 2, 0, -1);
+            const T c0j = CF(cc, 0, -1, 0), c1j = CF(cc, 1, -1, 0), c2j = CF(cc, 2, -1, 0);
+            point(0, aX && !kfA, c0 * wx, c0i * wx, c2 * wy, c2j * wy, c1 * wz, cm1 * wz, CF(cc, 3, 0, 0) * wm, T(1), T(1));
+            point(1, aY && !kfA, c2 * wx, c2i * wx, c1 * wy, c1j * wy, c0 * wz, cm0 * wz, CF(cc, 4, 0, 0) * wm, T(1), T(1));
+            point(2, aZ && !kfZ, c1 * wx, c1i * wx, c0 * wy, c0j * wy, c2 * wz, cm2 * wz, CF(cc, 5, 0, 0) * wm, T(1), T(1));
+            cm0 = c0; cm1 = c1; cm2 = c2;
         }
         if constexpr (S::V) {
-            const T fl = P.sigfloor;
-            point(3, inij, fijV || kfA, 3 * L.comp + nd, b3,
-                  fmax(CF(3, 0, 0, 0), fl) * P.idx2, fmax(CF(3, 0, 0, -1), fl) * P.idx2,
-                  fmax(CF(4, 0, 0, 0), fl) * P.idy2, fmax(CF(4, 0, -1, 0), fl) * P.idy2,
-                  fmax(CF(5, 0, 0, 0), fl) * P.idz2, fmax(CF(5, -1, 0, 0), fl) * P.idz2, T(0), T(1) + vshift, iscV);
+            const T fl = P.sigfloor, s2 = CF(cc, 5, 0, 0);
+            point(3, aV && !kfA, fmax(CF(cc, 3, 0, 0), fl) * wx, fmax(CF(cc, 3, 0, -1), fl) * wx,
+                  fmax(CF(cc, 4, 0, 0), fl) * wy, fmax(CF(cc, 4, -1, 0), fl) * wy, fmax(s2, fl) * wz,
+                  fmax(sm2, fl) * wz, T(0), T(1) + vshift, iscV);
+            sm2 = s2;
+            // a frozen V block: zero whatever the vector held
+            if (S::A && KIND != 2 && mask_v && inij) xout[3 * L.comp + nd] = T(0);
         }
-#undef CF
-#undef XS
         nd += plane;
         if (KIND == 2) {
 #pragma unroll
-            for (int q = 0; q < S::NQ; q++) {
-                r[q] += __shfl_xor_sync(0xffffffffu, r[q], 1);            // i pairs (2p+1, 2p+2)
-                red[q][threadIdx.y][threadIdx.x] = r[q];
+            for (int q = 0; q < NQ; q++) {
+                T v = r[q + S::Q0];
+                v += __shfl_xor_sync(0xffffffffu, v, 1);            // i pairs (2p+1, 2p+2)
+                red[q][threadIdx.y][threadIdx.x] = v;
             }
             __syncthreads();
             if (!(threadIdx.x & 1) && !(threadIdx.y & 1)) {
                 const bool first = ((k - k0) & 1) == 0;                    // k pairs (odd, even)
 #pragma unroll
-                for (int q = 0; q < S::NQ; q++) {
+                for (int q = 0; q < NQ; q++) {
                     const T v = red[q][threadIdx.y][threadIdx.x] + red[q][threadIdx.y + 1][threadIdx.x];
                     acc[q] = first ? v : acc[q] + v;
                 }
                 if (!first || k == kend) {
                     const int I = (i - 1) >> 1, J = (j - 1) >> 1, K = (k - 1) >> 1;
 #pragma unroll
-                    for (int q = 0; q < S::NQ; q++) {
+                    for (int q = 0; q < NQ; q++) {
                         const MGBlockDesc& cb = C.blk[q];
                         if (I < cb.n1 && J < cb.n2 && K < cb.n3)
                             bc[cb.off + I + (long long)J * cb.n1 + (long long)K * cb.n1 * cb.n2] =
@@ -790,6 +813,8 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
             }
         }
     }
+#undef CF
+#undef XS
 }
 
 // level 0: x += alpha P x_c on the active points (the Dirichlet points of every component,
@@ -832,7 +857,8 @@ static void mg0_prepare() {
     const unsigned long long bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return;
 #define ATTR(K, Q) \
-    cudaFuncSetAttribute(mg0_tiled<T, K, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg0_smem<T, K, Q>())
+    cudaFuncSetAttribute(mg0_tiled<T, K, Q, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg0_smem<T, K, Q>()); \
+    cudaFuncSetAttribute(mg0_tiled<T, K, Q, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg0_smem<T, K, Q>())
     ATTR(0, 0); ATTR(1, 0); ATTR(2, 0);
     ATTR(0, 1); ATTR(1, 1); ATTR(2, 1); ATTR(3, 1);
     ATTR(0, 2); ATTR(1, 2); ATTR(2, 2); ATTR(3, 2);
@@ -1206,10 +1232,15 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     struct Buf { T* p; const CUtensorMap* m; };
     // level-0 sweeps: KIND 0 writes XO from b; KIND 1 reads XI (tile copies) and writes XO;
     // KIND 2 reads XI and writes the level-1 right-hand side
+#define MG0U(KIND, XI, XO, BC, UNI)                                                                               \
+    mg0_tiled<T, KIND, QS, UNI><<<g0grid, g0block, mg0_smem<T, KIND, QS>(), st>>>(                                \
+        g0, P0, vshift0, omega, mv, b0, sc, *(XI).m, cmap, (XO), lv[1], (BC), err)
 #define MG0(KIND, XI, XO, BC)                                                                                     \
-    mg0_tiled<T, KIND, QS><<<g0grid, g0block, mg0_smem<T, KIND, QS>(), st>>>(g0, P0, vshift0, omega, mv, b0, sc,  \
-                                                                              *(XI).m, \
-                                                                       cmap, (XO), lv[1], (BC), err)
+    do {                                                                                                          \
+        if (cubic) MG0U(KIND, XI, XO, BC, true);                                                                  \
+        else MG0U(KIND, XI, XO, BC, false);                                                                       \
+    } while (0)
+    const bool cubic = P0.idx2 == P0.idy2 && P0.idx2 == P0.idz2;
     // level 0: nu1 + nu2 sweeps alternate between x0 and t0 (the prolongation is in place);
     // start in t0 when that count is even so that the last write lands in x0
     Buf x{x0, &x0map}, t{t0, &t0map};
@@ -1312,6 +1343,7 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
         launches++;
     }
 #undef MG0
+#undef MG0U
     return launches;
 }
 

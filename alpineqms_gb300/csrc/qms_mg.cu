@@ -33,6 +33,7 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <type_traits>
 #include <vector>
 
 namespace cg = cooperative_groups;
@@ -581,14 +582,15 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
 //           first sweep is x_1 = omega isc b pointwise (the diagonal cancels against
 //           the row scaling), so b's tile is staged in x_in's place and scaled on use
 //   KIND 2: b_c = sum over each 2x2x2 aggregate of (b - A x_in)  (restriction
-//           fused with the residual; pairs in i via lane shuffles, in j via
-//           shared memory, in k in registers -- no atomics, fixed order)
+//           fused with the residual; no atomics, fixed order)
 // b is scaled pointwise by the row scaling of the outer system when bscale is
 // given; that scaling is the operator diagonal, formed here from the coefficients.
 // A stage of a march is x's plane k + 1 (all components, +-1 halo in i and j) and
 // the coefficients' plane k, two TMA copies on one mbarrier, issued two planes
 // ahead; b is fetched into registers one plane ahead.
-// The kernels are bound by instruction issue, not by bytes, so: what plane k - 1
+// The kernels are bound by instruction issue, not by bytes, so: on grids of 1216 tiles or more a thread has
+// two rows (ROWS; j and j + 1: their common coefficients and x are read once, address arithmetic and
+// the plane's barrier shared), on smaller ones, where the march's latency counts, one; what plane k - 1
 // contributes (x and three coefficients at the thread's own node) stays in
 // registers; the sweeps use x' = (1 - omega) x + omega D^-1 (b + sum w x_n) (the
 // restriction keeps the difference form, whose rounding scales with the variation
@@ -599,7 +601,8 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
 // no correctly rounded divide).
 // Before these (coefficients and x of three planes read from shared memory, links multiplied by 1/h^2,
 // two mbarriers per plane, one plane ahead), ms per run of steps: 96^3 202 -> 191, 128^3 244 -> 229,
-// moving plate 256^3 780 -> 717, 64^3 in FP64 411 -> 337.
+// moving plate 256^3 780 -> 717, 64^3 in FP64 411 -> 337.  Two rows per thread instead of one: 96^3 191 ->
+// 186, 128^3 228 -> 219, 256^3 717 -> 690, but 48^3 161 -> 169 and FP64 as before (one row there).
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T mg_rcp(T d) {
@@ -625,8 +628,8 @@ template <> struct MG0Coef<float> { using type = __nv_bfloat16; };
 __device__ __forceinline__ float mg_cf(__nv_bfloat16 v) { return __bfloat162float(v); }
 __device__ __forceinline__ double mg_cf(double v) { return v; }
 
-template <typename T, int KIND, int QS, bool UNI>
-__global__ void __launch_bounds__(OTX * OTY, sizeof(T) == 4 ? QMS_STENCIL_MINB : 2)
+template <typename T, int KIND, int QS, bool UNI, int ROWS>
+__global__ void __launch_bounds__(OTX * OTY / ROWS, sizeof(T) == 4 ? (ROWS == 1 ? QMS_STENCIL_MINB : 6) : 2)
 mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __restrict__ b, int scaled,
           const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap, T* __restrict__ xout,
           MGLevelDev<T> C, T* __restrict__ bc, unsigned* __restrict__ err) {
@@ -637,14 +640,14 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
     T* xsm = reinterpret_cast<T*>(smem_raw);                  // [4 slots][NQ][PLXY][PLX]
     CT* csm = reinterpret_cast<CT*>(smem_raw + 4 * TL::XSLOT * sizeof(T));   // [3 slots][NC][PLCY][CX]
     __shared__ __align__(8) uint64_t bar[4], pbar;
-    __shared__ T red[KIND == 2 ? S::NQ : 1][OTY][OTX];
+    __shared__ T red[KIND == 2 && ROWS == 1 ? S::NQ : 1][OTY][OTX];
     constexpr bool STAGE = KIND != 0;
-    constexpr int NQ = S::NQ;
+    constexpr int NQ = S::NQ, Q0 = S::Q0, R = ROWS;
     const int tid = threadIdx.x + OTX * threadIdx.y;
     const int i0 = blockIdx.x * OTX + 1, j0 = blockIdx.y * OTY + 1, k0 = blockIdx.z * g.okb + 1;
-    const int li = threadIdx.x + 1, lj = threadIdx.y + 1;
-    const int i = i0 + threadIdx.x, j = j0 + threadIdx.y;
-    const bool inij = i <= g.Nx && j <= g.Ny;
+    // this thread's nodes: (i, j + r), r < R
+    const int li = threadIdx.x + 1, lj = threadIdx.y * R + 1;
+    const int i = i0 + threadIdx.x, j = j0 + threadIdx.y * R;
     const int kend = min(k0 + g.okb - 1, g.Nz);
     const QPL L = qms_pl(g);
     const int cx = i0 - 1, cy = j0 - 2;
@@ -673,52 +676,67 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
     __syncthreads();
     bool ok = mbar_wait(&pbar, 0, err);
     // the rows this thread solves: inside the grid and no Dirichlet row but for its k terms
-    const bool fxA = i <= 2 || i >= g.Nx - 1, fyA = j <= 2 || j >= g.Ny - 1;
-    const bool aX = inij && !(fyA || i == 1 || i >= g.xs), aY = inij && !(fxA || j == 1 || j >= g.ys);
-    const bool aZ = inij && !(fxA || fyA), aV = aZ && !mask_v;
-    // node offset at plane k0 (padded layout); block q's row is q * comp + node
-    long long nd = inij ? qms_pl_node(g, L, i, j, k0) : 0;
-    const long long plane = (long long)g.Ny * L.P;
+    const bool fxA = i <= 2 || i >= g.Nx - 1;
+    bool in[R], act[4][R];
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int jr = j + r;
+        const bool fyA = jr <= 2 || jr >= g.Ny - 1;
+        in[r] = i <= g.Nx && jr <= g.Ny;
+        act[0][r] = in[r] && !(fyA || i == 1 || i >= g.xs);
+        act[1][r] = in[r] && !(fxA || jr == 1 || jr >= g.ys);
+        act[2][r] = in[r] && !(fxA || fyA);
+        act[3][r] = act[2][r] && !mask_v;
+    }
+    // offset of node (i, j) at plane k in a block (32-bit: checked at creation); block q's row r is
+    // q * comp + nd + r * P
+    const int comp = (int)L.comp, plane = g.Ny * L.P, pitch = L.P;
+    int nd = ((k0 - 1) * g.Ny + (j - 1)) * L.P + i;
     const T iscV = scaled ? T(1) / (T(1) + vshift) : T(1);
     // 1/h^2 of the links, and the mass and b in their units
     const T wx = UNI ? T(1) : P.idx2, wy = UNI ? T(1) : P.idy2, wz = UNI ? T(1) : P.idz2;
     const T unit = UNI ? P.idx2 : T(1), iunit = UNI ? T(1) / P.idx2 : T(1), wm = P.idt * iunit;
     T acc[4] = {T(0), T(0), T(0), T(0)};
-    // right-hand side of this thread's four rows, fetched one plane ahead so that the loads
-    // are in flight while the previous plane is computed (KIND 3 has it in its tiles).  The row
-    // scaling of the outer system is the operator's diagonal, which is this level's diagonal d divided
-    // by dscale (1 + vshift on V, 1 on A): it is formed from the staged coefficients, not read.
-    T bn[4] = {T(0), T(0), T(0), T(0)};
-    auto fetch_b = [&](int kk, long long n) {
-        if (KIND == 3) return;
-        if (S::A) {
-            bn[0] = aX ? __ldg(b + n) : T(0);
-            bn[1] = aY ? __ldg(b + L.comp + n) : T(0);
-            bn[2] = aZ && kk <= g.zs ? __ldg(b + 2 * L.comp + n) : T(0);
-        }
-        if (S::V) bn[3] = aV ? __ldg(b + 3 * L.comp + n) : T(0);
+    // right-hand side of this thread's rows, fetched one plane ahead so that the loads are in flight
+    // while the previous plane is computed (KIND 3 has it in its tiles).  The row scaling of the outer
+    // system is the operator's diagonal, which is this level's diagonal d divided by dscale (1 + vshift
+    // on V, 1 on A): it is formed from the staged coefficients, not read.
+    T bn[4][R];
+    auto fetch_b = [&](int kk, int n) {
+#pragma unroll
+        for (int q = Q0; q < Q0 + NQ; q++)
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                bn[q][r] = KIND != 3 && act[q][r] && (q != 2 || kk <= g.zs) ? __ldg(b + q * comp + n + r * pitch) : T(0);
     };
     fetch_b(k0, nd);
 #define CF(s, q, dj, di) ((T)mg_cf((s)[((q) - S::C0) * PLCY * TL::CX + (lj + (dj)) * TL::CX + li + (di)]))
-#define XS(s, q, dj, di) (s)[((q) - S::Q0) * PLXY * PLX + (lj + (dj)) * PLX + li + (di)]
-    // plane k - 1 at this node: x of every component and the coefficients of the links along k
-    T xm[4], xc[4], cm0 = T(0), cm1 = T(0), cm2 = T(0), sm2 = T(0);
-    if (ok) {
+#define XS(s, q, dj, di) (s)[((q) - Q0) * PLXY * PLX + (lj + (dj)) * PLX + li + (di)]
+    // plane k - 1 at these nodes: x of every component and the coefficients of the links along k
+    T xm[4][R], xc[4][R], cm[6][R];
+    {
         const T* p0 = xsm + ((k0 - 1) & 3) * TL::XSLOT;
         const T* p1 = xsm + (k0 & 3) * TL::XSLOT;
         const CT* cp = csm + ((k0 - 1) % 3) * TL::CSLOT;
 #pragma unroll
-        for (int q = S::Q0; q < S::Q0 + NQ; q++) {
-            xm[q] = STAGE ? XS(p0, q, 0, 0) : T(0);
-            xc[q] = STAGE ? XS(p1, q, 0, 0) : T(0);
+        for (int r = 0; r < R; r++) {
+#pragma unroll
+            for (int q = Q0; q < Q0 + NQ; q++) {
+                xm[q][r] = STAGE && ok ? XS(p0, q, r, 0) : T(0);
+                xc[q][r] = STAGE && ok ? XS(p1, q, r, 0) : T(0);
+            }
+            if (S::A)
+#pragma unroll
+                for (int q = 0; q < 3; q++) cm[q][r] = ok ? CF(cp, q, r, 0) : T(0);
+            if (S::V) cm[5][r] = ok ? CF(cp, 5, r, 0) : T(0);
         }
-        if (S::A) { cm0 = CF(cp, 0, 0, 0); cm1 = CF(cp, 1, 0, 0); cm2 = CF(cp, 2, 0, 0); }
-        if (S::V) sm2 = CF(cp, 5, 0, 0);
     }
     for (int k = k0; k <= kend; k++) {
-        T bv[4];
+        T bv[4][R];
 #pragma unroll
-        for (int q = 0; q < 4; q++) bv[q] = bn[q];
+        for (int q = Q0; q < Q0 + NQ; q++)
+#pragma unroll
+            for (int r = 0; r < R; r++) bv[q][r] = bn[q][r];
         if (k < kend) fetch_b(k + 1, nd + plane);
         if (!__syncthreads_and(ok)) break;         // plane k-1's slots free; uniform stop on a lost copy
         if (tid == 0 && k + 2 <= kend) {
@@ -729,86 +747,128 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
         const T* x0 = xsm + (k & 3) * TL::XSLOT;
         const T* xq = xsm + ((k + 1) & 3) * TL::XSLOT;
         const CT* cc = csm + (k % 3) * TL::CSLOT;
-        const bool kfA = k <= 2 || k >= g.Nz - 1;       // k terms of qFixX / qFixY / qFixV
-        const bool kfZ = k == 1 || k >= g.zs;           // k term of qFixZ
-        T r[4] = {T(0), T(0), T(0), T(0)};
-        // one component: links (wxp, wxm, wyp, wym, wzp, wzm), extra diagonal
-        auto point = [&](int q, bool active, T wxp, T wxm, T wyp, T wym, T wzp, T wzm, T mass, T dscale, T isc) {
-            const T xp = STAGE ? XS(xq, q, 0, 0) : T(0);
-            if (active) {
+        const bool kA = k > 2 && k < g.Nz - 1;          // k terms of qFixX / qFixY / qFixV
+        const bool kZ = k > 1 && k < g.zs;              // k term of qFixZ
+        T res[4];                                       // KIND 2: this plane's residual, summed over the rows
+        // one component: links along x (cxp at the node, cxm before it), along y (ypr: row r, ym0: before
+        // row 0) and along z (zpr, zmr), extra diagonal
+        auto point = [&](int q, bool kok, const T (&cxp)[R], const T (&cxm)[R], const T (&cyp)[R], T cym,
+                         const T (&czp)[R], const T (&czm)[R], const T (&mass)[R], T dscale, T isc) {
+            T xp[R];
+            res[q] = T(0);
+#pragma unroll
+            for (int r = 0; r < R; r++) xp[r] = STAGE ? XS(xq, q, r, 0) : T(0);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                if (!(kok && act[q][r])) continue;
+                const T wxp = cxp[r] * wx, wxm = cxm[r] * wx, wyp = cyp[r] * wy, wym = (r > 0 ? cyp[r > 0 ? r - 1 : 0] : cym) * wy;
+                const T wzp = czp[r] * wz, wzm = czm[r] * wz;
                 const T wsum = ((wxp + wxm) + (wyp + wym)) + (wzp + wzm);
-                const T d = (wsum + mass) * dscale;
-                const long long row = q * L.comp + nd;
+                const T d = (wsum + mass[r]) * dscale;
+                const int row = q * comp + nd + r * pitch;
+                const T xs = xc[q][r];
                 if (KIND == 0) {
-                    xout[row] = scaled ? omega * isc * bv[q] : omega * bv[q] * iunit * mg_rcp(d);
-                } else if (KIND == 2) {
-                    const T xs = xc[q];
+                    xout[row] = scaled ? omega * isc * bv[q][r] : omega * bv[q][r] * iunit * mg_rcp(d);
+                    continue;
+                }
+                const T xip = XS(x0, q, r, 1), xim = XS(x0, q, r, -1);
+                const T xjp = r + 1 < R ? xc[q][r + 1 < R ? r + 1 : r] : XS(x0, q, R, 0);
+                const T xjm = r > 0 ? xc[q][r > 0 ? r - 1 : 0] : XS(x0, q, -1, 0);
+                if (KIND == 2) {
                     // difference form: d - sum(w) is the mass term, or the diagonal shift of V
-                    const T Ax = wxp * (xs - XS(x0, q, 0, 1)) + wxm * (xs - XS(x0, q, 0, -1)) +
-                                 wyp * (xs - XS(x0, q, 1, 0)) + wym * (xs - XS(x0, q, -1, 0)) + wzp * (xs - xp) +
-                                 wzm * (xs - xm[q]) + (d - wsum) * xs;
-                    r[q] = scaled ? unit * (bv[q] * d * isc - Ax) : bv[q] - unit * Ax;
+                    const T Ax = wxp * (xs - xip) + wxm * (xs - xim) + wyp * (xs - xjp) + wym * (xs - xjm) +
+                                 wzp * (xs - xp[r]) + wzm * (xs - xm[q][r]) + (d - wsum) * xs;
+                    res[q] += scaled ? unit * (bv[q][r] * d * isc - Ax) : bv[q][r] - unit * Ax;
                 } else {
-                    const T nb = wxp * XS(x0, q, 0, 1) + wxm * XS(x0, q, 0, -1) + wyp * XS(x0, q, 1, 0) +
-                                 wym * XS(x0, q, -1, 0) + wzp * xp + wzm * xm[q];
+                    const T nb = wxp * xip + wxm * xim + wyp * xjp + wym * xjm + wzp * xp[r] + wzm * xm[q][r];
                     // KIND 3: the staged values are b; x_1 = c b with c = omega isc, and the neighbours' sum
                     // scales with it
                     if (KIND == 3) {
                         const T cq = omega * isc;
-                        xout[row] = cq * ((T(2) - omega) * xc[q] + omega * nb * mg_rcp(d));
+                        xout[row] = cq * ((T(2) - omega) * xs + omega * nb * mg_rcp(d));
                     } else if (scaled) {
-                        xout[row] = (T(1) - omega) * xc[q] + omega * (isc * bv[q] + nb * mg_rcp(d));
+                        xout[row] = (T(1) - omega) * xs + omega * (isc * bv[q][r] + nb * mg_rcp(d));
                     } else {
-                        xout[row] = (T(1) - omega) * xc[q] + omega * (iunit * bv[q] + nb) * mg_rcp(d);
+                        xout[row] = (T(1) - omega) * xs + omega * (iunit * bv[q][r] + nb) * mg_rcp(d);
                     }
                 }
             }
-            xm[q] = xc[q];
-            xc[q] = xp;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                xm[q][r] = xc[q][r];
+                xc[q][r] = xp[r];
+            }
         };
         if constexpr (S::A) {
-            const T c0 = CF(cc, 0, 0, 0), c1 = CF(cc, 1, 0, 0), c2 = CF(cc, 2, 0, 0);
-            const T c0i = CF(cc, 0, 0, -1), c1i = CF(cc, 1, 0, -1), c2i = CF(cc, 2, 0, -1);
-            const T c0j = CF(cc, 0, -1, 0), c1j = CF(cc, 1, -1, 0), c2j = CF(cc, 2, -1, 0);
-            point(0, aX && !kfA, c0 * wx, c0i * wx, c2 * wy, c2j * wy, c1 * wz, cm1 * wz, CF(cc, 3, 0, 0) * wm, T(1), T(1));
-            point(1, aY && !kfA, c2 * wx, c2i * wx, c1 * wy, c1j * wy, c0 * wz, cm0 * wz, CF(cc, 4, 0, 0) * wm, T(1), T(1));
-            point(2, aZ && !kfZ, c1 * wx, c1i * wx, c0 * wy, c0j * wy, c2 * wz, cm2 * wz, CF(cc, 5, 0, 0) * wm, T(1), T(1));
-            cm0 = c0; cm1 = c1; cm2 = c2;
+            T c[3][R], ci[3][R], cj[3], mass[R];
+#pragma unroll
+            for (int q = 0; q < 3; q++) {
+                cj[q] = CF(cc, q, -1, 0);
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    c[q][r] = CF(cc, q, r, 0);
+                    ci[q][r] = CF(cc, q, r, -1);
+                }
+            }
+#pragma unroll
+            for (int r = 0; r < R; r++) mass[r] = CF(cc, 3, r, 0) * wm;
+            point(0, kA, c[0], ci[0], c[2], cj[2], c[1], cm[1], mass, T(1), T(1));
+#pragma unroll
+            for (int r = 0; r < R; r++) mass[r] = CF(cc, 4, r, 0) * wm;
+            point(1, kA, c[2], ci[2], c[1], cj[1], c[0], cm[0], mass, T(1), T(1));
+#pragma unroll
+            for (int r = 0; r < R; r++) mass[r] = CF(cc, 5, r, 0) * wm;
+            point(2, kZ, c[1], ci[1], c[0], cj[0], c[2], cm[2], mass, T(1), T(1));
+#pragma unroll
+            for (int q = 0; q < 3; q++)
+#pragma unroll
+                for (int r = 0; r < R; r++) cm[q][r] = c[q][r];
         }
         if constexpr (S::V) {
-            const T fl = P.sigfloor, s2 = CF(cc, 5, 0, 0);
-            point(3, aV && !kfA, fmax(CF(cc, 3, 0, 0), fl) * wx, fmax(CF(cc, 3, 0, -1), fl) * wx,
-                  fmax(CF(cc, 4, 0, 0), fl) * wy, fmax(CF(cc, 4, -1, 0), fl) * wy, fmax(s2, fl) * wz,
-                  fmax(sm2, fl) * wz, T(0), T(1) + vshift, iscV);
-            sm2 = s2;
-            // a frozen V block: zero whatever the vector held
-            if (S::A && KIND != 2 && mask_v && inij) xout[3 * L.comp + nd] = T(0);
+            const T fl = P.sigfloor;
+            T s0[R], s0i[R], s1[R], s2[R], s2m[R], none[R];
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                s0[r] = fmax(CF(cc, 3, r, 0), fl);
+                s0i[r] = fmax(CF(cc, 3, r, -1), fl);
+                s1[r] = fmax(CF(cc, 4, r, 0), fl);
+                s2[r] = fmax(CF(cc, 5, r, 0), fl);
+                s2m[r] = fmax(cm[5][r], fl);
+                none[r] = T(0);
+            }
+            point(3, kA, s0, s0i, s1, fmax(CF(cc, 4, -1, 0), fl), s2, s2m, none, T(1) + vshift, iscV);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                cm[5][r] = s2[r];
+                // a frozen V block: zero whatever the vector held
+                if (S::A && KIND != 2 && mask_v && in[r]) xout[3 * comp + nd + r * pitch] = T(0);
+            }
         }
         nd += plane;
         if (KIND == 2) {
+            // aggregates: i pairs (2p+1, 2p+2) a shuffle, j pairs this thread's two rows or, with one row per
+            // thread, shared memory, k pairs (odd, even) registers
+            const bool first = ((k - k0) & 1) == 0;
+            T v[4];
 #pragma unroll
-            for (int q = 0; q < NQ; q++) {
-                T v = r[q + S::Q0];
-                v += __shfl_xor_sync(0xffffffffu, v, 1);            // i pairs (2p+1, 2p+2)
-                red[q][threadIdx.y][threadIdx.x] = v;
+            for (int q = Q0; q < Q0 + NQ; q++) v[q] = res[q] + __shfl_xor_sync(0xffffffffu, res[q], 1);
+            if constexpr (R == 1) {
+#pragma unroll
+                for (int q = 0; q < NQ; q++) red[q][threadIdx.y][threadIdx.x] = v[q + Q0];
+                __syncthreads();
+#pragma unroll
+                for (int q = 0; q < NQ; q++) v[q + Q0] += red[q][threadIdx.y ^ 1][threadIdx.x];
             }
-            __syncthreads();
-            if (!(threadIdx.x & 1) && !(threadIdx.y & 1)) {
-                const bool first = ((k - k0) & 1) == 0;                    // k pairs (odd, even)
 #pragma unroll
-                for (int q = 0; q < NQ; q++) {
-                    const T v = red[q][threadIdx.y][threadIdx.x] + red[q][threadIdx.y + 1][threadIdx.x];
-                    acc[q] = first ? v : acc[q] + v;
-                }
-                if (!first || k == kend) {
-                    const int I = (i - 1) >> 1, J = (j - 1) >> 1, K = (k - 1) >> 1;
+            for (int q = Q0; q < Q0 + NQ; q++) acc[q] = first ? v[q] : acc[q] + v[q];
+            if (!(threadIdx.x & 1) && (R > 1 || !(threadIdx.y & 1)) && (!first || k == kend)) {
+                const int I = (i - 1) >> 1, J = (j - 1) >> 1, K = (k - 1) >> 1;
 #pragma unroll
-                    for (int q = 0; q < NQ; q++) {
-                        const MGBlockDesc& cb = C.blk[q];
-                        if (I < cb.n1 && J < cb.n2 && K < cb.n3)
-                            bc[cb.off + I + (long long)J * cb.n1 + (long long)K * cb.n1 * cb.n2] =
-                                (mask_v && q + S::Q0 == 3) ? T(0) : acc[q];
-                    }
+                for (int q = Q0; q < Q0 + NQ; q++) {
+                    const MGBlockDesc& cb = C.blk[q - Q0];
+                    if (I < cb.n1 && J < cb.n2 && K < cb.n3)
+                        bc[cb.off + I + (long long)J * cb.n1 + (long long)K * cb.n1 * cb.n2] =
+                            (mask_v && q == 3) ? T(0) : acc[q];
                 }
             }
         }
@@ -856,13 +916,24 @@ static void mg0_prepare() {
     cudaGetDevice(&dev);
     const unsigned long long bit = 1ull << (dev & 63);
     if (done.load(std::memory_order_acquire) & bit) return;
+    auto one = [](auto uni, auto rows) {
+        constexpr bool U = decltype(uni)::value;
+        constexpr int R = decltype(rows)::value;
 #define ATTR(K, Q) \
-    cudaFuncSetAttribute(mg0_tiled<T, K, Q, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg0_smem<T, K, Q>()); \
-    cudaFuncSetAttribute(mg0_tiled<T, K, Q, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg0_smem<T, K, Q>())
+    cudaFuncSetAttribute(mg0_tiled<T, K, Q, U, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg0_smem<T, K, Q>())
     ATTR(0, 0); ATTR(1, 0); ATTR(2, 0);
     ATTR(0, 1); ATTR(1, 1); ATTR(2, 1); ATTR(3, 1);
     ATTR(0, 2); ATTR(1, 2); ATTR(2, 2); ATTR(3, 2);
 #undef ATTR
+    };
+    using R1 = std::integral_constant<int, 1>;
+    one(std::true_type(), R1());
+    one(std::false_type(), R1());
+    if constexpr (sizeof(T) == 4) {
+        using R2 = std::integral_constant<int, 2>;
+        one(std::true_type(), R2());
+        one(std::false_type(), R2());
+    }
     cudaFuncSetAttribute(mg_sub<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, MGC_SMEM);
     cudaFuncSetAttribute(mg_sub<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     done.fetch_or(bit, std::memory_order_acq_rel);
@@ -1039,7 +1110,6 @@ int QmsMG<T>::build(const QGrid& g, const QCoef<T>& c, const QStepPar<T>& P, T v
         if (l == 1) CKM(cudaMemsetAsync(L.b, 0, bytes, st));
     }
     g0 = g; c0 = c; P0 = P; vshift0 = vshift;
-    g0block = dim3(OTX, OTY, 1);
     g0grid = qms_pl_tiles(g);
     const double ncut = vcut > 0.0 ? vcut : (sizeof(T) == 8 ? 1e-9 : 1e-5);
     mg_coarsen_fine<<<nblk(lv[1].total), 256, 0, st>>>(g, c, P, vshift, lv[0], lv[1], ncut);
@@ -1232,14 +1302,22 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     struct Buf { T* p; const CUtensorMap* m; };
     // level-0 sweeps: KIND 0 writes XO from b; KIND 1 reads XI (tile copies) and writes XO;
     // KIND 2 reads XI and writes the level-1 right-hand side
-#define MG0U(KIND, XI, XO, BC, UNI)                                                                               \
-    mg0_tiled<T, KIND, QS, UNI><<<g0grid, g0block, mg0_smem<T, KIND, QS>(), st>>>(                                \
+#define MG0U(KIND, XI, XO, BC, UNI, ROWS)                                                                         \
+    mg0_tiled<T, KIND, QS, UNI, ROWS><<<g0grid, dim3(OTX, OTY / ROWS), mg0_smem<T, KIND, QS>(), st>>>(            \
         g0, P0, vshift0, omega, mv, b0, sc, *(XI).m, cmap, (XO), lv[1], (BC), err)
 #define MG0(KIND, XI, XO, BC)                                                                                     \
     do {                                                                                                          \
-        if (cubic) MG0U(KIND, XI, XO, BC, true);                                                                  \
-        else MG0U(KIND, XI, XO, BC, false);                                                                       \
+        if (ROWS2 > 1 && two) {                                                                                   \
+            if (cubic) MG0U(KIND, XI, XO, BC, true, ROWS2);                                                       \
+            else MG0U(KIND, XI, XO, BC, false, ROWS2);                                                            \
+        } else {                                                                                                  \
+            if (cubic) MG0U(KIND, XI, XO, BC, true, 1);                                                           \
+            else MG0U(KIND, XI, XO, BC, false, 1);                                                                \
+        }                                                                                                         \
     } while (0)
+    // rows per thread: two on grids of many tiles (FP32)
+    constexpr int ROWS2 = sizeof(T) == 4 ? 2 : 1;
+    const bool two = (long long)g0grid.x * g0grid.y * g0grid.z >= QMS_CTA_TARGET;
     const bool cubic = P0.idx2 == P0.idy2 && P0.idx2 == P0.idz2;
     // level 0: nu1 + nu2 sweeps alternate between x0 and t0 (the prolongation is in place);
     // start in t0 when that count is even so that the last write lands in x0

@@ -73,7 +73,7 @@ struct QmsMG {
     // V solve drops eigenvalues of its operator scaled by those sums at or below vcut.
     // 0 = automatic: 1e-9 for an FP64 hierarchy, 1e-5 for FP32 (its cancellation noise is ~1e-7).
     double vcut = 0.0;
-    dim3 g0grid, g0block;
+    dim3 g0grid;
     std::string err;
 
     ~QmsMG();

@@ -1407,7 +1407,9 @@ int QmsSolver::step_graph(bool adv, const double v[3], const QStepStart& hs, boo
         if (e.k == k && e.xo == hs.xo && e.ls == hs.ls && e.wcalc == wcalc && e.dbx == dbx && e.v[0] == v[0] && e.v[1] == v[1] &&
             e.v[2] == v[2]) { G = &e; break; }
     if (!G) {
-        constexpr size_t kMax = 4;
+        // a run's counts fall from 13 to 3 or so: a cache of fewer than a run's graphs instantiated and
+        // destroyed them all again in the next one (a destruction now and then held a step up by 50 ms)
+        constexpr size_t kMax = 16;
         if (sgraphs.size() >= kMax) {
             size_t lru = 0;
             for (size_t q = 1; q < sgraphs.size(); q++) if (sgraphs[q].used < sgraphs[lru].used) lru = q;

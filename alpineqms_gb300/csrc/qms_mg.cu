@@ -23,6 +23,7 @@
 // back and processed by one launch through a packed block-descriptor table.
 // Smoother: weighted Jacobi.  Coarsest level: dense FP64 inverse per block.
 #include "qms_mg.h"
+#include "qms_pdl.cuh"
 #include "qms_pl.h"
 #include "qms_tile.cuh"
 
@@ -211,7 +212,7 @@ __global__ void mg_mask_links(MGLevelDev<T> C) {
 // A x at point t of block (n1, n2, n3) -- links to inactive points carry w = 0
 template <typename T>
 __device__ __forceinline__ T apply7(const MGLevelDev<T>& L, const MGBlockDesc& B, long long t, int i, int j, int k,
-                                    const T* __restrict__ x) {
+                                    const T* x) {
     const long long s2 = B.n1, s3 = (long long)B.n1 * B.n2;
     T acc = L.dg[t] * x[t];
     if (i > 0) acc -= L.w1[t - 1] * x[t - 1];
@@ -224,14 +225,13 @@ __device__ __forceinline__ T apply7(const MGLevelDev<T>& L, const MGBlockDesc& B
 }
 
 // ------------------------------------------------------------------ smoother
-// first sweep from a zero guess: x = omega D^-1 b   (b scaled by bscale on level 0)
+// first sweep from a zero guess: x = omega D^-1 b
 template <typename T>
-__global__ void mg_smooth0(MGLevelDev<T> L, const T* __restrict__ b, const float* __restrict__ bscale, T omega,
-                           T* __restrict__ x, int mask_v) {
+__global__ void mg_smooth0(MGLevelDev<T> L, const T* b, T omega, T* x, int mask_v) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (t >= L.total) return;
-    T bv = b[t];
-    if (bscale) bv *= (T)bscale[t];
+    const T bv = b[t];
     T di = L.dinv[t];
     if (mask_v && t >= L.blk[L.nb - 1].off) di = T(0);
     x[t] = omega * di * bv;
@@ -239,9 +239,9 @@ __global__ void mg_smooth0(MGLevelDev<T> L, const T* __restrict__ b, const float
 
 // x_out = x_in + omega D^-1 (b - A x_in)
 template <typename T>
-__global__ void mg_smooth(MGLevelDev<T> L, const T* __restrict__ b, const float* __restrict__ bscale, T omega,
-                          const T* __restrict__ xin, T* __restrict__ xout, int mask_v) {
+__global__ void mg_smooth(MGLevelDev<T> L, const T* b, T omega, const T* xin, T* xout, int mask_v) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (t >= L.total) return;
     T di = L.dinv[t];
     if (mask_v && t >= L.blk[L.nb - 1].off) di = T(0);
@@ -251,8 +251,7 @@ __global__ void mg_smooth(MGLevelDev<T> L, const T* __restrict__ b, const float*
     long long q = t - B.off;
     int i, j, k;
     mg_ijk(q, B.n1, B.n2, i, j, k);
-    T bv = b[t];
-    if (bscale) bv *= (T)bscale[t];
+    const T bv = b[t];
     xout[t] = xin[t] + omega * di * (bv - apply7(L, B, t, i, j, k, xin));
 }
 
@@ -264,9 +263,8 @@ __global__ void mg_smooth(MGLevelDev<T> L, const T* __restrict__ b, const float*
 #define MGR_Y 4
 #define MGR_Z 2
 template <typename T>
-__global__ void __launch_bounds__(MGR_X * MGR_Y * MGR_Z) mg_restrict(MGLevelDev<T> F, const T* __restrict__ bf,
-                                                                    const T* __restrict__ xf, MGLevelDev<T> C,
-                                                                    T* __restrict__ bc, int mask_v, int xtiles) {
+__global__ void __launch_bounds__(MGR_X * MGR_Y * MGR_Z) mg_restrict(MGLevelDev<T> F, const T* bf, const T* xf,
+                                                                    MGLevelDev<T> C, T* bc, int mask_v, int xtiles) {
     __shared__ T sh[MGR_Z][MGR_Y][MGR_X];
     const int b = blockIdx.x / xtiles;
     const MGBlockDesc& fb = F.blk[b];
@@ -274,6 +272,7 @@ __global__ void __launch_bounds__(MGR_X * MGR_Y * MGR_Z) mg_restrict(MGLevelDev<
     const int i = (blockIdx.x - b * xtiles) * MGR_X + threadIdx.x, j = blockIdx.y * MGR_Y + threadIdx.y;
     const int k = blockIdx.z * MGR_Z + threadIdx.z;
     T r = T(0);
+    pdl_wait();
     if (i < fb.n1 && j < fb.n2 && k < fb.n3) {
         const long long f = fb.off + i + (long long)j * fb.n1 + (long long)k * fb.n1 * fb.n2;
         if (F.dinv[f] != T(0)) r = bf[f] - apply7(F, fb, f, i, j, k, xf);
@@ -291,8 +290,9 @@ __global__ void __launch_bounds__(MGR_X * MGR_Y * MGR_Z) mg_restrict(MGLevelDev<
 
 // x_out = x_in + alpha x_c(aggregate of f) on active fine points (x_out may alias x_in)
 template <typename T>
-__global__ void mg_prolong(MGLevelDev<T> F, const T* xin, T* xf, MGLevelDev<T> C, const T* __restrict__ xc, T alpha) {
+__global__ void mg_prolong(MGLevelDev<T> F, const T* xin, T* xf, MGLevelDev<T> C, const T* xc, T alpha) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (t >= F.total) return;
     if (F.dinv[t] == T(0)) { xf[t] = T(0); return; }
     const int b = find_block(F, t);
@@ -424,6 +424,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
     const int c = (int)G.cl.block_rank();
     __shared__ int at[MGC_LEVELS + 1];
     if (mask_v && b == sub.L[0].nb - 1) {        // the whole cluster: V frozen at zero
+        pdl_wait();
         const MGBlockDesc& B = sub.L[0].blk[b];
         const long long n = (long long)B.n1 * B.n2 * B.n3;
         for (long long q = c * MGC_THREADS + tid; q < n; q += size * MGC_THREADS) sub.L[0].x[B.off + q] = T(0);
@@ -435,7 +436,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
     }
     __syncthreads();
     auto slab = [&](int l) { return MGSlab(sub.L[l].blk[b], lg, c, at[l]); };
-    // the links of every level (and the first one's right-hand side) on their way; x's copies start at
+    // the links of every level on their way; x's copies start at
     // zero: the halos beyond the grid are never written, zero like the links that point there
 #pragma unroll 1
     for (int l = 0; l <= last; l++) {
@@ -452,7 +453,6 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
                 cp_async_elem(d + S.P4, L.w1 + t, in);
                 cp_async_elem(d + 2 * S.P4, L.w2 + t, in);
                 cp_async_elem(d + 3 * S.P4, L.w3 + t, in);
-                if (l == 0 && q >= S.s3) cp_async_elem(G.sm + S.b + q - S.s3, L.b + t, true);
             }
         }
         if (l == 0) cp_async_commit();
@@ -467,6 +467,13 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
     double mrow[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) mrow[e] = r0 < m && lane + 32 * e < m ? M[(long long)r0 * m + lane + 32 * e] : 0.0;
+    // the links are the geometry's; the first level's right-hand side is the kernel's before this one
+    pdl_wait();
+    if (last > 0) {
+        const MGSlab S = slab(0);
+        const long long off = sub.L[0].blk[b].off + (long long)S.z0 * S.s3;
+        for (int q = tid; q < S.np; q += MGC_THREADS) G.sm[S.b + q] = sub.L[0].b[off + q];
+    }
     asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     G.cl.sync();
     // down: pre-smoothing from zero, and the residual summed over each 2x2x2 aggregate into the
@@ -630,9 +637,9 @@ __device__ __forceinline__ double mg_cf(double v) { return v; }
 
 template <typename T, int KIND, int QS, bool UNI, int ROWS>
 __global__ void __launch_bounds__(OTX * OTY / ROWS, sizeof(T) == 4 ? (ROWS == 1 ? QMS_STENCIL_MINB : 6) : 2)
-mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __restrict__ b, int scaled,
-          const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap, T* __restrict__ xout,
-          MGLevelDev<T> C, T* __restrict__ bc, unsigned* __restrict__ err) {
+mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* b, int scaled,
+          const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap, T* xout,
+          MGLevelDev<T> C, T* bc, unsigned* err) {
     using S = MG0Set<QS>;
     using CT = typename MG0Coef<T>::type;
     using TL = PLTiles<T, S::NQ, S::NC, CT>;
@@ -665,13 +672,16 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
         mbar_init(&pbar, 1);
         fence_mbar_init();
         mbar_expect_tx(&pbar, (STAGE ? 2 * TL::XBYTES : 0u) + TL::CBYTES);
-        load_c(k0 - 1, &pbar);
+        load_c(k0 - 1, &pbar);                  // (the coefficients are the geometry's)
+        pdl_wait();
         if (STAGE) {
             load_x(k0 - 1, &pbar);
             load_x(k0, &pbar);
         }
         issue(k0);
         if (k0 + 1 <= kend) issue(k0 + 1);
+    } else {
+        pdl_wait();
     }
     __syncthreads();
     bool ok = mbar_wait(&pbar, 0, err);
@@ -707,7 +717,7 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
         for (int q = Q0; q < Q0 + NQ; q++)
 #pragma unroll
             for (int r = 0; r < R; r++)
-                bn[q][r] = KIND != 3 && act[q][r] && (q != 2 || kk <= g.zs) ? __ldg(b + q * comp + n + r * pitch) : T(0);
+                bn[q][r] = KIND != 3 && act[q][r] && (q != 2 || kk <= g.zs) ? b[q * comp + n + r * pitch] : T(0);
     };
     fetch_b(k0, nd);
 #define CF(s, q, dj, di) ((T)mg_cf((s)[((q) - S::C0) * PLCY * TL::CX + (lj + (dj)) * TL::CX + li + (di)]))
@@ -885,13 +895,14 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* __rest
 #define MGP_X 16
 #define MGP_Y 16
 template <typename T, int QS>
-__global__ void __launch_bounds__(MGP_X * MGP_Y) mg0_prolong(QGrid g, int mask_v, T* __restrict__ x, MGLevelDev<T> C,
-                                                            const T* __restrict__ xc, T alpha) {
+__global__ void __launch_bounds__(MGP_X * MGP_Y) mg0_prolong(QGrid g, int mask_v, T* x, MGLevelDev<T> C, const T* xc,
+                                                            T alpha) {
     using S = MG0Set<QS>;
     constexpr int W = 16 / (int)sizeof(T);
     struct alignas(16) Packet { T v[W]; };
     const QPL L = qms_pl(g);
     const int c0 = (blockIdx.x * MGP_X + threadIdx.x) * W, j = blockIdx.y * MGP_Y + threadIdx.y + 1, k = blockIdx.z + 1;
+    pdl_wait();
     if (c0 >= g.xs || j > g.ys) return;                       // i >= xs, j > ys: Dirichlet rows only
     const int J = (j - 1) >> 1, K = (k - 1) >> 1, I0 = (c0 - 1) >> 1;
     const bool fy = j <= 2 || j >= g.Ny - 1, fz = k <= 2 || k >= g.Nz - 1;
@@ -905,7 +916,7 @@ __global__ void __launch_bounds__(MGP_X * MGP_Y) mg0_prolong(QGrid g, int mask_v
         Packet v = *xp;
         T c[W / 2 + 1];
 #pragma unroll
-        for (int e = 0; e <= W / 2; e++) c[e] = I0 + e >= 0 && I0 + e < cb.n1 ? __ldg(cr + I0 + e) : T(0);
+        for (int e = 0; e <= W / 2; e++) c[e] = I0 + e >= 0 && I0 + e < cb.n1 ? cr[I0 + e] : T(0);
 #pragma unroll
         for (int e = 0; e < W; e++)
             if (c0 + e >= lo && c0 + e <= hi) v.v[e] += alpha * c[(e + 1) / 2];
@@ -1319,8 +1330,8 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     // level-0 sweeps: KIND 0 writes XO from b; KIND 1 reads XI (tile copies) and writes XO;
     // KIND 2 reads XI and writes the level-1 right-hand side
 #define MG0U(KIND, XI, XO, BC, UNI, ROWS)                                                                         \
-    mg0_tiled<T, KIND, QS, UNI, ROWS><<<g0grid, dim3(OTX, OTY / ROWS), mg0_smem<T, KIND, QS>(), st>>>(            \
-        g0, P0, vshift0, omega, mv, b0, sc, *(XI).m, cmap, (XO), lv[1], (BC), err)
+    pdl_launch(mg0_tiled<T, KIND, QS, UNI, ROWS>, g0grid, dim3(OTX, OTY / ROWS), mg0_smem<T, KIND, QS>(), st, 0,  \
+               g0, P0, vshift0, omega, mv, b0, sc, *(XI).m, cmap, (XO), lv[1], (BC), err)
 #define MG0(KIND, XI, XO, BC)                                                                                     \
     do {                                                                                                          \
         if (ROWS2 > 1 && two) {                                                                                   \
@@ -1379,26 +1390,17 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
             sub.nl = nl - lt;
             sub.lg = sub_lg;
             for (int q = 0; q < sub.nl; q++) sub.L[q] = lv[lt + q];
-            cudaLaunchConfig_t cfg = {};
-            cfg.gridDim = dim3(L.nb << sub_lg);
-            cfg.blockDim = dim3(MGC_THREADS);
-            cfg.dynamicSmemBytes = sub_smem[QS];
-            cfg.stream = st;
-            cudaLaunchAttribute at[1];
-            at[0].id = cudaLaunchAttributeClusterDimension;
-            at[0].val.clusterDim = {1u << sub_lg, 1, 1};
-            cfg.attrs = at;
-            cfg.numAttrs = 1;
-            cudaLaunchKernelEx(&cfg, mg_sub<T>, sub, (const double*)dminv, dmo, omega, alpha, nuc1, nuc2, mv);
+            pdl_launch(mg_sub<T>, dim3(L.nb << sub_lg), dim3(MGC_THREADS), sub_smem[QS], st, 1u << sub_lg, sub, dminv, dmo,
+                       omega, alpha, nuc1, nuc2, mv);
             launches++;
             break;
         }
         T* xl = L.x;
         T* tl = L.t;
-        mg_smooth0<<<nblk(L.total), 256, 0, st>>>(L, L.b, nullptr, omega, xl, mv);
+        pdl_launch(mg_smooth0<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, mv);
         launches++;
         for (int s = 1; s < nuc1; s++) {
-            mg_smooth<<<nblk(L.total), 256, 0, st>>>(L, L.b, nullptr, omega, xl, tl, mv);
+            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl, mv);
             std::swap(xl, tl);
             launches++;
         }
@@ -1411,18 +1413,18 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
             e3 = std::max(e3, L.blk[q].n3);
         }
         const int xt = (e1 + MGR_X - 1) / MGR_X;
-        mg_restrict<<<dim3(L.nb * xt, (e2 + MGR_Y - 1) / MGR_Y, (e3 + MGR_Z - 1) / MGR_Z), dim3(MGR_X, MGR_Y, MGR_Z),
-                      0, st>>>(L, L.b, xl, lv[l + 1], lv[l + 1].b, mv, xt);
+        pdl_launch(mg_restrict<T>, dim3(L.nb * xt, (e2 + MGR_Y - 1) / MGR_Y, (e3 + MGR_Z - 1) / MGR_Z),
+                   dim3(MGR_X, MGR_Y, MGR_Z), 0, st, 0, L, L.b, xl, lv[l + 1], lv[l + 1].b, mv, xt);
         launches++;
     }
     for (int l = lt - 1; l >= 1; l--) {
         MGLevelDev<T>& L = lv[l];
         T* xl = L.x;
         T* tl = L.t;
-        mg_prolong<<<nblk(L.total), 256, 0, st>>>(L, xl, xl, lv[l + 1], lv[l + 1].x, alpha);
+        pdl_launch(mg_prolong<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, xl, xl, lv[l + 1], lv[l + 1].x, alpha);
         launches++;
         for (int s = 0; s < nuc2; s++) {
-            mg_smooth<<<nblk(L.total), 256, 0, st>>>(L, L.b, nullptr, omega, xl, tl, mv);
+            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl, mv);
             std::swap(xl, tl);
             launches++;
         }
@@ -1430,8 +1432,8 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
         L.t = tl;
     }
     const int cols = MGP_X * 16 / (int)sizeof(T);
-    mg0_prolong<T, QS><<<dim3((g0.xs + cols - 1) / cols, (g0.ys + MGP_Y - 1) / MGP_Y, g0.Nz), dim3(MGP_X, MGP_Y), 0,
-                         st>>>(g0, mv, x.p, lv[1], lv[1].x, alpha);
+    pdl_launch(mg0_prolong<T, QS>, dim3((g0.xs + cols - 1) / cols, (g0.ys + MGP_Y - 1) / MGP_Y, g0.Nz),
+               dim3(MGP_X, MGP_Y), 0, st, 0, g0, mv, x.p, lv[1], lv[1].x, alpha);
     launches++;
     for (int s = 0; s < n2; s++) {
         sweep(x, t.p);
@@ -1458,13 +1460,14 @@ namespace {
 #define QMS_REGION_CHUNK 1024
 template <typename T>
 __global__ void __launch_bounds__(256) qk_region_solve(const int* __restrict__ cptr, const int* __restrict__ rchunk,
-                                                      const int* __restrict__ rows, const T* __restrict__ b,
+                                                      const int* __restrict__ rows, const T* b,
                                                       const float* __restrict__ bscale, double* part, int K,
-                                                      const double* __restrict__ Kp, double* __restrict__ y,
+                                                      const double* __restrict__ Kp, double* y,
                                                       unsigned* counter) {
     __shared__ double sh[32], s[QMS_REGION_MAX];
     __shared__ bool lastcta;
     double acc = 0.0;
+    pdl_wait();
     for (int e = cptr[blockIdx.x] + threadIdx.x; e < cptr[blockIdx.x + 1]; e += blockDim.x) {
         const int row = rows[e];
         acc += (double)b[row] * (bscale ? (double)bscale[row] : 1.0);
@@ -1479,13 +1482,14 @@ __global__ void __launch_bounds__(256) qk_region_solve(const int* __restrict__ c
     __syncthreads();
     if (!lastcta) return;
     __threadfence();
-    for (int r = threadIdx.x; r < K; r += blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    for (int r = threadIdx.x >> 5; r < K; r += blockDim.x >> 5) {
         double t = 0.0;
-        for (int q = rchunk[r]; q < rchunk[r + 1]; q++) t += __ldcg(part + q);
-        s[r] = t;
+        for (int q = rchunk[r] + lane; q < rchunk[r + 1]; q += 32) t += __ldcg(part + q);
+        t = qWarpSum(t);
+        if (lane == 0) s[r] = t;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
     for (int r = threadIdx.x >> 5; r < K; r += blockDim.x >> 5) {
         double t = 0.0;
         for (int q = lane; q < K; q += 32) t += Kp[(long long)r * K + q] * s[q];
@@ -1497,8 +1501,9 @@ __global__ void __launch_bounds__(256) qk_region_solve(const int* __restrict__ c
 // z[row] += y[region of row]
 template <typename T>
 __global__ void qk_region_scatter(int total, const int* __restrict__ rows, const int* __restrict__ rid,
-                                  const double* __restrict__ y, T* __restrict__ z) {
+                                  const double* y, T* z) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
     if (e < total) z[rows[e]] += (T)y[rid[e]];
 }
 
@@ -1724,9 +1729,10 @@ int QmsRegions::build(const QGrid& g, const uint8_t* slots, const double* rows6,
 template <typename T>
 void QmsRegions::apply(const T* b, const float* bscale, T* z, cudaStream_t st, long long& launches) {
     if (K == 0) return;
-    qk_region_solve<T><<<nchunk, 256, 0, st>>>(cptr, rchunk, rows, b, bscale, part, K, Kp, y, counter);
+    pdl_launch(qk_region_solve<T>, dim3(nchunk), dim3(256), 0, st, 0, cptr, rchunk, rows, b, bscale, part, K, Kp, y,
+               counter);
     const int total = total_entries;
-    qk_region_scatter<T><<<(total + 255) / 256, 256, 0, st>>>(total, rows, rid, y, z);
+    pdl_launch(qk_region_scatter<T>, dim3((total + 255) / 256), dim3(256), 0, st, 0, total, rows, rid, y, z);
     launches += 2;
 }
 template void QmsRegions::apply<float>(const float*, const float*, float*, cudaStream_t, long long&);

@@ -11,6 +11,7 @@
 #include "qms_internal.h"
 #include "qms_df.cuh"
 #include "qms_op_rows.cuh"
+#include "qms_pdl.cuh"
 #include "qms_pl.h"
 #include "qms_tile.cuh"
 
@@ -122,8 +123,7 @@ __device__ __forceinline__ T pl_div(T a, T d) {
 template <typename T, int VM, int MODE, typename YT = T, typename WT = T>
 __global__ void __launch_bounds__(OTX * OTY, sizeof(T) == 4 ? QMS_STENCIL_MINB : 2)
 qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap,
-         YT* __restrict__ y, const WT* __restrict__ w, double* __restrict__ partials, unsigned* __restrict__ err,
-         WT* __restrict__ yfull = nullptr) {
+         YT* y, const WT* w, double* partials, unsigned* err, WT* yfull) {
     // VCOUPLE reads only what the V rows' A couplings need: the three A blocks of x (xmap over
     // them) and the three conductivities (cmap over them)
     constexpr bool VC = MODE == QOPH_VCOUPLE;
@@ -159,11 +159,14 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
         for (int q = 0; q < 4; q++) mbar_init(&xbar[q], 1);
         for (int q = 0; q < 3; q++) mbar_init(&cbar[q], 1);
         fence_mbar_init();
+        issue_c(k0 - 1);                        // (the coefficients are the geometry's)
+        issue_c(k0);
+        pdl_wait();
         issue_x(k0 - 1);
         issue_x(k0);
         issue_x(k0 + 1);
-        issue_c(k0 - 1);
-        issue_c(k0);
+    } else {
+        pdl_wait();
     }
     __syncthreads();
     bool ok = mbar_wait(&xbar[(k0 - 1) & 3], xpar(k0 - 1), err) && mbar_wait(&xbar[k0 & 3], xpar(k0), err) &&
@@ -894,12 +897,12 @@ static void op_pl_launch(dim3 gs, dim3 bs, size_t shm, cudaStream_t st, int mode
         return;                                   // FP64 inner vectors: no or general advection only
     } else {
         if (mode == QOPH_APPLY)
-            qk_op_pl<T, VM, QOPH_APPLY><<<gs, bs, shm, st>>>(g, P, xmap, cmap, y, w, partials, err);
+            pdl_launch(qk_op_pl<T, VM, QOPH_APPLY>, gs, bs, shm, st, 0, g, P, xmap, cmap, y, w, partials, err, nullptr);
         else if (mode == QOPH_VCOUPLE)
-            qk_op_pl<T, VM, QOPH_VCOUPLE><<<gs, bs, PLTiles<T, 3, 3>::SMEM, st>>>(g, P, xmap, cmap, y, w, partials,
-                                                                                    err);
+            pdl_launch(qk_op_pl<T, VM, QOPH_VCOUPLE>, gs, bs, PLTiles<T, 3, 3>::SMEM, st, 0, g, P, xmap, cmap, y, w,
+                       partials, err, nullptr);
         else
-            qk_op_pl<T, VM, QOPH_SCALED><<<gs, bs, shm, st>>>(g, P, xmap, cmap, y, w, partials, err);
+            pdl_launch(qk_op_pl<T, VM, QOPH_SCALED>, gs, bs, shm, st, 0, g, P, xmap, cmap, y, w, partials, err, nullptr);
     }
 }
 
@@ -924,8 +927,8 @@ void qms_launch_resid_df(const QGrid& g, const QStepPar<qdf>& P, const CUtensorM
     const dim3 bs(OTX, OTY, 1), gs = qms_pl_tiles(g);
     const size_t shm = PLTiles<qdf>::SMEM;
     const int vm = qms_vel_mask(P, adv, true);
-    QMS_WITH_VM(vm, (qk_op_pl<qdf, VM, QOPH_RESID, float, qdf><<<gs, bs, shm, st>>>(g, P, xmap, cmap, r, b, partials, err,
-                                                                                   rfull)));
+    QMS_WITH_VM(vm, (pdl_launch(qk_op_pl<qdf, VM, QOPH_RESID, float, qdf>, gs, bs, shm, st, 0, g, P, xmap, cmap, r, b,
+                                partials, err, rfull)));
 }
 
 void qms_launch_delta_split(const QGrid& g, const double* x, const double* x0, qdf* dx, double* partials,

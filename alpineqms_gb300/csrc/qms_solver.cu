@@ -16,6 +16,7 @@
 // host; the host only reads the residual estimate to decide when to stop.
 #include "qms_internal.h"
 #include "qms_solver.h"
+#include "qms_pdl.cuh"
 #include "qms_pl.h"
 
 #include <atomic>
@@ -312,10 +313,9 @@ __device__ __forceinline__ bool gm_last_block(unsigned* counter) {
 // eight blocks per SM whatever the registers, a second wave of a few blocks followed (256^3, 8
 // vectors: 367 us instead of 405).
 template <typename T, int NV>
-__global__ void __launch_bounds__(256) qk_gm_dots(long long n, GmPtrs V, const T* __restrict__ w,
-                                                  double* __restrict__ part0, int row0, int final, int j, int m,
-                                                  double* __restrict__ Hm, double* __restrict__ Gm,
-                                                  unsigned* __restrict__ counter) {
+__global__ void __launch_bounds__(256) qk_gm_dots(long long n, GmPtrs V, const T* w, double* part0, int row0,
+                                                  int final, int j, int m, double* Hm, double* Gm,
+                                                  unsigned* counter) {
     using PK = GmPack<T>;
     using PV = typename PK::V;
     float acc[NV + 1];
@@ -326,6 +326,7 @@ __global__ void __launch_bounds__(256) qk_gm_dots(long long n, GmPtrs V, const T
     for (int i = 0; i < NV; i++) vp[i] = (const PV*)V.p[i];
     const PV* wp = (const PV*)w;
     const long long np = n / PK::W;
+    pdl_wait();
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < np; t += (long long)gridDim.x * blockDim.x) {
         const PV wv = wp[t];
         PV vv[NV];
@@ -379,14 +380,14 @@ __global__ void __launch_bounds__(256) qk_gm_dots(long long n, GmPtrs V, const T
 // applies the Givens rotations and forms the residual estimate; Gm layout: [0]: beta,
 // [1]: |g_{j+1}|, [2]: 1/h_{j+1,j}, cs[m] at 8, sn[m] at 8+m, g[m+1] at 8+2m
 template <typename T, int NV>
-__global__ void __launch_bounds__(256) qk_gm_orth(long long n, int j, int m, GmPtrs V, double* __restrict__ Hcol0,
-                                                  int row0, T* __restrict__ w, double* __restrict__ part,
-                                                  double* __restrict__ Gm, T* __restrict__ vout, int final,
-                                                  unsigned* __restrict__ counter, unsigned* __restrict__ status) {
+__global__ void __launch_bounds__(256) qk_gm_orth(long long n, int j, int m, GmPtrs V, double* Hcol0, int row0,
+                                                  T* w, double* part, double* Gm, T* vout, int final,
+                                                  unsigned* counter, unsigned* status) {
     using PK = GmPack<T>;
     using PV = typename PK::V;
     T h[NV];
     const PV* vp[NV];
+    pdl_wait();
 #pragma unroll
     for (int i = 0; i < NV; i++) { h[i] = (T)Hcol0[(row0 + i) * m + j]; vp[i] = (const PV*)V.p[i]; }
     const bool direct = final && Gm[3] != 0.0;
@@ -458,7 +459,8 @@ __global__ void __launch_bounds__(256) qk_gm_orth(long long n, int j, int m, GmP
 
 // V_{j+1} = w / h_{j+1,j} (nothing to do when the orthogonalisation wrote it, Gm[3])
 template <typename T>
-__global__ void qk_gm_scale(long long n, const T* __restrict__ w, T* __restrict__ vout, const double* __restrict__ Gm) {
+__global__ void qk_gm_scale(long long n, const T* w, T* vout, const double* Gm) {
+    pdl_wait();
     if (Gm[3] != 0.0) return;
     const T inv = (T)Gm[2];
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
@@ -551,7 +553,7 @@ static int gm_dots(int nv, int vb, cudaStream_t st, long long n, const GmPtrs& V
     switch (now) {
 #define C(N) case N: { static std::atomic<int> per{0}; \
         if (row0 == 0) nb = gm_blocks((const void*)qk_gm_dots<T, N>, per, vb); \
-        qk_gm_dots<T, N><<<nb, 256, 0, st>>>(n, V, w, part, row0, final, j, m, Hm, Gm, counter); } break;
+        pdl_launch(qk_gm_dots<T, N>, dim3(nb), dim3(256), 0, st, 0, n, V, w, part, row0, final, j, m, Hm, Gm, counter); } break;
         GM_CASES(C)
 #undef C
     }
@@ -563,7 +565,7 @@ static int gm_orth(int nv, int vb, cudaStream_t st, long long n, int j, int m, c
     const int now = std::min(nv, GM_PASS), final = now == nv ? 1 : 0;
     switch (now) {
 #define C(N) case N: { static std::atomic<int> per{0}; \
-        qk_gm_orth<T, N><<<gm_blocks((const void*)qk_gm_orth<T, N>, per, vb), 256, 0, st>>>(n, j, m, V, Hm, row0, w, part, Gm, vout, final, counter, status); } break;
+        pdl_launch(qk_gm_orth<T, N>, dim3(gm_blocks((const void*)qk_gm_orth<T, N>, per, vb)), dim3(256), 0, st, 0, n, j, m, V, Hm, row0, w, part, Gm, vout, final, counter, status); } break;
         GM_CASES(C)
 #undef C
     }
@@ -1144,7 +1146,7 @@ void QmsSolver::gmres_steps(bool adv, bool transient, const double v[3], int j0,
         op_pl<T>(adv, QOPH_SCALED, P, zj, w, nullptr, nullptr);
         nlaunch += gm_dots<T>(j + 1, vb, st, n, Vp, w, part, 0, j, m, gm_H, gm_scal, gm_count);
         nlaunch += gm_orth<T>(j + 1, vb, st, n, j, m, Vp, gm_H, 0, w, part, gm_scal, (T*)gmV[j + 1], gm_count, status);
-        qk_gm_scale<T><<<std::min(vb, 152), 256, 0, st>>>(n, w, (T*)gmV[j + 1], gm_scal);
+        pdl_launch(qk_gm_scale<T>, dim3(std::min(vb, 152)), dim3(256), 0, st, 0, n, w, (T*)gmV[j + 1], gm_scal);
         nlaunch++;
     }
 }

@@ -227,24 +227,22 @@ __device__ __forceinline__ T apply7(const MGLevelDev<T>& L, const MGBlockDesc& B
 // ------------------------------------------------------------------ smoother
 // first sweep from a zero guess: x = omega D^-1 b
 template <typename T>
-__global__ void mg_smooth0(MGLevelDev<T> L, const T* b, T omega, T* x, int mask_v) {
+__global__ void mg_smooth0(MGLevelDev<T> L, const T* b, T omega, T* x) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait();
     if (t >= L.total) return;
     const T bv = b[t];
     T di = L.dinv[t];
-    if (mask_v && t >= L.blk[L.nb - 1].off) di = T(0);
     x[t] = omega * di * bv;
 }
 
 // x_out = x_in + omega D^-1 (b - A x_in)
 template <typename T>
-__global__ void mg_smooth(MGLevelDev<T> L, const T* b, T omega, const T* xin, T* xout, int mask_v) {
+__global__ void mg_smooth(MGLevelDev<T> L, const T* b, T omega, const T* xin, T* xout) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     pdl_wait();
     if (t >= L.total) return;
     T di = L.dinv[t];
-    if (mask_v && t >= L.blk[L.nb - 1].off) di = T(0);
     if (di == T(0)) { xout[t] = T(0); return; }
     const int bk = find_block(L, t);
     const MGBlockDesc& B = L.blk[bk];
@@ -264,7 +262,7 @@ __global__ void mg_smooth(MGLevelDev<T> L, const T* b, T omega, const T* xin, T*
 #define MGR_Z 2
 template <typename T>
 __global__ void __launch_bounds__(MGR_X * MGR_Y * MGR_Z) mg_restrict(MGLevelDev<T> F, const T* bf, const T* xf,
-                                                                    MGLevelDev<T> C, T* bc, int mask_v, int xtiles) {
+                                                                    MGLevelDev<T> C, T* bc, int xtiles) {
     __shared__ T sh[MGR_Z][MGR_Y][MGR_X];
     const int b = blockIdx.x / xtiles;
     const MGBlockDesc& fb = F.blk[b];
@@ -285,7 +283,7 @@ __global__ void __launch_bounds__(MGR_X * MGR_Y * MGR_Z) mg_restrict(MGLevelDev<
     if (I >= cb.n1 || J >= cb.n2 || K >= cb.n3) return;
     r = (sh[0][threadIdx.y][threadIdx.x] + sh[0][threadIdx.y + 1][threadIdx.x]) +
         (sh[1][threadIdx.y][threadIdx.x] + sh[1][threadIdx.y + 1][threadIdx.x]);
-    bc[cb.off + I + (long long)J * cb.n1 + (long long)K * cb.n1 * cb.n2] = mask_v && b == C.nb - 1 ? T(0) : r;
+    bc[cb.off + I + (long long)J * cb.n1 + (long long)K * cb.n1 * cb.n2] = r;
 }
 
 // x_out = x_in + alpha x_c(aggregate of f) on active fine points (x_out may alias x_in)
@@ -416,20 +414,13 @@ template <typename T>
 __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__ MGSub<T> sub,
                                                        const double* __restrict__ minv,
                                                        const long long* __restrict__ moff, T omega, T alpha, int nu1,
-                                                       int nu2, int mask_v) {
+                                                       int nu2) {
     const int lg = sub.lg, size = 1 << lg, b = blockIdx.x >> lg, last = sub.nl - 1, tid = threadIdx.x;
     const int m = sub.L[last].blk[b].n1 * sub.L[last].blk[b].n2 * sub.L[last].blk[b].n3;
     double* db = reinterpret_cast<double*>(mgc_raw);
     MGCluster<T> G{cg::this_cluster(), reinterpret_cast<T*>(mgc_raw) + m * (int)(sizeof(double) / sizeof(T))};
     const int c = (int)G.cl.block_rank();
     __shared__ int at[MGC_LEVELS + 1];
-    if (mask_v && b == sub.L[0].nb - 1) {        // the whole cluster: V frozen at zero
-        pdl_wait();
-        const MGBlockDesc& B = sub.L[0].blk[b];
-        const long long n = (long long)B.n1 * B.n2 * B.n3;
-        for (long long q = c * MGC_THREADS + tid; q < n; q += size * MGC_THREADS) sub.L[0].x[B.off + q] = T(0);
-        return;
-    }
     if (tid == 0) {
         int o = 0;
         for (int l = 0; l <= last; l++) { at[l] = o; o += (int)mgc_len(sub.L[l].blk[b], lg, l < last); }
@@ -637,7 +628,7 @@ __device__ __forceinline__ double mg_cf(double v) { return v; }
 
 template <typename T, int KIND, int QS, bool UNI, int ROWS>
 __global__ void __launch_bounds__(OTX * OTY / ROWS, sizeof(T) == 4 ? (ROWS == 1 ? QMS_STENCIL_MINB : 6) : 2)
-mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* b, int scaled,
+mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, const T* b, int scaled,
           const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap, T* xout,
           MGLevelDev<T> C, T* bc, unsigned* err) {
     using S = MG0Set<QS>;
@@ -696,7 +687,7 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* b, int
         act[0][r] = in[r] && !(fyA || i == 1 || i >= g.xs);
         act[1][r] = in[r] && !(fxA || jr == 1 || jr >= g.ys);
         act[2][r] = in[r] && !(fxA || fyA);
-        act[3][r] = act[2][r] && !mask_v;
+        act[3][r] = act[2][r];
     }
     // offset of node (i, j) at plane k in a block (32-bit: checked at creation); block q's row r is
     // q * comp + nd + r * P
@@ -850,8 +841,6 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* b, int
 #pragma unroll
             for (int r = 0; r < R; r++) {
                 cm[5][r] = s2[r];
-                // a frozen V block: zero whatever the vector held
-                if (S::A && KIND != 2 && mask_v && in[r]) xout[3 * comp + nd + r * pitch] = T(0);
             }
         }
         nd += plane;
@@ -878,7 +867,7 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* b, int
                     const MGBlockDesc& cb = C.blk[q - Q0];
                     if (I < cb.n1 && J < cb.n2 && K < cb.n3)
                         bc[cb.off + I + (long long)J * cb.n1 + (long long)K * cb.n1 * cb.n2] =
-                            (mask_v && q == 3) ? T(0) : acc[q];
+                            acc[q];
                 }
             }
         }
@@ -887,15 +876,14 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, int mask_v, const T* b, int
 #undef XS
 }
 
-// level 0: x += alpha P x_c on the active points (the Dirichlet points of every component, and V when
-// masked, stay zero; C and xc: the level-1 view of the blocks of QS).  A thread has one 16-byte packet of
+// level 0: x += alpha P x_c on the active points (the Dirichlet points of every component stay zero; C and xc: the level-1 view of the blocks of QS).  A thread has one 16-byte packet of
 // columns (columns W v .. W v + W - 1 are i = W v ..; pairs (2I + 1, 2I + 2) share a coarse value) of each
 // component: bound by the bytes of x, which a thread per node moved 4 at a time (256^3, the A blocks:
 // 147 us before; runs of steps 128^3 220 -> 214 ms, 256^3 713 -> 694).
 #define MGP_X 16
 #define MGP_Y 16
 template <typename T, int QS>
-__global__ void __launch_bounds__(MGP_X * MGP_Y) mg0_prolong(QGrid g, int mask_v, T* x, MGLevelDev<T> C, const T* xc,
+__global__ void __launch_bounds__(MGP_X * MGP_Y) mg0_prolong(QGrid g, T* x, MGLevelDev<T> C, const T* xc,
                                                             T alpha) {
     using S = MG0Set<QS>;
     constexpr int W = 16 / (int)sizeof(T);
@@ -927,7 +915,7 @@ __global__ void __launch_bounds__(MGP_X * MGP_Y) mg0_prolong(QGrid g, int mask_v
         block(1, !fz && j > 1 && j < g.ys, 3, g.Nx - 2);
         block(2, !fy && k > 1 && k < g.zs, 3, g.Nx - 2);
     }
-    if (S::V) block(3, !fy && !fz && !mask_v, 3, g.Nx - 2);
+    if (S::V) block(3, !fy && !fz, 3, g.Nx - 2);
 }
 
 template <typename T, int KIND, int QS = 0>
@@ -1305,23 +1293,22 @@ int QmsMG<T>::build(const QGrid& g, const QCoef<T>& c, const QStepPar<T>& P, T v
 // result in x0; t0 is a level-0 temporary.  Returns the number of kernel launches.
 template <typename T>
 int QmsMG<T>::vcycle(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map, T* t0, const CUtensorMap& t0map,
-                     const CUtensorMap& cmap, bool mask_v, unsigned* err, cudaStream_t st, int qs,
+                     const CUtensorMap& cmap, unsigned* err, cudaStream_t st, int qs,
                      const CUtensorMap* b0map) {
-    if (qs == 1) return vcycle_q<1>(b0, scaled, x0, x0map, t0, t0map, cmap, mask_v, err, st, b0map);
-    if (qs == 2) return vcycle_q<2>(b0, scaled, x0, x0map, t0, t0map, cmap, mask_v, err, st, b0map);
-    return vcycle_q<0>(b0, scaled, x0, x0map, t0, t0map, cmap, mask_v, err, st, nullptr);
+    if (qs == 1) return vcycle_q<1>(b0, scaled, x0, x0map, t0, t0map, cmap, err, st, b0map);
+    if (qs == 2) return vcycle_q<2>(b0, scaled, x0, x0map, t0, t0map, cmap, err, st, b0map);
+    return vcycle_q<0>(b0, scaled, x0, x0map, t0, t0map, cmap, err, st, nullptr);
 }
 
 template <typename T>
 template <int QS>
 int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map, T* t0, const CUtensorMap& t0map,
-                       const CUtensorMap& cmap, bool mask_v, unsigned* err, cudaStream_t st,
+                       const CUtensorMap& cmap, unsigned* err, cudaStream_t st,
                        const CUtensorMap* b0map) {
     int launches = 0;
     std::vector<MGLevelDev<T>>& lv = QS == 0 ? this->lv : views[QS];   // levels >= 1 of the cycle's blocks
     const long long* dmo = dmoff + (QS == 2 ? 3 : 0);                    // their dense coarsest inverses
     const int nl = (int)lv.size();
-    const int mv = (QS == 0 && mask_v) ? 1 : 0;
     // sweeps on each side: the V-block cycle may use its own count
     const int n1 = (QS == 2 && nu_v > 0) ? nu_v : nu1, n2 = (QS == 2 && nu_v > 0) ? nu_v : nu2;
     const int sc = scaled ? 1 : 0;
@@ -1331,7 +1318,7 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     // KIND 2 reads XI and writes the level-1 right-hand side
 #define MG0U(KIND, XI, XO, BC, UNI, ROWS)                                                                         \
     pdl_launch(mg0_tiled<T, KIND, QS, UNI, ROWS>, g0grid, dim3(OTX, OTY / ROWS), mg0_smem<T, KIND, QS>(), st, 0,  \
-               g0, P0, vshift0, omega, mv, b0, sc, *(XI).m, cmap, (XO), lv[1], (BC), err)
+               g0, P0, vshift0, omega, b0, sc, *(XI).m, cmap, (XO), lv[1], (BC), err)
 #define MG0(KIND, XI, XO, BC)                                                                                     \
     do {                                                                                                          \
         if (ROWS2 > 1 && two) {                                                                                   \
@@ -1391,16 +1378,16 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
             sub.lg = sub_lg;
             for (int q = 0; q < sub.nl; q++) sub.L[q] = lv[lt + q];
             pdl_launch(mg_sub<T>, dim3(L.nb << sub_lg), dim3(MGC_THREADS), sub_smem[QS], st, 1u << sub_lg, sub, dminv, dmo,
-                       omega, alpha, nuc1, nuc2, mv);
+                       omega, alpha, nuc1, nuc2);
             launches++;
             break;
         }
         T* xl = L.x;
         T* tl = L.t;
-        pdl_launch(mg_smooth0<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, mv);
+        pdl_launch(mg_smooth0<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl);
         launches++;
         for (int s = 1; s < nuc1; s++) {
-            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl, mv);
+            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl);
             std::swap(xl, tl);
             launches++;
         }
@@ -1414,7 +1401,7 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
         }
         const int xt = (e1 + MGR_X - 1) / MGR_X;
         pdl_launch(mg_restrict<T>, dim3(L.nb * xt, (e2 + MGR_Y - 1) / MGR_Y, (e3 + MGR_Z - 1) / MGR_Z),
-                   dim3(MGR_X, MGR_Y, MGR_Z), 0, st, 0, L, L.b, xl, lv[l + 1], lv[l + 1].b, mv, xt);
+                   dim3(MGR_X, MGR_Y, MGR_Z), 0, st, 0, L, L.b, xl, lv[l + 1], lv[l + 1].b, xt);
         launches++;
     }
     for (int l = lt - 1; l >= 1; l--) {
@@ -1424,7 +1411,7 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
         pdl_launch(mg_prolong<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, xl, xl, lv[l + 1], lv[l + 1].x, alpha);
         launches++;
         for (int s = 0; s < nuc2; s++) {
-            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl, mv);
+            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl);
             std::swap(xl, tl);
             launches++;
         }
@@ -1433,7 +1420,7 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     }
     const int cols = MGP_X * 16 / (int)sizeof(T);
     pdl_launch(mg0_prolong<T, QS>, dim3((g0.xs + cols - 1) / cols, (g0.ys + MGP_Y - 1) / MGP_Y, g0.Nz),
-               dim3(MGP_X, MGP_Y), 0, st, 0, g0, mv, x.p, lv[1], lv[1].x, alpha);
+               dim3(MGP_X, MGP_Y), 0, st, 0, g0, x.p, lv[1], lv[1].x, alpha);
     launches++;
     for (int s = 0; s < n2; s++) {
         sweep(x, t.p);

@@ -115,10 +115,10 @@ __device__ __forceinline__ T pl_div(T a, T d) {
     else return a / d;
 }
 
-// MODE: QOPH_APPLY (y = M x), QOPH_SCALED (y = D^-1 M x), QOPH_VCOUPLE (V rows only:
+// MODE: QOPH_APPLY_A (y_A = M_AA x_A; no velocity), QOPH_SCALED (y = D^-1 M x), QOPH_VCOUPLE (V rows only:
 // y = w - D^-1 M (x_A, 0)) or QOPH_RESID (T = qdf: y = (float) (w - D^-1 M x), the refinement
 // residual in double-float arithmetic, with w the residual of the anchor and x the change of
-// the solution since then).  Partials (optional, FP64 across warps): APPLY / SCALED [0] += y . w
+// the solution since then).  Partials (optional, FP64 across warps): APPLY_A / SCALED [0] += y . w
 // (w may be null), [1] += y . y; RESID |r_A|^2, |r_V|^2; none with VCOUPLE.
 template <typename T, int VM, int MODE, typename YT = T, typename WT = T>
 __global__ void __launch_bounds__(OTX * OTY, sizeof(T) == 4 ? QMS_STENCIL_MINB : 2)
@@ -127,8 +127,9 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
     // VCOUPLE reads only what the V rows' A couplings need: the three A blocks of x (xmap over
     // them) and the three conductivities (cmap over them)
     constexpr bool VC = MODE == QOPH_VCOUPLE;
+    constexpr bool AO = MODE == QOPH_APPLY_A;      // the A blocks alone: conjugate gradients with V = 0
     constexpr int C0 = VC ? 3 : 0;
-    using TL = PLTiles<T, VC ? 3 : 4, VC ? 3 : 6>;
+    using TL = PLTiles<T, VC || AO ? 3 : 4, VC ? 3 : 6>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     T* xsm = reinterpret_cast<T*>(smem_raw);                  // [4 slots][4][PLXY][PLX]
     T* csm = xsm + 4 * TL::XSLOT;                             // [3 slots][6][PLCY][PLX]
@@ -193,7 +194,8 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
         } else if constexpr (MODE == QOPH_VCOUPLE) {   // the A rows are not wanted (dead code)
             if (!is_a) y[row] = w[row] - pl_div(acc, diag);
         } else {
-            const T out = MODE == QOPH_APPLY ? acc : pl_div(acc, diag);
+            if (AO && !is_a) return;                   // the V row is not wanted (dead code)
+            const T out = AO ? acc : pl_div(acc, diag);
             y[row] = out;
             if (partials) {
                 if (w) red0 += (RT)(out * w[row]);
@@ -218,7 +220,7 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
         const T* ccur = csm + (k % 3) * TL::CSLOT;
         if (inij) {
             auto xsf = [&](int comp, int dk, int dj, int di) -> T {
-                if (MODE == QOPH_VCOUPLE && comp == 3) return T(0);
+                if ((VC || AO) && comp == 3) return T(0);
                 const T* b = dk < 0 ? xm : (dk > 0 ? xp : x0);
                 return b[(comp * PLXY + lj + dj) * PLX + li + di];
             };
@@ -851,7 +853,9 @@ static int qms_vel_mask(const QStepPar<T>& P, bool adv, bool axes) {
 
 template <typename T, int VM>
 static void op_pl_attrs(int shm) {
-    cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_APPLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
+    if (VM == 0)
+        cudaFuncSetAttribute(qk_op_pl<T, 0, QOPH_APPLY_A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)PLTiles<T, 3, 6>::SMEM);
     cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
     cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_VCOUPLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)PLTiles<T, 3, 3>::SMEM);
@@ -896,8 +900,9 @@ static void op_pl_launch(dim3 gs, dim3 bs, size_t shm, cudaStream_t st, int mode
     if constexpr (sizeof(T) == 8 && VM != 0 && VM != 7) {
         return;                                   // FP64 inner vectors: no or general advection only
     } else {
-        if (mode == QOPH_APPLY)
-            pdl_launch(qk_op_pl<T, VM, QOPH_APPLY>, gs, bs, shm, st, 0, g, P, xmap, cmap, y, w, partials, err, nullptr);
+        if (mode == QOPH_APPLY_A)                 // (no velocity: VM is 0)
+            pdl_launch(qk_op_pl<T, 0, QOPH_APPLY_A>, gs, bs, PLTiles<T, 3, 6>::SMEM, st, 0, g, P, xmap, cmap, y, w,
+                       partials, err, nullptr);
         else if (mode == QOPH_VCOUPLE)
             pdl_launch(qk_op_pl<T, VM, QOPH_VCOUPLE>, gs, bs, PLTiles<T, 3, 3>::SMEM, st, 0, g, P, xmap, cmap, y, w,
                        partials, err, nullptr);

@@ -17,7 +17,8 @@ dim3 qms_node_block();
 dim3 qms_pl_tiles(const QGrid& g);
 long long qms_op_pl_num_blocks(const QGrid& g);
 
-// y = M x (mode QOPH_APPLY) or D^-1 M x (QOPH_SCALED) on padded vectors; x and the node
+// y_A = M_AA x_A without velocity (mode QOPH_APPLY_A, the map of x's A blocks) or D^-1 M x (QOPH_SCALED) on
+// padded vectors; x and the node
 // coefficients come through their tensor maps (qms_make_pl_map, 10 and 9 rows per box).
 // QOPH_VCOUPLE takes the maps of x's three A blocks and of the three conductivities.
 template <typename T>

@@ -45,8 +45,8 @@ enum FinOp {
     FIN_CG_INIT, FIN_CG_ALPHA, FIN_CG_BETA
 };
 
-__global__ void qk_finalize(const double* __restrict__ part, long long nb, int nsum, double* __restrict__ S, int op,
-                            unsigned* __restrict__ status) {
+__global__ void qk_finalize(const double* part, long long nb, int nsum, double* S, int op, unsigned* status) {
+    pdl_wait();
     // a quarter of the block's warps per sum (16 warps, up to 4 sums), added up in a fixed order
     __shared__ double sh[4][4];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = wid >> 2, part_w = wid & 3;
@@ -224,38 +224,83 @@ __global__ void qk_jacobi(long long n, long long mask_from, const T* __restrict_
     }
 }
 
+// 16-byte packets: the padded layout's length is a multiple of 4 elements and every vector
+// starts on a 256-byte boundary, so sweeps over vectors move whole packets
+template <typename T> struct GmPack;
+template <> struct GmPack<float> {
+    using V = float4;
+    static constexpr int W = 4;
+    static __device__ __forceinline__ float at(const V& v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
+};
+template <> struct GmPack<double> {
+    using V = double2;
+    static constexpr int W = 2;
+    static __device__ __forceinline__ double at(const V& v, int q) { return q == 0 ? v.x : v.y; }
+};
+
+// The conjugate-gradient vectors, 16-byte packets over the three A blocks (the V block is frozen at
+// zero).  Bound by bytes: e takes its step together with p's (one read of p less than apart), 9 blocks
+// of vector traffic per iteration in all where 13 were (V block included).
+template <typename T>
+__device__ __forceinline__ long long cg_packets(long long n) { return n * (long long)sizeof(T) / 16; }
+
 // partials of r.z and z.z; optionally p = z (first iteration)
 template <typename T>
-__global__ void qk_cg_dot(long long n, const T* __restrict__ r, const T* __restrict__ z, T* __restrict__ p,
-                          double* __restrict__ part) {
+__global__ void __launch_bounds__(256) qk_cg_dot(long long n, const T* r, const T* z, T* p, double* part) {
+    using PK = GmPack<T>;
+    using PV = typename PK::V;
     float a0 = 0.f, a1 = 0.f;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        T zv = z[t];
-        if (p) p[t] = zv;
-        a0 += (float)(r[t] * zv);
-        a1 += (float)(zv * zv);
+    pdl_wait();
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cg_packets<T>(n); t += (long long)gridDim.x * blockDim.x) {
+        const PV zv = reinterpret_cast<const PV*>(z)[t], rv = reinterpret_cast<const PV*>(r)[t];
+        if (p) reinterpret_cast<PV*>(p)[t] = zv;
+#pragma unroll
+        for (int q = 0; q < PK::W; q++) {
+            a0 += (float)(PK::at(rv, q) * PK::at(zv, q));
+            a1 += (float)(PK::at(zv, q) * PK::at(zv, q));
+        }
     }
     store_partials<T>(part, a0, a1);
 }
 
+// v += sign alpha d
 template <typename T>
-__global__ void qk_cg_update(long long n, const T* __restrict__ p, const T* __restrict__ q,
-                             const double* __restrict__ S, T* __restrict__ e, T* __restrict__ r) {
-    const T al = (T)S[S_ALPHA];
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        e[t] += al * p[t];
-        r[t] -= al * q[t];
+__global__ void __launch_bounds__(256) qk_cg_axpy(long long n, const T* d, const double* S, T sign, T* v) {
+    using PK = GmPack<T>;
+    using PV = typename PK::V;
+    pdl_wait();
+    const T al = sign * (T)S[S_ALPHA];
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cg_packets<T>(n); t += (long long)gridDim.x * blockDim.x) {
+        const PV dv = reinterpret_cast<const PV*>(d)[t];
+        PV vv = reinterpret_cast<PV*>(v)[t];
+        T* vq = reinterpret_cast<T*>(&vv);
+#pragma unroll
+        for (int q = 0; q < PK::W; q++) vq[q] += al * PK::at(dv, q);
+        reinterpret_cast<PV*>(v)[t] = vv;
     }
 }
 
+// e += alpha p, then p = z + beta p
 template <typename T>
-__global__ void qk_cg_p(long long n, const T* __restrict__ z, T* __restrict__ p, const double* __restrict__ S) {
-    const T be = (T)S[S_BETA];
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        p[t] = z[t] + be * p[t];
+__global__ void __launch_bounds__(256) qk_cg_ep(long long n, const T* z, T* p, T* e, const double* S) {
+    using PK = GmPack<T>;
+    using PV = typename PK::V;
+    pdl_wait();
+    const T al = (T)S[S_ALPHA], be = (T)S[S_BETA];
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < cg_packets<T>(n); t += (long long)gridDim.x * blockDim.x) {
+        const PV zv = reinterpret_cast<const PV*>(z)[t];
+        PV pv = reinterpret_cast<PV*>(p)[t], ev = reinterpret_cast<PV*>(e)[t];
+        T* pq = reinterpret_cast<T*>(&pv);
+        T* eq = reinterpret_cast<T*>(&ev);
+#pragma unroll
+        for (int q = 0; q < PK::W; q++) {
+            eq[q] += al * pq[q];
+            pq[q] = PK::at(zv, q) + be * pq[q];
+        }
+        reinterpret_cast<PV*>(p)[t] = pv;
+        reinterpret_cast<PV*>(e)[t] = ev;
+    }
 }
-
-
 
 // --------------------------------------------------------------------------
 // FGMRES (right preconditioned, restarted by the outer refinement) with the
@@ -270,20 +315,6 @@ struct GmPtrs { const void* p[GM_MAXM + 1]; };
 // block partials of V_i . w for i = 0..NV-1 (classical Gram-Schmidt projections).
 // NV is a compile-time count so every load of the unrolled loop is unconditional
 // and independent (memory-level parallelism over all basis vectors).
-// 16-byte packets: the padded layout's length is a multiple of 4 elements and every vector
-// starts on a 256-byte boundary, so the Gram-Schmidt sweeps move whole packets
-template <typename T> struct GmPack;
-template <> struct GmPack<float> {
-    using V = float4;
-    static constexpr int W = 4;
-    static __device__ __forceinline__ float at(const V& v, int q) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; }
-};
-template <> struct GmPack<double> {
-    using V = double2;
-    static constexpr int W = 2;
-    static __device__ __forceinline__ double at(const V& v, int q) { return q == 0 ? v.x : v.y; }
-};
-
 // True in every thread of the block that arrives last (its threads then see what the others wrote
 // before); the counter is zero again for the next launch.
 __device__ __forceinline__ bool gm_last_block(unsigned* counter) {
@@ -922,7 +953,7 @@ QCoef<float> QmsSolver::coef32() const { return QCoef<float>{g, ids, dtab32, (fl
 QCoef<double> QmsSolver::coef64() const { return QCoef<double>{g, ids, dtab64, 1.0 / QMS_MU0, nc64}; }
 
 int QmsSolver::finalize(int fop, int nsum, long long nb) {
-    qk_finalize<<<1, 512, 0, st>>>(part, nb, nsum, S, fop, status);
+    pdl_launch(qk_finalize, dim3(1), dim3(512), 0, st, 0, part, nb, nsum, S, fop, status);
     nlaunch++;
     return 0;
 }
@@ -950,7 +981,8 @@ template <typename T>
 void QmsSolver::op_pl(bool adv, int mode, const QStepPar<T>& P, const T* xin, T* y, const T* w, double* partials) {
     const double ncell = (double)g.xs * g.ys * g.zs;
     OpEv* ev = prof_begin(sizeof(T) == 8 ? 1 : 0, (double)g.n * sizeof(T) * (2 + (w && w != xin ? 1 : 0)) + ncell);
-    qms_launch_op_pl<T>(g, P, tmap(xin), sizeof(T) == 8 ? cmap64 : cmap32, adv, mode, y, w, partials, status, st);
+    qms_launch_op_pl<T>(g, P, mode == QOPH_APPLY_A ? tmapq(xin, 1) : tmap(xin), sizeof(T) == 8 ? cmap64 : cmap32, adv, mode,
+                        y, w, partials, status, st);
     nlaunch++;
     prof_end(ev);
 }
@@ -1039,11 +1071,11 @@ void QmsSolver::precond(const T* r, const float* bscale, T* z, bool mask_v, bool
             }
             if (f32)
                 nlaunch += mgf[transient ? 1 : 0].vcycle((const float*)b, bscale != nullptr, (float*)z, tmapq(z, qs),
-                                                         mgtmp, tmapq(mgtmp, qs), cmq, mask_v, status, st, qs, bm);
+                                                         mgtmp, tmapq(mgtmp, qs), cmq, status, st, qs, bm);
             else
                 nlaunch += mgd[transient ? 1 : 0].vcycle((const double*)b, bscale != nullptr, (double*)z,
-                                                         tmapq(z, qs), (double*)mgtmp, tmapq(mgtmp, qs), cmq, mask_v,
-                                                         status, st, qs);
+                                                         tmapq(z, qs), (double*)mgtmp, tmapq(mgtmp, qs), cmq, status,
+                                                         st, qs);
         };
         if (P && !mask_v && bscale && desc.mg_coupling == 1) {
             // lower block-triangular: the A blocks first, then the V block on the residual that
@@ -1055,9 +1087,11 @@ void QmsSolver::precond(const T* r, const float* bscale, T* z, bool mask_v, bool
             cycle(tv, 2, f32 ? cmapV16 : cmapV64);
             nlaunch++;
             regions.apply<T>(tv, bscale, z, st, nlaunch);
+        } else if (mask_v) {
+            cycle(r, 1, cm);                     // z's V block stays as it is (zero)
         } else {
             cycle(r, 0, cm);
-            if (!mask_v) regions.apply<T>(r, bscale, z, st, nlaunch);
+            regions.apply<T>(r, bscale, z, st, nlaunch);
         }
         prof_end(ev);
     } else if (jacobi_pcg) {
@@ -1279,33 +1313,39 @@ int QmsSolver::inner_pcg(bool transient, int& iters) {
     const float* dg = transient ? dg_tr : dg_steady;
     QStepPar<T> P = qms_step_par<T>(g, 0, 0, 0, desc.dt, transient);
     const int vb = (int)vec_blocks;
-    // V block frozen at zero: the steady magnetostatic system with v = 0 has V = 0
+    // V block frozen at zero: the steady magnetostatic system with v = 0 has V = 0.  The vectors' V parts
+    // are left alone (z's and the correction e's are zero), and the cycles work on the A blocks.
+    const long long nA = 3 * qms_pl(g).comp;
     resid_to_inner<T>(r);
     qk_cg_init<T><<<vb, 256, 0, st>>>(n, dg, r, e);
     nlaunch++;
+    CK(cudaMemsetAsync(z + nA, 0, (n - nA) * sizeof(T), st));
     precond<T>(r, nullptr, z, true, transient, true);
-    qk_cg_dot<T><<<vb, 256, 0, st>>>(n, r, z, p, part);
+    pdl_launch(qk_cg_dot<T>, dim3(vb), dim3(256), 0, st, 0, nA, r, z, p, part);
     nlaunch++;
     finalize(FIN_CG_INIT, 2, vec_blocks);
     const double tol2 = desc.inner_rtol * desc.inner_rtol;
     iters = 0;
     for (int it = 0; it < desc.max_inner; it++) {
-        op_pl<T>(false, QOPH_APPLY, P, p, q, p, part);
+        op_pl<T>(false, QOPH_APPLY_A, P, p, q, p, part);
         finalize(FIN_CG_ALPHA, 1, nbpl);
-        qk_cg_update<T><<<vb, 256, 0, st>>>(n, p, q, S, e, r);
+        pdl_launch(qk_cg_axpy<T>, dim3(vb), dim3(256), 0, st, 0, nA, q, S, T(-1), r);
         nlaunch++;
         precond<T>(r, nullptr, z, true, transient, true);
-        qk_cg_dot<T><<<vb, 256, 0, st>>>(n, r, z, (T*)nullptr, part);
+        pdl_launch(qk_cg_dot<T>, dim3(vb), dim3(256), 0, st, 0, nA, r, z, nullptr, part);
         nlaunch++;
         finalize(FIN_CG_BETA, 2, vec_blocks);
         iters = it + 1;
-        if ((it + 1) % desc.check_every == 0 || it + 1 == desc.max_inner) {
+        bool done = it + 1 == desc.max_inner;
+        if ((it + 1) % desc.check_every == 0 || done) {
             int rc = read_scalars();
             if (rc) return rc;
-            if (hS[S_RZ] <= tol2 * hS[S_RZ0]) break;
+            done = done || hS[S_RZ] <= tol2 * hS[S_RZ0];
         }
-        qk_cg_p<T><<<vb, 256, 0, st>>>(n, z, p, S);
+        if (done) pdl_launch(qk_cg_axpy<T>, dim3(vb), dim3(256), 0, st, 0, nA, p, S, T(1), e);
+        else pdl_launch(qk_cg_ep<T>, dim3(vb), dim3(256), 0, st, 0, nA, z, p, e, S);
         nlaunch++;
+        if (done) break;
     }
     qms_launch_ref_add_pl<T>(g, e, S + S_NRM, x, st);
     nlaunch++;

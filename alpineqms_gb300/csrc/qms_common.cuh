@@ -161,6 +161,7 @@ struct QStepPar {
     T i2dx2, i2dy2, i2dz2; // 1/(2h^2)
     T i2dxdy, i2dxdz, i2dydz;
     T sigfloor;            // (double)1.0e-12f, F:1237
+    T idtx = T(0);         // 1/(dt h), cubic cells only (qms_unit_par)
 };
 
 template <typename T>

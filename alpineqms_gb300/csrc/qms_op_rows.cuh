@@ -7,106 +7,123 @@
 //   xs(q, dk, dj, di): unknown block q at (i + di, j + dj, k + dk), dk in {-1, 0, 1}
 //   cf(q, dk, dj, di): node coefficient q (1/mu_x,y,z, sigma_x,y,z) at (i + di, j + dj, k + dk),
 //                      dk in {-1, 0}
-//   emit(row, acc, diag, is_a, x_row): the row's value M x, its diagonal and its own unknown
+//   emit(row, acc, diag, is_a, x_row, fixed): the row's value M x, its diagonal, its own unknown and whether it is
+//                      a Dirichlet row (value and diagonal then without units)
 // fij*/kf*: the (i, j) and k parts of the Dirichlet predicates qFixX/Y/Z/V.
+// UNI: cubic cells (dx = dy = dz), everything in units of 1 / h^2: P is then qms_unit_par's (1/dt, 1/h and the
+// advection factors times h^2), the links' 1 / h^2 is one and left out of the products at compile time,
+// and acc and diag come in those units.  A row's products fall by about a third (the kernels over
+// these rows are bound by instruction issue).
 // VM: which velocity components may be nonzero (bit 0 x, 1 y, 2 z; 0 = no advection term);
 // the terms of components outside VM are left out at compile time (they are exact zeros).
 #pragma once
 #include "qms_common.cuh"
 
-template <typename T, int VM, typename XS, typename CF, typename EMIT>
+template <typename T>
+static inline QStepPar<T> qms_unit_par(const QGrid& g, QStepPar<T> p) {
+    const double u = g.dx * g.dx;
+    p.idtx = (T)((double)p.idt * g.dx);
+    p.idt = (T)((double)p.idt * u);
+    p.idx2 = p.idy2 = p.idz2 = p.idxdy = p.idxdz = p.idydz = T(1);
+    p.i2dx = p.i2dy = p.i2dz = (T)(0.5 * g.dx);
+    p.idx = p.idy = p.idz = (T)g.dx;
+    p.i2dx2 = p.i2dy2 = p.i2dz2 = p.i2dxdy = p.i2dxdz = p.i2dydz = T(0.5);
+    return p;
+}
+template <typename T, int VM, bool UNI = false, typename XS, typename CF, typename EMIT>
 __device__ __forceinline__ void qms_op_node(const QGrid& g, const QStepPar<T>& P, int i, int j, int k, bool fijX,
                                             bool fijY, bool fijZ, bool kfA, bool kfZ, long long rX, long long rY,
                                             long long rZ, long long rV, XS xs, CF cf, EMIT emit) {
+        auto lk = [](T c, T w) -> T { if constexpr (UNI) return c; else return c * w; };   // a link times its 1 / h^2
         constexpr bool HX = (VM & 1) != 0, HY = (VM & 2) != 0, HZ = (VM & 4) != 0;
         // ---------------------------------------------------------------- Ax
         if (i <= g.xs) {
             const long long row = rX;
             if (fijX || kfA) {
-                emit(row, xs(0, 0, 0, 0), T(1), true, xs(0, 0, 0, 0));
+                emit(row, xs(0, 0, 0, 0), T(1), true, xs(0, 0, 0, 0), true);
             } else {
                 const T s = cf(3, 0, 0, 0);
                 const T my_km = cf(1, -1, 0, 0), my_k = cf(1, 0, 0, 0);
                 const T mz_jm = cf(2, 0, -1, 0), mz_j = cf(2, 0, 0, 0);
                 const T mx_im = cf(0, 0, 0, -1), mx_i = cf(0, 0, 0, 0);
                 const T svy = HY ? s * P.vy : T(0), svz = HZ ? s * P.vz : T(0);
-                const T d = (mz_j + mz_jm) * P.idy2 + (my_k + my_km) * P.idz2 + (mx_i + mx_im) * P.idx2 + s * P.idt;
+                const T d = lk(mz_j + mz_jm, P.idy2) + lk(my_k + my_km, P.idz2) + lk(mx_i + mx_im, P.idx2) + s * P.idt;
                 // difference form: every coupling pair is applied to a difference of unknowns,
                 // so the rounding error scales with the variation of x, not with x itself
                 const T X0 = xs(0, 0, 0, 0);
                 T acc = s * P.idt * X0;
-                acc += my_km * P.idz2 * (X0 - xs(0, -1, 0, 0)) + my_k * P.idz2 * (X0 - xs(0, 1, 0, 0));
-                acc += mz_jm * P.idy2 * (X0 - xs(0, 0, -1, 0)) + mz_j * P.idy2 * (X0 - xs(0, 0, 1, 0));
-                acc += mx_im * P.idx2 * (X0 - xs(0, 0, 0, -1)) + mx_i * P.idx2 * (X0 - xs(0, 0, 0, 1));
+                acc += lk(my_km, P.idz2) * (X0 - xs(0, -1, 0, 0)) + lk(my_k, P.idz2) * (X0 - xs(0, 1, 0, 0));
+                acc += lk(mz_jm, P.idy2) * (X0 - xs(0, 0, -1, 0)) + lk(mz_j, P.idy2) * (X0 - xs(0, 0, 1, 0));
+                acc += lk(mx_im, P.idx2) * (X0 - xs(0, 0, 0, -1)) + lk(mx_i, P.idx2) * (X0 - xs(0, 0, 0, 1));
                 if constexpr (HZ) acc += svz * P.i2dz * (xs(0, -1, 0, 0) - xs(0, 1, 0, 0));
                 if constexpr (HY) acc += svy * P.i2dy * (xs(0, 0, -1, 0) - xs(0, 0, 1, 0));
-                acc += (HY ? mz_jm * P.idxdy - svy * P.i2dx : mz_jm * P.idxdy) * (xs(1, 0, -1, 0) - xs(1, 0, -1, 1));
-                acc += (HY ? mz_j * P.idxdy + svy * P.i2dx : mz_j * P.idxdy) * (xs(1, 0, 0, 1) - xs(1, 0, 0, 0));
-                acc += (HZ ? my_km * P.idxdz - svz * P.i2dx : my_km * P.idxdz) * (xs(2, -1, 0, 0) - xs(2, -1, 0, 1));
-                acc += (HZ ? my_k * P.idxdz + svz * P.i2dx : my_k * P.idxdz) * (xs(2, 0, 0, 1) - xs(2, 0, 0, 0));
+                acc += (HY ? lk(mz_jm, P.idxdy) - svy * P.i2dx : lk(mz_jm, P.idxdy)) * (xs(1, 0, -1, 0) - xs(1, 0, -1, 1));
+                acc += (HY ? lk(mz_j, P.idxdy) + svy * P.i2dx : lk(mz_j, P.idxdy)) * (xs(1, 0, 0, 1) - xs(1, 0, 0, 0));
+                acc += (HZ ? lk(my_km, P.idxdz) - svz * P.i2dx : lk(my_km, P.idxdz)) * (xs(2, -1, 0, 0) - xs(2, -1, 0, 1));
+                acc += (HZ ? lk(my_k, P.idxdz) + svz * P.i2dx : lk(my_k, P.idxdz)) * (xs(2, 0, 0, 1) - xs(2, 0, 0, 0));
                 acc += s * P.idx * (xs(3, 0, 0, 1) - xs(3, 0, 0, 0));
-                emit(row, acc, d, true, xs(0, 0, 0, 0));
+                emit(row, acc, d, true, xs(0, 0, 0, 0), false);
             }
         }
         // ---------------------------------------------------------------- Ay
         if (j <= g.ys) {
             const long long row = rY;
             if (fijY || kfA) {
-                emit(row, xs(1, 0, 0, 0), T(1), true, xs(1, 0, 0, 0));
+                emit(row, xs(1, 0, 0, 0), T(1), true, xs(1, 0, 0, 0), true);
             } else {
                 const T s = cf(4, 0, 0, 0);
                 const T mz_im = cf(2, 0, 0, -1), mz_i = cf(2, 0, 0, 0);
                 const T mx_km = cf(0, -1, 0, 0), mx_k = cf(0, 0, 0, 0);
                 const T my_jm = cf(1, 0, -1, 0), my_j = cf(1, 0, 0, 0);
                 const T svx = HX ? s * P.vx : T(0), svz = HZ ? s * P.vz : T(0);
-                const T d = (mz_i + mz_im) * P.idx2 + (mx_k + mx_km) * P.idz2 + (my_j + my_jm) * P.idy2 + s * P.idt;
+                const T d = lk(mz_i + mz_im, P.idx2) + lk(mx_k + mx_km, P.idz2) + lk(my_j + my_jm, P.idy2) + s * P.idt;
                 const T Y0 = xs(1, 0, 0, 0);
                 T acc = s * P.idt * Y0;
-                acc += mx_km * P.idz2 * (Y0 - xs(1, -1, 0, 0)) + mx_k * P.idz2 * (Y0 - xs(1, 1, 0, 0));
-                acc += my_jm * P.idy2 * (Y0 - xs(1, 0, -1, 0)) + my_j * P.idy2 * (Y0 - xs(1, 0, 1, 0));
-                acc += mz_im * P.idx2 * (Y0 - xs(1, 0, 0, -1)) + mz_i * P.idx2 * (Y0 - xs(1, 0, 0, 1));
+                acc += lk(mx_km, P.idz2) * (Y0 - xs(1, -1, 0, 0)) + lk(mx_k, P.idz2) * (Y0 - xs(1, 1, 0, 0));
+                acc += lk(my_jm, P.idy2) * (Y0 - xs(1, 0, -1, 0)) + lk(my_j, P.idy2) * (Y0 - xs(1, 0, 1, 0));
+                acc += lk(mz_im, P.idx2) * (Y0 - xs(1, 0, 0, -1)) + lk(mz_i, P.idx2) * (Y0 - xs(1, 0, 0, 1));
                 if constexpr (HZ) acc += svz * P.i2dz * (xs(1, -1, 0, 0) - xs(1, 1, 0, 0));
                 if constexpr (HX) acc += svx * P.i2dx * (xs(1, 0, 0, -1) - xs(1, 0, 0, 1));
-                acc += (HX ? mz_im * P.idxdy - svx * P.i2dy : mz_im * P.idxdy) * (xs(0, 0, 0, -1) - xs(0, 0, 1, -1));
-                acc += (HX ? mz_i * P.idxdy + svx * P.i2dy : mz_i * P.idxdy) * (xs(0, 0, 1, 0) - xs(0, 0, 0, 0));
-                acc += (HZ ? mx_km * P.idydz - svz * P.i2dy : mx_km * P.idydz) * (xs(2, -1, 0, 0) - xs(2, -1, 1, 0));
-                acc += (HZ ? mx_k * P.idydz + svz * P.i2dy : mx_k * P.idydz) * (xs(2, 0, 1, 0) - xs(2, 0, 0, 0));
+                acc += (HX ? lk(mz_im, P.idxdy) - svx * P.i2dy : lk(mz_im, P.idxdy)) * (xs(0, 0, 0, -1) - xs(0, 0, 1, -1));
+                acc += (HX ? lk(mz_i, P.idxdy) + svx * P.i2dy : lk(mz_i, P.idxdy)) * (xs(0, 0, 1, 0) - xs(0, 0, 0, 0));
+                acc += (HZ ? lk(mx_km, P.idydz) - svz * P.i2dy : lk(mx_km, P.idydz)) * (xs(2, -1, 0, 0) - xs(2, -1, 1, 0));
+                acc += (HZ ? lk(mx_k, P.idydz) + svz * P.i2dy : lk(mx_k, P.idydz)) * (xs(2, 0, 1, 0) - xs(2, 0, 0, 0));
                 acc += s * P.idy * (xs(3, 0, 1, 0) - xs(3, 0, 0, 0));
-                emit(row, acc, d, true, xs(1, 0, 0, 0));
+                emit(row, acc, d, true, xs(1, 0, 0, 0), false);
             }
         }
         // ---------------------------------------------------------------- Az
         if (k <= g.zs) {
             const long long row = rZ;
             if (fijZ || kfZ) {
-                emit(row, xs(2, 0, 0, 0), T(1), true, xs(2, 0, 0, 0));
+                emit(row, xs(2, 0, 0, 0), T(1), true, xs(2, 0, 0, 0), true);
             } else {
                 const T s = cf(5, 0, 0, 0);
                 const T my_im = cf(1, 0, 0, -1), my_i = cf(1, 0, 0, 0);
                 const T mx_jm = cf(0, 0, -1, 0), mx_j = cf(0, 0, 0, 0);
                 const T mz_km = cf(2, -1, 0, 0), mz_k = cf(2, 0, 0, 0);
                 const T svx = HX ? s * P.vx : T(0), svy = HY ? s * P.vy : T(0);
-                const T d = (my_i + my_im) * P.idx2 + (mx_j + mx_jm) * P.idy2 + (mz_k + mz_km) * P.idz2 + s * P.idt;
+                const T d = lk(my_i + my_im, P.idx2) + lk(mx_j + mx_jm, P.idy2) + lk(mz_k + mz_km, P.idz2) + s * P.idt;
                 const T Z0 = xs(2, 0, 0, 0);
                 T acc = s * P.idt * Z0;
-                acc += mz_km * P.idz2 * (Z0 - xs(2, -1, 0, 0)) + mz_k * P.idz2 * (Z0 - xs(2, 1, 0, 0));
-                acc += mx_jm * P.idy2 * (Z0 - xs(2, 0, -1, 0)) + mx_j * P.idy2 * (Z0 - xs(2, 0, 1, 0));
-                acc += my_im * P.idx2 * (Z0 - xs(2, 0, 0, -1)) + my_i * P.idx2 * (Z0 - xs(2, 0, 0, 1));
+                acc += lk(mz_km, P.idz2) * (Z0 - xs(2, -1, 0, 0)) + lk(mz_k, P.idz2) * (Z0 - xs(2, 1, 0, 0));
+                acc += lk(mx_jm, P.idy2) * (Z0 - xs(2, 0, -1, 0)) + lk(mx_j, P.idy2) * (Z0 - xs(2, 0, 1, 0));
+                acc += lk(my_im, P.idx2) * (Z0 - xs(2, 0, 0, -1)) + lk(my_i, P.idx2) * (Z0 - xs(2, 0, 0, 1));
                 if constexpr (HY) acc += svy * P.i2dy * (xs(2, 0, -1, 0) - xs(2, 0, 1, 0));
                 if constexpr (HX) acc += svx * P.i2dx * (xs(2, 0, 0, -1) - xs(2, 0, 0, 1));
-                acc += (HX ? my_im * P.idxdz - svx * P.i2dz : my_im * P.idxdz) * (xs(0, 0, 0, -1) - xs(0, 1, 0, -1));
-                acc += (HX ? my_i * P.idxdz + svx * P.i2dz : my_i * P.idxdz) * (xs(0, 1, 0, 0) - xs(0, 0, 0, 0));
-                acc += (HY ? mx_jm * P.idydz - svy * P.i2dz : mx_jm * P.idydz) * (xs(1, 0, -1, 0) - xs(1, 1, -1, 0));
-                acc += (HY ? mx_j * P.idydz + svy * P.i2dz : mx_j * P.idydz) * (xs(1, 1, 0, 0) - xs(1, 0, 0, 0));
+                acc += (HX ? lk(my_im, P.idxdz) - svx * P.i2dz : lk(my_im, P.idxdz)) * (xs(0, 0, 0, -1) - xs(0, 1, 0, -1));
+                acc += (HX ? lk(my_i, P.idxdz) + svx * P.i2dz : lk(my_i, P.idxdz)) * (xs(0, 1, 0, 0) - xs(0, 0, 0, 0));
+                acc += (HY ? lk(mx_jm, P.idydz) - svy * P.i2dz : lk(mx_jm, P.idydz)) * (xs(1, 0, -1, 0) - xs(1, 1, -1, 0));
+                acc += (HY ? lk(mx_j, P.idydz) + svy * P.i2dz : lk(mx_j, P.idydz)) * (xs(1, 1, 0, 0) - xs(1, 0, 0, 0));
                 acc += s * P.idz * (xs(3, 1, 0, 0) - xs(3, 0, 0, 0));
-                emit(row, acc, d, true, xs(2, 0, 0, 0));
+                emit(row, acc, d, true, xs(2, 0, 0, 0), false);
             }
         }
         // ---------------------------------------------------------------- V
         {
             const long long row = rV;
             if (fijZ || kfA) {
-                emit(row, xs(3, 0, 0, 0), T(1), false, xs(3, 0, 0, 0));
+                emit(row, xs(3, 0, 0, 0), T(1), false, xs(3, 0, 0, 0), true);
             } else {
                 const T sx0 = cf(3, 0, 0, 0), sx1 = cf(3, 0, 0, -1);
                 const T sy0 = cf(4, 0, 0, 0), sy1 = cf(4, 0, -1, 0);
@@ -114,18 +131,19 @@ __device__ __forceinline__ void qms_op_node(const QGrid& g, const QStepPar<T>& P
                 const T fx0 = fmax(sx0, P.sigfloor), fx1 = fmax(sx1, P.sigfloor);
                 const T fy0 = fmax(sy0, P.sigfloor), fy1 = fmax(sy1, P.sigfloor);
                 const T fz0 = fmax(sz0, P.sigfloor), fz1 = fmax(sz1, P.sigfloor);
-                const T d = (fx0 + fx1) * P.idx2 + (fy0 + fy1) * P.idy2 + (fz0 + fz1) * P.idz2;
+                const T d = lk(fx0 + fx1, P.idx2) + lk(fy0 + fy1, P.idy2) + lk(fz0 + fz1, P.idz2);
                 const T V0 = xs(3, 0, 0, 0);
-                T acc = fz1 * P.idz2 * (V0 - xs(3, -1, 0, 0)) + fz0 * P.idz2 * (V0 - xs(3, 1, 0, 0));
-                acc += fy1 * P.idy2 * (V0 - xs(3, 0, -1, 0)) + fy0 * P.idy2 * (V0 - xs(3, 0, 1, 0));
-                acc += fx1 * P.idx2 * (V0 - xs(3, 0, 0, -1)) + fx0 * P.idx2 * (V0 - xs(3, 0, 0, 1));
+                T acc = lk(fz1, P.idz2) * (V0 - xs(3, -1, 0, 0)) + lk(fz0, P.idz2) * (V0 - xs(3, 1, 0, 0));
+                acc += lk(fy1, P.idy2) * (V0 - xs(3, 0, -1, 0)) + lk(fy0, P.idy2) * (V0 - xs(3, 0, 1, 0));
+                acc += lk(fx1, P.idx2) * (V0 - xs(3, 0, 0, -1)) + lk(fx0, P.idx2) * (V0 - xs(3, 0, 0, 1));
                 const T axm = xs(0, 0, 0, -1), ax0 = xs(0, 0, 0, 0);
                 const T aym = xs(1, 0, -1, 0), ay0 = xs(1, 0, 0, 0);
                 const T azm = xs(2, -1, 0, 0), az0 = xs(2, 0, 0, 0);
                 // div(sigma A) / dt: s0 a0 - s1 a1 = s0 (a0 - a1) + (s0 - s1) a1 (exact inside a body)
-                acc += P.idt * ((sx0 * (ax0 - axm) + (sx0 - sx1) * axm) * P.idx +
-                                (sy0 * (ay0 - aym) + (sy0 - sy1) * aym) * P.idy +
-                                (sz0 * (az0 - azm) + (sz0 - sz1) * azm) * P.idz);
+                const T jx = sx0 * (ax0 - axm) + (sx0 - sx1) * axm, jy = sy0 * (ay0 - aym) + (sy0 - sy1) * aym;
+                const T jz = sz0 * (az0 - azm) + (sz0 - sz1) * azm;
+                if constexpr (UNI) acc += P.idtx * (jx + jy + jz);
+                else acc += P.idt * (jx * P.idx + jy * P.idy + jz * P.idz);
                 // div(sigma v x curl A), grouped by velocity component into differences
                 const T vx = P.vx, vy = P.vy, vz = P.vz;
                 // Ax neighbours
@@ -170,7 +188,7 @@ __device__ __forceinline__ void qms_op_node(const QGrid& g, const QStepPar<T>& P
                     acc += vz * P.i2dy2 * (sy1 * (SC - (xs(2, -1, -1, 0) + xs(2, 0, -1, 0))) +
                                            sy0 * (SC - (xs(2, -1, 1, 0) + xs(2, 0, 1, 0))));
                 }
-                emit(row, acc, d, false, xs(3, 0, 0, 0));
+                emit(row, acc, d, false, xs(3, 0, 0, 0), false);
             }
         }
 }

@@ -45,11 +45,13 @@ __device__ __forceinline__ T op_div(T a, T d) {
     else return a / d;
 }
 
-// VM: the velocity components the advection term may use (qms_op_rows.cuh)
-template <typename T, int VM, int MODE>
+// VM: the velocity components the advection term may use; UNI: cubic cells, the rows in units of 1 / h^2
+// (qms_op_rows.cuh), iunit = h^2 (RESID, whose FP64 instructions bound it: GB300 issues two FP64
+// operations per clock and SM; 192x192x160 with a general velocity: 4.34 ms before, 3.92 now)
+template <typename T, int VM, int MODE, bool UNI = false>
 __global__ void __launch_bounds__(OTX * OTY, sizeof(T) == 4 ? QMS_STENCIL_MINB : 2)
 qk_operator_t(QGrid g, QCoef<T> c, QStepPar<T> P, const T* __restrict__ x, const T* __restrict__ b,
-              T* __restrict__ y, const T* __restrict__ w, double* __restrict__ partials) {
+              T* __restrict__ y, const T* __restrict__ w, double* __restrict__ partials, T iunit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileCoef<T>& tc = *reinterpret_cast<TileCoef<T>*>(smem_raw);
     XTile<T>& xt = *reinterpret_cast<XTile<T>*>(smem_raw + sizeof(TileCoef<T>));
@@ -66,10 +68,11 @@ qk_operator_t(QGrid g, QCoef<T> c, QStepPar<T> P, const T* __restrict__ x, const
     const int sZj = g.Nx, sZk = g.Nx * g.Ny;      // Az: (Nx, Ny, zs); V: (Nx, Ny, Nz)
     using RT = typename std::conditional<MODE == QOP_RESID, double, float>::type;
     RT red0 = 0, red1 = 0, red2 = 0, red3 = 0;
-    auto emit = [&](long long row, T acc, T diag, bool is_a, T xc_center) {
+    auto emit = [&](long long row, T acc, T diag, bool is_a, T xc_center, bool fixed) {
         T out;
         if (MODE == QOP_APPLY) out = acc;
         else if (MODE == QOP_SCALED) out = op_div(acc, diag);
+        else if (UNI) out = (fixed ? b[row] - acc : b[row] * iunit - acc) / diag;
         else out = (b[row] - acc) / diag;
         y[row] = out;
         if (partials) {
@@ -112,7 +115,7 @@ qk_operator_t(QGrid g, QCoef<T> c, QStepPar<T> P, const T* __restrict__ x, const
                 return xt.v[dk < 0 ? xm : (dk > 0 ? xp : x0)][comp][lj + dj][li + di];
             };
             auto cff = [&](int q, int dk, int dj, int di) -> T { return tc.c[dk < 0 ? prv : cur][q][lj + dj][li + di]; };
-            qms_op_node<T, VM>(g, P, i, j, k, fijX, fijY, fijZ, kfA, kfZ, rX, rY, rZ, rV, xsf, cff, emit);
+            qms_op_node<T, VM, UNI>(g, P, i, j, k, fijX, fijY, fijZ, kfA, kfZ, rX, rY, rZ, rV, xsf, cff, emit);
         }
         rX += sXk; rY += sYk; rZ += sZk; rV += sZk;
     }
@@ -224,7 +227,10 @@ static void qms_operator_prepare() {
     const int shm = (int)(sizeof(TileCoef<T>) + sizeof(XTile<T>));
     for (auto f : {qk_operator_t<T, 0, QOP_APPLY>, qk_operator_t<T, 0, QOP_SCALED>, qk_operator_t<T, 0, QOP_RESID>,
                    qk_operator_t<T, 7, QOP_APPLY>, qk_operator_t<T, 7, QOP_SCALED>, qk_operator_t<T, 7, QOP_RESID>,
-                   qk_operator_t<T, 1, QOP_RESID>, qk_operator_t<T, 2, QOP_RESID>, qk_operator_t<T, 4, QOP_RESID>})
+                   qk_operator_t<T, 1, QOP_RESID>, qk_operator_t<T, 2, QOP_RESID>, qk_operator_t<T, 4, QOP_RESID>,
+                   qk_operator_t<T, 0, QOP_RESID, true>, qk_operator_t<T, 1, QOP_RESID, true>,
+                   qk_operator_t<T, 2, QOP_RESID, true>, qk_operator_t<T, 4, QOP_RESID, true>,
+                   qk_operator_t<T, 7, QOP_RESID, true>})
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
@@ -235,21 +241,30 @@ void qms_launch_operator(const QGrid& g, const QCoef<T>& c, const QStepPar<T>& P
     dim3 bs = opt_block(), gs = opt_grid(g);
     const size_t shm = sizeof(TileCoef<T>) + sizeof(XTile<T>);
     qms_operator_prepare<T>();
-#define L(VM, MODE) qk_operator_t<T, VM, MODE><<<gs, bs, shm, st>>>(g, c, P, x, b, y, w, partials)
-    // the residual (the FP64 anchor of every solve) also has one instantiation per velocity axis
+#define L(VM, MODE) qk_operator_t<T, VM, MODE><<<gs, bs, shm, st>>>(g, c, P, x, b, y, w, partials, T(0))
+    // the residual (the FP64 anchor of every solve) also has one instantiation per velocity axis, and those
+    // for cubic cells
+#define LR(VM)                                                                                                  \
+    do {                                                                                                        \
+        if (g.dx == g.dy && g.dx == g.dz)                                                                       \
+            qk_operator_t<T, VM, QOP_RESID, true><<<gs, bs, shm, st>>>(g, c, qms_unit_par<T>(g, P), x, b, y, w, \
+                                                                       partials, (T)(g.dx * g.dx));             \
+        else L(VM, QOP_RESID);                                                                                  \
+    } while (0)
     const int m = (P.vx != T(0) ? 1 : 0) | (P.vy != T(0) ? 2 : 0) | (P.vz != T(0) ? 4 : 0);
     if (adv) {
         if (mode == QOP_APPLY) L(7, QOP_APPLY);
         else if (mode == QOP_SCALED) L(7, QOP_SCALED);
-        else if (m == 1) L(1, QOP_RESID);
-        else if (m == 2) L(2, QOP_RESID);
-        else if (m == 4) L(4, QOP_RESID);
-        else L(7, QOP_RESID);
+        else if (m == 1) LR(1);
+        else if (m == 2) LR(2);
+        else if (m == 4) LR(4);
+        else LR(7);
     } else {
         if (mode == QOP_APPLY) L(0, QOP_APPLY);
         else if (mode == QOP_SCALED) L(0, QOP_SCALED);
-        else L(0, QOP_RESID);
+        else LR(0);
     }
+#undef LR
 #undef L
 }
 

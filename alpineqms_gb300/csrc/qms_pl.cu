@@ -18,6 +18,7 @@
 #include <cudaTypedefs.h>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 
 // ---------------------------------------------------------------------------
 // Self-test of the bounded tile wait (mbar_wait_n, the wait every staged kernel uses): one CTA
@@ -120,10 +121,12 @@ __device__ __forceinline__ T pl_div(T a, T d) {
 // residual in double-float arithmetic, with w the residual of the anchor and x the change of
 // the solution since then).  Partials (optional, FP64 across warps): APPLY_A / SCALED [0] += y . w
 // (w may be null), [1] += y . y; RESID |r_A|^2, |r_V|^2; none with VCOUPLE.
-template <typename T, int VM, int MODE, typename YT = T, typename WT = T>
+// UNI: cubic cells, the rows in units of 1 / h^2 (qms_op_rows.cuh); `unit` is 1 / h^2 (APPLY_A).  FP64 inner
+// vectors, 64^3 run of steps: 334 -> 321 ms; in FP32 within the noise of a run.
+template <typename T, int VM, int MODE, bool UNI = false, typename YT = T, typename WT = T>
 __global__ void __launch_bounds__(OTX * OTY, sizeof(T) == 4 ? QMS_STENCIL_MINB : 2)
 qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap,
-         YT* y, const WT* w, double* partials, unsigned* err, WT* yfull) {
+         YT* y, const WT* w, double* partials, unsigned* err, WT* yfull, T unit) {
     // VCOUPLE reads only what the V rows' A couplings need: the three A blocks of x (xmap over
     // them) and the three conductivities (cmap over them)
     constexpr bool VC = MODE == QOPH_VCOUPLE;
@@ -181,7 +184,7 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
     // FP64 arithmetic per row would make the kernel FP64-throughput bound), FP64 across warps
     using RT = float;
     RT red0 = 0, red1 = 0;
-    auto emit = [&](long long row, T acc, T diag, bool is_a, T) {
+    auto emit = [&](long long row, T acc, T diag, bool is_a, T, bool fixed) {
         if constexpr (MODE == QOPH_RESID) {
             const T out = w[row] - acc / diag;
             y[row] = out.h;
@@ -195,7 +198,7 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
             if (!is_a) y[row] = w[row] - pl_div(acc, diag);
         } else {
             if (AO && !is_a) return;                   // the V row is not wanted (dead code)
-            const T out = AO ? acc : pl_div(acc, diag);
+            const T out = AO ? (UNI && !fixed ? acc * unit : acc) : pl_div(acc, diag);
             y[row] = out;
             if (partials) {
                 if (w) red0 += (RT)(out * w[row]);
@@ -229,7 +232,7 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
                 return (dk < 0 ? cprv : ccur)[((q - C0) * PLCY + lj + dj) * PLX + li + di];
             };
             const bool kfA = k <= 2 || k >= g.Nz - 1, kfZ = k == 1 || k == g.zs;
-            qms_op_node<T, VM>(g, P, i, j, k, fijX, fijY, fijZ, kfA, kfZ, rX, L.comp + rX, 2 * L.comp + rX,
+            qms_op_node<T, VM, UNI>(g, P, i, j, k, fijX, fijY, fijZ, kfA, kfZ, rX, L.comp + rX, 2 * L.comp + rX,
                                 3 * L.comp + rX, xsf, cff, emit);
         }
         rX += plane;
@@ -853,12 +856,17 @@ static int qms_vel_mask(const QStepPar<T>& P, bool adv, bool axes) {
 
 template <typename T, int VM>
 static void op_pl_attrs(int shm) {
-    if (VM == 0)
-        cudaFuncSetAttribute(qk_op_pl<T, 0, QOPH_APPLY_A>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)PLTiles<T, 3, 6>::SMEM);
-    cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
-    cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_VCOUPLE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)PLTiles<T, 3, 3>::SMEM);
+    auto one = [&](auto uni) {
+        constexpr bool U = decltype(uni)::value;
+        if (VM == 0)
+            cudaFuncSetAttribute(qk_op_pl<T, 0, QOPH_APPLY_A, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)PLTiles<T, 3, 6>::SMEM);
+        cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_SCALED, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
+        cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_VCOUPLE, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)PLTiles<T, 3, 3>::SMEM);
+    };
+    one(std::true_type());
+    one(std::false_type());
 }
 
 template <typename T>
@@ -876,11 +884,11 @@ static void op_pl_prepare() {
         op_pl_attrs<T, 2>(shm);
         op_pl_attrs<T, 4>(shm);
         const int shd = (int)PLTiles<qdf>::SMEM;
-        cudaFuncSetAttribute(qk_op_pl<qdf, 0, QOPH_RESID, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-        cudaFuncSetAttribute(qk_op_pl<qdf, 1, QOPH_RESID, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-        cudaFuncSetAttribute(qk_op_pl<qdf, 2, QOPH_RESID, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-        cudaFuncSetAttribute(qk_op_pl<qdf, 4, QOPH_RESID, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-        cudaFuncSetAttribute(qk_op_pl<qdf, 7, QOPH_RESID, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 0, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 1, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 2, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 4, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 7, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
     }
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
@@ -900,14 +908,20 @@ static void op_pl_launch(dim3 gs, dim3 bs, size_t shm, cudaStream_t st, int mode
     if constexpr (sizeof(T) == 8 && VM != 0 && VM != 7) {
         return;                                   // FP64 inner vectors: no or general advection only
     } else {
-        if (mode == QOPH_APPLY_A)                 // (no velocity: VM is 0)
-            pdl_launch(qk_op_pl<T, 0, QOPH_APPLY_A>, gs, bs, PLTiles<T, 3, 6>::SMEM, st, 0, g, P, xmap, cmap, y, w,
-                       partials, err, nullptr);
-        else if (mode == QOPH_VCOUPLE)
-            pdl_launch(qk_op_pl<T, VM, QOPH_VCOUPLE>, gs, bs, PLTiles<T, 3, 3>::SMEM, st, 0, g, P, xmap, cmap, y, w,
-                       partials, err, nullptr);
-        else
-            pdl_launch(qk_op_pl<T, VM, QOPH_SCALED>, gs, bs, shm, st, 0, g, P, xmap, cmap, y, w, partials, err, nullptr);
+        auto go = [&](auto uni, const QStepPar<T>& Q) {
+            constexpr bool U = decltype(uni)::value;
+            if (mode == QOPH_APPLY_A)             // (no velocity: VM is 0)
+                pdl_launch(qk_op_pl<T, 0, QOPH_APPLY_A, U>, gs, bs, PLTiles<T, 3, 6>::SMEM, st, 0, g, Q, xmap, cmap, y, w,
+                           partials, err, nullptr, P.idx2);
+            else if (mode == QOPH_VCOUPLE)
+                pdl_launch(qk_op_pl<T, VM, QOPH_VCOUPLE, U>, gs, bs, PLTiles<T, 3, 3>::SMEM, st, 0, g, Q, xmap, cmap, y, w,
+                           partials, err, nullptr, P.idx2);
+            else
+                pdl_launch(qk_op_pl<T, VM, QOPH_SCALED, U>, gs, bs, shm, st, 0, g, Q, xmap, cmap, y, w, partials, err,
+                           nullptr, P.idx2);
+        };
+        if (g.dx == g.dy && g.dx == g.dz) go(std::true_type(), qms_unit_par<T>(g, P));
+        else go(std::false_type(), P);
     }
 }
 
@@ -932,8 +946,8 @@ void qms_launch_resid_df(const QGrid& g, const QStepPar<qdf>& P, const CUtensorM
     const dim3 bs(OTX, OTY, 1), gs = qms_pl_tiles(g);
     const size_t shm = PLTiles<qdf>::SMEM;
     const int vm = qms_vel_mask(P, adv, true);
-    QMS_WITH_VM(vm, (pdl_launch(qk_op_pl<qdf, VM, QOPH_RESID, float, qdf>, gs, bs, shm, st, 0, g, P, xmap, cmap, r, b,
-                                partials, err, rfull)));
+    QMS_WITH_VM(vm, (pdl_launch(qk_op_pl<qdf, VM, QOPH_RESID, false, float, qdf>, gs, bs, shm, st, 0, g, P, xmap, cmap, r, b,
+                                partials, err, rfull, qdf(1))));
 }
 
 void qms_launch_delta_split(const QGrid& g, const double* x, const double* x0, qdf* dx, double* partials,

@@ -232,7 +232,7 @@ __device__ __forceinline__ T apply7(const MGLevelDev<T>& L, const MGBlockDesc& B
 // meet a zero link).  All loads of a point are independent, and those of the geometry's links precede the
 // wait for the kernel before.  Passes of a level per cycle: 6 instead of 8 (the first two sweeps in one, the
 // prolongation with the sweep after it), without index divisions and the diagonal array: 96^3 ellipsoids 168
-// -> 163 ms a run, 128^3 209 -> 204, moving plate 256^3 667 -> 645.
+// -> 163 ms a run, 128^3 209 -> 204, moving plate 256^3 673 -> 647 from one state and 642 -> 643 from another.
 template <typename T>
 struct MGPoint {
     long long nb[6];                            // neighbours: +1, -1, +n1, -n1, +s3, -s3

@@ -224,6 +224,20 @@ __device__ __forceinline__ T apply7(const MGLevelDev<T>& L, const MGBlockDesc& B
     return acc;
 }
 
+#define MGC_SWEEPS 8                            // a side: up to this many sweeps have weights of their own
+// Weight of sweep s of nu on one side of the cycle: the reciprocal Chebyshev nodes of [0.4, 2], scaled by
+// omega / 0.85; one sweep, or more than MGC_SWEEPS: omega.  Their product polynomial is at most 1 / T_3(1.5)
+// = 0.11 there for three sweeps; three of weight 0.85 reach 0.34 at 2.  Both sides take the same weights and
+// the factors commute, so the cycle stays symmetric.  FGMRES steps a run, equal weights -> these: 96^3 494 ->
+// 486, 128^3 336 -> 326, moving plate 256^3 178 -> 167, core 832 -> 800.  Intervals from 0.3, 0.5 and 0.8:
+// 256^3 173, 165 and 182, 128^3 326, 328 and 334.
+template <typename T>
+static inline T mg_weight(T omega, int s, int nu) {
+    if (nu < 2 || nu > MGC_SWEEPS) return omega;
+    const double a = 0.4, b = 2.0, c = std::cos(3.14159265358979323846 * (2 * s + 1) / (2.0 * nu));
+    return (T)((double)omega / 0.85 / (0.5 * (b + a) - 0.5 * (b - a) * c));
+}
+
 // ------------------------------------------------------------------ smoother
 // Weighted Jacobi on a level of stored links, x' = (1 - omega) x + omega D^-1 (b + sum w x_n); inactive
 // points have D^-1 = 0 and stay zero.  Links to points beyond the block's faces are zero, and so are the
@@ -263,7 +277,7 @@ __global__ void mg_smooth0(MGLevelDev<T> L, const T* b, T omega, T* x) {
 // the first two sweeps from a zero guess in one pass: x_1 = omega D^-1 b formed at the point and its
 // neighbours (a launch and two passes over x less than apart)
 template <typename T>
-__global__ void __launch_bounds__(256) mg_smooth01(MGLevelDev<T> L, const T* b, T omega, T* x) {
+__global__ void __launch_bounds__(256) mg_smooth01(MGLevelDev<T> L, const T* b, T omega1, T omega, T* x) {
     long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const bool in = t < L.total;
     if (!in) t = 0;
@@ -276,8 +290,8 @@ __global__ void __launch_bounds__(256) mg_smooth01(MGLevelDev<T> L, const T* b, 
     const T bv = b[t];
     T sum = bv;
 #pragma unroll
-    for (int e = 0; e < 6; e++) sum += P.w[e] * (omega * dn[e] * b[P.nb[e]]);
-    if (in) x[t] = (T(1) - omega) * di * bv + di * sum;
+    for (int e = 0; e < 6; e++) sum += P.w[e] * (omega1 * dn[e] * b[P.nb[e]]);
+    if (in) x[t] = (T(1) - omega) * (omega1 * L.dinv[t]) * bv + di * sum;
 }
 
 // x_out = x_in + omega D^-1 (b - A x_in)
@@ -381,6 +395,7 @@ template <typename T>
 struct MGSub {
     int nl;                                     // levels; the last is the coarsest
     int lg;                                     // 2^lg CTAs in the cluster
+    T w1[MGC_SWEEPS], w2[MGC_SWEEPS];           // weights of the sweeps before and after the correction
     MGLevelDev<T> L[MGC_LEVELS];
 };
 // planes of a level that one CTA of 2^lg holds, and the shared memory (elements) of a level: two copies of x
@@ -469,7 +484,7 @@ struct MGCluster {
 template <typename T>
 __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__ MGSub<T> sub,
                                                        const double* __restrict__ minv,
-                                                       const long long* __restrict__ moff, T omega, T alpha, int nu1,
+                                                       const long long* __restrict__ moff, T alpha, int nu1,
                                                        int nu2) {
     const int lg = sub.lg, size = 1 << lg, b = blockIdx.x >> lg, last = sub.nl - 1, tid = threadIdx.x;
     const int m = sub.L[last].blk[b].n1 * sub.L[last].blk[b].n2 * sub.L[last].blk[b].n3;
@@ -534,11 +549,11 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
         const MGSlab S = slab(l), SC = slab(l + 1);
         if (!S.spread && c != 0) break;
 #pragma unroll 2
-        for (int q = tid; q < S.np; q += MGC_THREADS) G.put(S, S.x, q, omega * G.sm[S.w + S.s3 + q] * G.sm[S.b + q]);
+        for (int q = tid; q < S.np; q += MGC_THREADS) G.put(S, S.x, q, sub.w1[0] * G.sm[S.w + S.s3 + q] * G.sm[S.b + q]);
         G.sync(S.spread);
         int cur = 0;
 #pragma unroll 1
-        for (int s = 1; s < nu1; s++) G.sweep(S, cur, omega);
+        for (int s = 1; s < nu1; s++) G.sweep(S, cur, sub.w1[s & (MGC_SWEEPS - 1)]);
         const int X = S.x + cur * S.xlen, R = S.x + (cur ^ 1) * S.xlen;   // the residual into the other copy
 #pragma unroll 2
         for (int q = tid; q < S.np; q += MGC_THREADS) {
@@ -615,7 +630,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
         G.sync(S.spread);
         int cur = down;
 #pragma unroll 1
-        for (int s = 0; s < nu2; s++) G.sweep(S, cur, omega);
+        for (int s = 0; s < nu2; s++) G.sweep(S, cur, sub.w2[s & (MGC_SWEEPS - 1)]);
     }
     if (last > 0) {
         const MGSlab S = slab(0);
@@ -684,7 +699,7 @@ __device__ __forceinline__ double mg_cf(double v) { return v; }
 
 template <typename T, int KIND, int QS, bool UNI, int ROWS>
 __global__ void __launch_bounds__(OTX * OTY / ROWS, sizeof(T) == 4 ? (ROWS == 1 ? QMS_STENCIL_MINB : 6) : 2)
-mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, const T* b, int scaled,
+mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, T omega1, const T* b, int scaled,
           const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap cmap, T* xout,
           MGLevelDev<T> C, T* bc, unsigned* err) {
     using S = MG0Set<QS>;
@@ -838,11 +853,11 @@ mg0_tiled(QGrid g, QStepPar<T> P, T vshift, T omega, const T* b, int scaled,
                     res[q] += scaled ? unit * (bv[q][r] * d * isc - Ax) : bv[q][r] - unit * Ax;
                 } else {
                     const T nb = wxp * xip + wxm * xim + wyp * xjp + wym * xjm + wzp * xp[r] + wzm * xm[q][r];
-                    // KIND 3: the staged values are b; x_1 = c b with c = omega isc, and the neighbours' sum
-                    // scales with it
+                    // KIND 3: the staged values are b; x_1 = c b with c = omega1 isc, and the neighbours' sum
+                    // scales with it (omega1: the first sweep's weight, omega: the second's)
                     if (KIND == 3) {
-                        const T cq = omega * isc;
-                        xout[row] = cq * ((T(2) - omega) * xs + omega * nb * mg_rcp(d));
+                        const T cq = omega1 * isc;
+                        xout[row] = ((T(1) - omega) * cq + omega * isc) * xs + omega * cq * (nb * mg_rcp(d));
                     } else if (scaled) {
                         xout[row] = (T(1) - omega) * xs + omega * (isc * bv[q][r] + nb * mg_rcp(d));
                     } else {
@@ -1372,22 +1387,23 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     struct Buf { T* p; const CUtensorMap* m; };
     // level-0 sweeps: KIND 0 writes XO from b; KIND 1 reads XI (tile copies) and writes XO;
     // KIND 2 reads XI and writes the level-1 right-hand side
-#define MG0U(KIND, XI, XO, BC, UNI, ROWS)                                                                         \
+#define MG0U(KIND, XI, XO, BC, OM, OM1, UNI, ROWS)                                                               \
     pdl_launch(mg0_tiled<T, KIND, QS, UNI, ROWS>, g0grid, dim3(OTX, OTY / ROWS), mg0_smem<T, KIND, QS>(), st, 0,  \
-               g0, P0, vshift0, omega, b0, sc, *(XI).m, cmap, (XO), lv[1], (BC), err)
-#define MG0(KIND, XI, XO, BC)                                                                                     \
+               g0, P0, vshift0, (OM), (OM1), b0, sc, *(XI).m, cmap, (XO), lv[1], (BC), err)
+#define MG0(KIND, XI, XO, BC, OM, OM1)                                                                           \
     do {                                                                                                          \
         if (ROWS2 > 1 && two) {                                                                                   \
-            if (cubic) MG0U(KIND, XI, XO, BC, true, ROWS2);                                                       \
-            else MG0U(KIND, XI, XO, BC, false, ROWS2);                                                            \
+            if (cubic) MG0U(KIND, XI, XO, BC, OM, OM1, true, ROWS2);                                             \
+            else MG0U(KIND, XI, XO, BC, OM, OM1, false, ROWS2);                                                  \
         } else {                                                                                                  \
-            if (cubic) MG0U(KIND, XI, XO, BC, true, 1);                                                           \
-            else MG0U(KIND, XI, XO, BC, false, 1);                                                                \
+            if (cubic) MG0U(KIND, XI, XO, BC, OM, OM1, true, 1);                                                 \
+            else MG0U(KIND, XI, XO, BC, OM, OM1, false, 1);                                                      \
         }                                                                                                         \
     } while (0)
     // rows per thread: two on grids of many tiles (FP32)
     constexpr int ROWS2 = sizeof(T) == 4 ? 2 : 1;
     const bool two = (long long)g0grid.x * g0grid.y * g0grid.z >= QMS_CTA_TARGET;
+    auto wgt = [&](int s, int nu) { return mg_weight<T>(omega, s, nu); };
     const bool cubic = P0.idx2 == P0.idy2 && P0.idx2 == P0.idz2;
     // level 0: nu1 + nu2 sweeps alternate between x0 and t0 (the prolongation is in place);
     // start in t0 when that count is even so that the last write lands in x0
@@ -1398,28 +1414,28 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
         // the first two sweeps in one pass, from b's tiles (KIND 3), into the buffer the second
         // sweep writes
         Buf bb{const_cast<T*>(b0), b0map};
-        MG0(3, bb, t.p, nullptr);
+        MG0(3, bb, t.p, nullptr, wgt(1, n1), wgt(0, n1));
         std::swap(x, t);
         launches++;
         s = 2;
     } else {
-        MG0(0, x, x.p, nullptr);
+        MG0(0, x, x.p, nullptr, wgt(0, n1), T(0));
         launches++;
     }
     // the A-block sweeps are the largest single kernel of a transient step: optionally timed,
     // with their algorithmic bytes (x and b read, x written, one material byte per cell)
     const double asweep_bytes = 3.0 * sizeof(T) * (double)g0.oV + (double)g0.xs * g0.ys * g0.zs;
-    auto sweep = [&](Buf& xi, T* xo) {
+    auto sweep = [&](Buf& xi, T* xo, T om) {
         void* tok = (QS == 1 && prof) ? prof->begin(MGPROF_A_SWEEP, asweep_bytes) : nullptr;
-        MG0(1, xi, xo, nullptr);
+        MG0(1, xi, xo, nullptr, om, T(0));
         if (tok) prof->end(tok);
     };
     for (; s < n1; s++) {
-        sweep(x, t.p);
+        sweep(x, t.p, wgt(s, n1));
         std::swap(x, t);
         launches++;
     }
-    MG0(2, x, nullptr, lv[1].b);
+    MG0(2, x, nullptr, lv[1].b, omega, T(0));
     launches++;
     // levels >= 1: nu_coarse sweeps on each side when set
     const int nuc1 = (QS == 2 && nu_v > 0) ? nu_v : (nu_coarse > 0 ? nu_coarse : nu1);
@@ -1432,22 +1448,23 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
             MGSub<T> sub{};
             sub.nl = nl - lt;
             sub.lg = sub_lg;
+            for (int q = 0; q < MGC_SWEEPS; q++) { sub.w1[q] = wgt(q, nuc1); sub.w2[q] = wgt(q, nuc2); }
             for (int q = 0; q < sub.nl; q++) sub.L[q] = lv[lt + q];
             pdl_launch(mg_sub<T>, dim3(L.nb << sub_lg), dim3(MGC_THREADS), sub_smem[QS], st, 1u << sub_lg, sub, dminv, dmo,
-                       omega, alpha, nuc1, nuc2);
+                       alpha, nuc1, nuc2);
             launches++;
             break;
         }
         T* xl = L.x;
         T* tl = L.t;
         if (nuc1 >= 2) {
-            pdl_launch(mg_smooth01<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl);
+            pdl_launch(mg_smooth01<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, wgt(0, nuc1), wgt(1, nuc1), xl);
         } else {
-            pdl_launch(mg_smooth0<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl);
+            pdl_launch(mg_smooth0<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, wgt(0, nuc1), xl);
         }
         launches++;
         for (int s = 2; s < nuc1; s++) {
-            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl);
+            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, wgt(s, nuc1), xl, tl);
             std::swap(xl, tl);
             launches++;
         }
@@ -1468,12 +1485,12 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
         MGLevelDev<T>& L = lv[l];
         T* xl = L.x;
         T* tl = L.t;
-        pdl_launch(mg_prolong_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl, lv[l + 1],
+        pdl_launch(mg_prolong_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, wgt(0, nuc2), xl, tl, lv[l + 1],
                    lv[l + 1].x, alpha);
         std::swap(xl, tl);
         launches++;
         for (int s = 1; s < nuc2; s++) {
-            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, omega, xl, tl);
+            pdl_launch(mg_smooth<T>, dim3(nblk(L.total)), dim3(256), 0, st, 0, L, L.b, wgt(s, nuc2), xl, tl);
             std::swap(xl, tl);
             launches++;
         }
@@ -1485,7 +1502,7 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
                dim3(MGP_X, MGP_Y), 0, st, 0, g0, x.p, lv[1], lv[1].x, alpha);
     launches++;
     for (int s = 0; s < n2; s++) {
-        sweep(x, t.p);
+        sweep(x, t.p, wgt(s, n2));
         std::swap(x, t);
         launches++;
     }

@@ -85,7 +85,8 @@ typedef struct {
     int device;              /* CUDA device ordinal */
     int precond;             /* QMS_PRECOND_MG (default) or QMS_PRECOND_JACOBI */
     int mg_sweeps;           /* Jacobi sweeps before and after each coarse correction */
-    double mg_omega;         /* Jacobi weight */
+    double mg_omega;         /* scale of the Jacobi weights (of the one sweep, or of the Chebyshev weights of
+                                several; 0.85 by default) */
     double mg_vshift;        /* relative diagonal shift of the preconditioner's V block (0 by default:
                                 the coarsest V solve is a pseudo-inverse that drops the floating
                                 potential of isolated conductors) */

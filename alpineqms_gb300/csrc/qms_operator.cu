@@ -47,7 +47,8 @@ __device__ __forceinline__ T op_div(T a, T d) {
 
 // VM: the velocity components the advection term may use; UNI: cubic cells, the rows in units of 1 / h^2
 // (qms_op_rows.cuh), iunit = h^2 (RESID, whose FP64 instructions bound it: GB300 issues two FP64
-// operations per clock and SM; 192x192x160 with a general velocity: 4.34 ms before, 3.92 now)
+// operations per clock and SM; 192x192x160 with a general velocity: 4.34 ms before, 3.92 now;
+// error against 64-bit rows 1.3e-16 and 2.3e-16 before, 2.3e-16 and 2.8e-16 now: the products' other grouping)
 template <typename T, int VM, int MODE, bool UNI = false>
 __global__ void __launch_bounds__(OTX * OTY, sizeof(T) == 4 ? QMS_STENCIL_MINB : 2)
 qk_operator_t(QGrid g, QCoef<T> c, QStepPar<T> P, const T* __restrict__ x, const T* __restrict__ b,

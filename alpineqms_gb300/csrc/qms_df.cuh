@@ -76,12 +76,15 @@ __device__ __forceinline__ qdf fmax(qdf a, qdf b) { return (a.h > b.h || (a.h ==
 // Split of a double into a qdf with integer operations only (no FP64 instruction): the high
 // word keeps the leading 24 significant bits (truncated), the low word the float nearest to
 // the remaining 29 bits.  Magnitudes below 2^-126 give 0, and the low word below 2^-74 is
-// dropped (absolute errors under 1e-29); values this small do not occur in the solver.
+// dropped (absolute errors under 1e-29); values this small do not occur in the solver.  Values from
+// 2^128 up, infinities and NaN give an infinity: a state that is not finite has to show in the residual
+// (as zeros it looked like one that a cycle had not changed).
 __device__ __forceinline__ qdf qdf_split(double d) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(d);
     const unsigned e = (unsigned)(u >> 52) & 0x7FFu;
-    if (e < 897u || e > 1150u) return qdf(0.f, 0.f);
+    if (e < 897u) return qdf(0.f, 0.f);
     const unsigned sign = (unsigned)(u >> 63) << 31;
+    if (e > 1150u) return qdf(__uint_as_float(sign | 0x7F800000u), 0.f);
     const float h = __uint_as_float(sign | ((e - 896u) << 23) | ((unsigned)(u >> 29) & 0x7FFFFFu));
     const unsigned mlo = (unsigned)(u & 0x1FFFFFFFull);
     float l = 0.f;

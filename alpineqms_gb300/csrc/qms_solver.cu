@@ -1540,6 +1540,21 @@ int QmsSolver::step_graph(bool adv, const double v[3], const QStepStart& hs, boo
     return 0;
 }
 
+// The inner vectors' padding and the Dirichlet rows beyond the tiles are zero and read by the sums over
+// whole vectors, and no kernel of a solve writes them but in such a sum's wake: a projection that is not
+// finite puts NaN there, where 0 * NaN would end every later solve too.
+int QmsSolver::clear_inner() {
+    auto clear = [&](void* p, size_t es) { return p ? cudaMemsetAsync(p, 0, npl * es, st) : cudaSuccess; };
+    for (void* p : vec) CK(clear(p, tsize));
+    for (void* p : gmV) CK(clear(p, tsize));
+    for (void* p : gmZ) CK(clear(p, tsize));
+    CK(clear(mgtmp, tsize));
+    CK(clear(mgtmp2, tsize));
+    CK(clear(rpl, 4));
+    for (qdf* p : {xdf, r0df, rfin, wh[0], wh[1], wh[2], wh[3]}) CK(clear(p, 8));
+    return 0;
+}
+
 int QmsSolver::solve(bool transient, const double v[3], const double B[3], const double G[9]) {
     CK(cudaSetDevice(dev));
     QmsExcite ex;
@@ -1828,6 +1843,7 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
     stats.status |= stt & ~(unsigned)QMS_ST_BREAKDOWN;
     stats.outer_iterations = outer;
     stats.final_residual = rel;
+    if (stats.status & QMS_ST_NAN) return clear_inner();
     return 0;
 }
 

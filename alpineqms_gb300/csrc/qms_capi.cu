@@ -250,6 +250,7 @@ int qms_set_state(qms_handle* h, const double* x_in) {
     h->s.hist_len = 0;             // ... and has no history to extrapolate
     h->s.w_len = 0;
     h->s.last_chained = false;
+    h->s.forget_counts();          // ... and its run does not depend on the runs before
     return 0;
 }
 

@@ -873,10 +873,7 @@ size_t qms_device_bytes_impl(const qms_desc& d) {
 int QmsSolver::set_materials(const uint8_t* host_slots, const double* rows6, int nmat) {
     CK(cudaSetDevice(dev));
     drop_graphs();
-    gm_k_est = 0;
-    gm_rate = 0.0;
-    gm_ls_floor = 0;
-    gm_ls_floor_age = 0;
+    forget_counts();
     if (nmat < 0 || nmat > QMS_MAX_SLOTS - 1) { err = "nmat must be in 0..255"; return QMS_ERR_ARG; }
     const long long ncell = (long long)g.xs * g.ys * g.zs;
     if (host_slots) {

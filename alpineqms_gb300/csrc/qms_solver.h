@@ -231,6 +231,13 @@ struct QmsSolver {
     int gm_ls_floor = 0;        // its lowest value for now, and that value's age in solves
     int gm_ls_floor_age = 0;
     double gm_rate = 0.0;       // log of the residual estimate per FGMRES step, smoothed over cycles
+    // what a run's solves leave for its later ones; a state that is set starts a run, whose results then
+    // are the same whatever the handle solved before
+    void forget_counts() {
+        gm_k_est = 0;
+        gm_rate = 0.0;
+        gm_ls_floor = gm_ls_floor_age = 0;
+    }
     void* gmV[65] = {};         // FGMRES basis (m + 1) and preconditioned directions (m), m <= 64
     void* gmZ[64] = {};
     double* gm_H = nullptr;     // Hessenberg matrix (m+1) x m, row-major with stride m

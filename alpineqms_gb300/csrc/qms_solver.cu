@@ -20,6 +20,7 @@
 #include "qms_pl.h"
 
 #include <atomic>
+#include <chrono>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -1223,8 +1224,20 @@ int QmsSolver::inner_gmres(bool adv, bool transient, const double v[3], int& ite
     return 0;
 }
 
+static double wall_s() {
+    return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count();
+}
+
 // Steps j0 .. j0 + kSeg - 1 of a cycle as one CUDA graph, captured once per j0 for the operator of
-// this solve and replayed; the operator of another velocity starts over.
+// this solve and replayed; the operator of another velocity starts over.  Until then the steps are
+// launched directly: kSegDirect times (a replay saves some 10 us over direct launches, a capture alone
+// takes 0.2 to 0.7 ms), and for as long as captures would take more than an eighth of the time that the
+// handle has spent in cycles.  Among 16 solves that share the driver's locks a capture takes 50 to 100 ms,
+// up to 0.7 s while requests are being set up: first steps that captured all of their segments took up
+// to 1.8 s.  24 requests at 50 ms, 99th percentile of a step with 10 (50) steps each: 1.1-1.8 s
+// (0.38-0.46) with captures at once, 0.51-0.77 (0.43-0.62) so, 0.49-0.90 by the eighth alone, 0.51-0.64
+// and 0.34-0.41 from 32 and 48 direct launches on.  Repeated runs of 48^3 take 2 and 5 % longer with
+// the latter two; first runs on 16x14x12 and 32^3 take 3.5 and 2 % longer so than with captures at once.
 int QmsSolver::gmres_segment(bool adv, bool transient, const double v[3], int j0, int j1, bool graph) {
     auto steps = [&] {
         if (fp64_inner) gmres_steps<double>(adv, transient, v, j0, j1);
@@ -1244,7 +1257,14 @@ int QmsSolver::gmres_segment(bool adv, bool transient, const double v[3], int j0
     const size_t at = (size_t)(j0 / kSeg);
     if (segs.size() <= at) segs.resize(at + 1);
     SegGraph& G = segs[at];
+    if (!G.exec && (G.direct < kSegDirect || capture_s + capture_last_s > cycles_s / 8)) {
+        G.direct = std::min(G.direct + 1, kSegDirect);
+        steps();
+        CK(cudaGetLastError());
+        return 0;
+    }
     if (!G.exec) {
+        const double t0 = wall_s();
         const long long n0 = nlaunch;
         CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
         steps();
@@ -1254,6 +1274,8 @@ int QmsSolver::gmres_segment(bool adv, bool transient, const double v[3], int j0
         if (graph_) cudaGraphDestroy(graph_);
         G.launches = nlaunch - n0;
         nlaunch = n0;
+        capture_last_s = wall_s() - t0;
+        capture_s += capture_last_s;
         if (e != cudaSuccess) {
             cudaGetLastError();
             G.exec = nullptr;
@@ -1273,6 +1295,7 @@ int QmsSolver::gmres_segment(bool adv, bool transient, const double v[3], int j0
 // motion: 84 steps per time step instead of 28).
 int QmsSolver::gmres_cycle(bool adv, bool transient, const double v[3], double stop, bool graph, int& iters) {
     const int m = std::min(desc.gmres_m, GM_MAXM);
+    const double t0 = wall_s();
     if (fp64_inner) gmres_begin<double>();
     else gmres_begin<float>();
     int k = 0, upto = kSeg;
@@ -1297,6 +1320,7 @@ int QmsSolver::gmres_cycle(bool adv, bool transient, const double v[3], double s
     }
     if (fp64_inner) gmres_end<double>(k);
     else gmres_end<float>(k);
+    cycles_s += wall_s() - t0;
     iters = k;
     CK(cudaGetLastError());
     return 0;

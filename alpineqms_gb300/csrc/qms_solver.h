@@ -196,15 +196,18 @@ struct QmsSolver {
     int gmres_segment(bool adv, bool transient, const double v[3], int j0, int j1, bool graph);
     int gmres_cycle(bool adv, bool transient, const double v[3], double stop, bool graph, int& iters);
     // kSeg steps of an FGMRES cycle captured as one graph, for the operator (seg_tr, seg_v)
-    static constexpr int kSeg = 2;
+    static constexpr int kSeg = 2, kSegDirect = 16;
     struct SegGraph {
         cudaGraphExec_t exec = nullptr;
         long long launches = 0;
+        int direct = 0;             // launches without the graph
     };
     std::vector<SegGraph> segs;
     bool seg_valid = false, seg_tr = false;
     double seg_v[3] = {0, 0, 0};
     void drop_segments();
+    // seconds spent in cycles and in captures of their segments so far, and in the last capture
+    double cycles_s = 0.0, capture_s = 0.0, capture_last_s = 2e-4;
     // Whole chained transient steps as one CUDA graph each: the status reset, the step start (its
     // rotating history pointers copied from pinned host memory by a node of the graph), the start
     // residual, and a conditional WHILE node whose body is one refinement cycle (FGMRES with k

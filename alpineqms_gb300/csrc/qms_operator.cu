@@ -45,14 +45,16 @@ __device__ __forceinline__ T op_div(T a, T d) {
     else return a / d;
 }
 
-// VM: the velocity components the advection term may use; UNI: cubic cells, the rows in units of 1 / h^2
-// (qms_op_rows.cuh), iunit = h^2 (RESID, whose FP64 instructions bound it: GB300 issues two FP64
-// operations per clock and SM; 192x192x160 with a general velocity: 4.34 ms before, 3.92 now;
-// error against 64-bit rows 1.3e-16 and 2.3e-16 before, 2.3e-16 and 2.8e-16 now: the products' other grouping)
-template <typename T, int VM, int MODE, bool UNI = false>
+// VM: the velocity components the advection term may use; UNI: cubic cells, the rows' links in units of
+// 1 / h^2 and the terms in 1 / dt apart (qms_op_rows.cuh, QROW_TIME), unit = 1 / h^2 (RESID, whose FP64
+// instructions bound it: GB300 issues two FP64 operations per clock and SM; 192x192x160 with a general
+// velocity: 4.34 ms with general rows, 3.92 so).  Error against rows in 80 bits, mean of 32 states
+// (24x20x17 and 37x33x12): 1.70e-16 with general rows, 1.42e-16 so, 1.84e-16 with the time terms in the
+// unit too; plain 64-bit arithmetic is 1.94e-16 off.
+template <typename T, int VM, int MODE, int UNI = QROW_PLAIN>
 __global__ void __launch_bounds__(OTX * OTY, sizeof(T) == 4 ? QMS_STENCIL_MINB : 2)
 qk_operator_t(QGrid g, QCoef<T> c, QStepPar<T> P, const T* __restrict__ x, const T* __restrict__ b,
-              T* __restrict__ y, const T* __restrict__ w, double* __restrict__ partials, T iunit) {
+              T* __restrict__ y, const T* __restrict__ w, double* __restrict__ partials, T unit) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TileCoef<T>& tc = *reinterpret_cast<TileCoef<T>*>(smem_raw);
     XTile<T>& xt = *reinterpret_cast<XTile<T>*>(smem_raw + sizeof(TileCoef<T>));
@@ -69,11 +71,14 @@ qk_operator_t(QGrid g, QCoef<T> c, QStepPar<T> P, const T* __restrict__ x, const
     const int sZj = g.Nx, sZk = g.Nx * g.Ny;      // Az: (Nx, Ny, zs); V: (Nx, Ny, Nz)
     using RT = typename std::conditional<MODE == QOP_RESID, double, float>::type;
     RT red0 = 0, red1 = 0, red2 = 0, red3 = 0;
-    auto emit = [&](long long row, T acc, T diag, bool is_a, T xc_center, bool fixed) {
+    auto emit = [&](long long row, T acc, T diag, bool is_a, T xc_center, bool fixed, T tacc, T tdiag) {
         T out;
         if (MODE == QOP_APPLY) out = acc;
         else if (MODE == QOP_SCALED) out = op_div(acc, diag);
-        else if (UNI) out = (fixed ? b[row] - acc : b[row] * iunit - acc) / diag;
+        else if (UNI) {
+            const T u = fixed ? T(1) : unit;
+            out = ((b[row] - tacc) - u * acc) / (tdiag + u * diag);
+        }
         else out = (b[row] - acc) / diag;
         y[row] = out;
         if (partials) {
@@ -229,9 +234,9 @@ static void qms_operator_prepare() {
     for (auto f : {qk_operator_t<T, 0, QOP_APPLY>, qk_operator_t<T, 0, QOP_SCALED>, qk_operator_t<T, 0, QOP_RESID>,
                    qk_operator_t<T, 7, QOP_APPLY>, qk_operator_t<T, 7, QOP_SCALED>, qk_operator_t<T, 7, QOP_RESID>,
                    qk_operator_t<T, 1, QOP_RESID>, qk_operator_t<T, 2, QOP_RESID>, qk_operator_t<T, 4, QOP_RESID>,
-                   qk_operator_t<T, 0, QOP_RESID, true>, qk_operator_t<T, 1, QOP_RESID, true>,
-                   qk_operator_t<T, 2, QOP_RESID, true>, qk_operator_t<T, 4, QOP_RESID, true>,
-                   qk_operator_t<T, 7, QOP_RESID, true>})
+                   qk_operator_t<T, 0, QOP_RESID, QROW_TIME>, qk_operator_t<T, 1, QOP_RESID, QROW_TIME>,
+                   qk_operator_t<T, 2, QOP_RESID, QROW_TIME>, qk_operator_t<T, 4, QOP_RESID, QROW_TIME>,
+                   qk_operator_t<T, 7, QOP_RESID, QROW_TIME>})
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
@@ -248,8 +253,8 @@ void qms_launch_operator(const QGrid& g, const QCoef<T>& c, const QStepPar<T>& P
 #define LR(VM)                                                                                                  \
     do {                                                                                                        \
         if (g.dx == g.dy && g.dx == g.dz)                                                                       \
-            qk_operator_t<T, VM, QOP_RESID, true><<<gs, bs, shm, st>>>(g, c, qms_unit_par<T>(g, P), x, b, y, w, \
-                                                                       partials, (T)(g.dx * g.dx));             \
+            qk_operator_t<T, VM, QOP_RESID, QROW_TIME><<<gs, bs, shm, st>>>(                                    \
+                g, c, qms_unit_par<T>(g, P, QROW_TIME), x, b, y, w, partials, P.idx2);                          \
         else L(VM, QOP_RESID);                                                                                  \
     } while (0)
     const int m = (P.vx != T(0) ? 1 : 0) | (P.vy != T(0) ? 2 : 0) | (P.vz != T(0) ? 4 : 0);

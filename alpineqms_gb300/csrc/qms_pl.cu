@@ -184,7 +184,7 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
     // FP64 arithmetic per row would make the kernel FP64-throughput bound), FP64 across warps
     using RT = float;
     RT red0 = 0, red1 = 0;
-    auto emit = [&](long long row, T acc, T diag, bool is_a, T, bool fixed) {
+    auto emit = [&](long long row, T acc, T diag, bool is_a, T, bool fixed, T, T) {
         if constexpr (MODE == QOPH_RESID) {
             const T out = w[row] - acc / diag;
             y[row] = out.h;
@@ -232,7 +232,7 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
                 return (dk < 0 ? cprv : ccur)[((q - C0) * PLCY + lj + dj) * PLX + li + di];
             };
             const bool kfA = k <= 2 || k >= g.Nz - 1, kfZ = k == 1 || k == g.zs;
-            qms_op_node<T, VM, UNI>(g, P, i, j, k, fijX, fijY, fijZ, kfA, kfZ, rX, L.comp + rX, 2 * L.comp + rX,
+            qms_op_node<T, VM, UNI ? QROW_UNIT : QROW_PLAIN>(g, P, i, j, k, fijX, fijY, fijZ, kfA, kfZ, rX, L.comp + rX, 2 * L.comp + rX,
                                 3 * L.comp + rX, xsf, cff, emit);
         }
         rX += plane;

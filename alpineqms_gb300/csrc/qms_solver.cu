@@ -239,6 +239,15 @@ template <> struct GmPack<double> {
     static __device__ __forceinline__ double at(const V& v, int q) { return q == 0 ? v.x : v.y; }
 };
 
+// the products of two packets, added up in T: a thread's FP32 sum then takes one number per packet
+template <typename T>
+__device__ __forceinline__ float gm_dot(const typename GmPack<T>::V& a, const typename GmPack<T>::V& b) {
+    T s = GmPack<T>::at(a, 0) * GmPack<T>::at(b, 0);
+#pragma unroll
+    for (int q = 1; q < GmPack<T>::W; q++) s += GmPack<T>::at(a, q) * GmPack<T>::at(b, q);
+    return (float)s;
+}
+
 // The conjugate-gradient vectors, 16-byte packets over the three A blocks (the V block is frozen at
 // zero).  Bound by bytes: e takes its step together with p's (one read of p less than apart), 9 blocks
 // of vector traffic per iteration in all where 13 were (V block included).
@@ -344,6 +353,9 @@ __device__ __forceinline__ bool gm_last_block(unsigned* counter) {
 // steps instead of 299, 64x64x80 core 261 instead of 303).  The grid is one resident wave: with
 // eight blocks per SM whatever the registers, a second wave of a few blocks followed (256^3, 8
 // vectors: 367 us instead of 405).
+// A thread then adds up more, one number per packet (gm_dot): at 256^3 w . w is 0.6e-9 to 1.1e-9 of itself
+// off with six and three blocks per SM, 1.8e-9 to 8.5e-9 with an addition per element, and was 1.4e-9 with
+// eight blocks (normal random w); V_i . w is 0.7e-11 to 1.8e-11 of |V_i| |w| off, and was 5.0e-11.
 template <typename T, int NV>
 __global__ void __launch_bounds__(256) qk_gm_dots(long long n, GmPtrs V, const T* w, double* part0, int row0,
                                                   int final, int j, int m, double* Hm, double* Gm,
@@ -365,11 +377,8 @@ __global__ void __launch_bounds__(256) qk_gm_dots(long long n, GmPtrs V, const T
 #pragma unroll
         for (int i = 0; i < NV; i++) vv[i] = __ldg(vp[i] + t);
 #pragma unroll
-        for (int i = 0; i < NV; i++)
-#pragma unroll
-            for (int q = 0; q < PK::W; q++) acc[i] += (float)(PK::at(vv[i], q) * PK::at(wv, q));
-#pragma unroll
-        for (int q = 0; q < PK::W; q++) acc[NV] += (float)(PK::at(wv, q) * PK::at(wv, q));
+        for (int i = 0; i < NV; i++) acc[i] += gm_dot<T>(vv[i], wv);
+        acc[NV] += gm_dot<T>(wv, wv);
     }
     __shared__ double sums[GM_MAXM + 2];
     __shared__ float sh[NV + 1][8];

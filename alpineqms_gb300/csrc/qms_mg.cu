@@ -411,13 +411,6 @@ __host__ __device__ __forceinline__ long long mgc_len(const MGBlockDesc& B, int 
     const int P = mgc_planes(B, lg);
     return 2 * mgc_xlen(B, lg) + (long long)(P + (links ? 4 * (P + 1) : 0)) * B.n1 * B.n2;
 }
-// fast reciprocal in FP32 (a preconditioner needs no correctly rounded divide)
-template <typename T>
-__device__ __forceinline__ T mgc_rcp(T d) {
-    if constexpr (sizeof(T) == 4) return __fdividef(1.0f, d);
-    else return T(1) / d;
-}
-
 extern __shared__ __align__(16) unsigned char mgc_raw[];
 
 // one CTA's slab of a level; x, b, w: indexes in the CTA's shared memory (of T): own point q of x at
@@ -558,7 +551,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
 #pragma unroll 2
         for (int q = tid; q < S.np; q += MGC_THREADS) {
             const T di = G.sm[S.w + S.s3 + q];
-            G.put(S, R, q, di != T(0) ? G.rest(S, X, q) - G.sm[X + S.s3 + q] * mgc_rcp(di) : T(0));
+            G.put(S, R, q, di != T(0) ? G.rest(S, X, q) - G.sm[X + S.s3 + q] / di : T(0));
         }
         G.sync(S.spread);
         const int n1 = S.n1, s3 = S.s3;

@@ -139,6 +139,7 @@ SIGNATURES = [
     ("qms_set_state", ctypes.c_int, [_H, _VP]),
     ("qms_assemble_csr", ctypes.c_int, [_H, ctypes.c_int, _DP, _DP, _DP, _VP, _VP, _VP, _VP, _VP]),
     ("qms_apply", ctypes.c_int, [_H, ctypes.c_int, _DP, ctypes.c_int, _VP, _VP]),
+    ("qms_apply_inner", ctypes.c_int, [_H, ctypes.c_int, ctypes.c_int, _DP, _VP, _VP, _VP]),
     ("qms_csr_spmv", ctypes.c_int, [_H, _VP, _VP, _VP, _VP, _VP]),
     ("qms_residual_norm", ctypes.c_int, [_H, ctypes.c_int, _DP, _DP]),
     ("qms_profile_enable", ctypes.c_int, [_H, ctypes.c_int]),

@@ -292,6 +292,18 @@ int qms_apply(qms_handle* h, int transient, const double v[3], int fp32, const v
     return 0;
 }
 
+int qms_apply_inner(qms_handle* h, int rows, int transient, const double v[3], const double* d_x, const double* d_w,
+                    double* d_y) {
+    HCHECK(h);
+    if (!v || !d_x || !d_y || rows < QMS_ROWS_SCALED || rows > QMS_ROWS_A || (rows == QMS_ROWS_COUPLE && !d_w)) {
+        h->s.err = "null argument or unknown rows";
+        return QMS_ERR_ARG;
+    }
+    CKH(cudaSetDevice(h->s.dev));
+    return h->s.fp64_inner ? h->s.apply_inner<double>(rows, transient != 0, v, d_x, d_w, d_y)
+                           : h->s.apply_inner<float>(rows, transient != 0, v, d_x, d_w, d_y);
+}
+
 int qms_csr_spmv(qms_handle* h, const int64_t* d_ia, const int32_t* d_ja, const double* d_a, const double* d_x,
                  double* d_y) {
     HCHECK(h);

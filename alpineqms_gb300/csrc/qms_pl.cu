@@ -818,7 +818,7 @@ __global__ void qk_ref_add_pl(QGrid g, const T* __restrict__ e, const double* __
     if (i > g.Nx || j > g.Ny) return;
     const QPL L = qms_pl(g);
     const long long t = qms_pl_node(g, L, i, j, k);
-    const double s = scale[0];
+    const double s = scale ? scale[0] : 1.0;
     if (i <= g.xs) x[qAX(g, i, j, k)] += s * (double)e[t];
     if (j <= g.ys) x[qAY(g, i, j, k)] += s * (double)e[L.comp + t];
     if (k <= g.zs) x[qAZ(g, i, j, k)] += s * (double)e[2 * L.comp + t];

@@ -110,6 +110,6 @@ void qms_launch_diag_pl(const QGrid& g, const QCoef<float>& c, const QStepPar<fl
 // out[PL] = r64[ref] * scale[0] (scale may be null: 1)
 template <typename T>
 void qms_launch_pl_from_ref(const QGrid& g, const double* r64, const double* scale, T* out, cudaStream_t st);
-// x[ref] += scale[0] * e[PL]
+// x[ref] += scale[0] * e[PL] (scale may be null: 1)
 template <typename T>
 void qms_launch_ref_add_pl(const QGrid& g, const T* e, const double* scale, double* x, cudaStream_t st);

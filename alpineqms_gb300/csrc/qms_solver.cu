@@ -1877,6 +1877,34 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
     return 0;
 }
 
+// the operator's rows on vectors in the reference's order, through work vectors (zero again afterwards)
+template <typename T>
+int QmsSolver::apply_inner(int rows, bool transient, const double v[3], const double* dx, const double* dw,
+                           double* dy) {
+    const bool adv = rows != QMS_ROWS_A && (v[0] != 0.0 || v[1] != 0.0 || v[2] != 0.0);
+    const QStepPar<T> P = qms_step_par<T>(g, adv ? v[0] : 0.0, adv ? v[1] : 0.0, adv ? v[2] : 0.0, desc.dt, transient);
+    T* xi = (T*)vec[1];
+    T* wi = (T*)vec[2];
+    T* yi = (T*)vec[3];
+    CK(cudaMemsetAsync(yi, 0, npl * sizeof(T), st));
+    qms_launch_pl_from_ref<T>(g, dx, nullptr, xi, st);
+    if (rows == QMS_ROWS_COUPLE) {
+        qms_launch_pl_from_ref<T>(g, dw, nullptr, wi, st);
+        qms_launch_op_pl<T>(g, P, tmapq(xi, 1), sizeof(T) == 4 ? cmapV32 : cmapV64, adv, QOPH_VCOUPLE, yi, wi, nullptr,
+                            status, st);
+    } else {
+        op_pl<T>(adv, rows == QMS_ROWS_A ? QOPH_APPLY_A : QOPH_SCALED, P, xi, yi, nullptr, nullptr);
+    }
+    CK(cudaMemsetAsync(dy, 0, g.n * sizeof(double), st));
+    qms_launch_ref_add_pl<T>(g, yi, nullptr, dy, st);
+    for (void* p : {vec[1], vec[2], vec[3]}) CK(cudaMemsetAsync(p, 0, npl * sizeof(T), st));
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(st));
+    return 0;
+}
+template int QmsSolver::apply_inner<float>(int, bool, const double*, const double*, const double*, double*);
+template int QmsSolver::apply_inner<double>(int, bool, const double*, const double*, const double*, double*);
+
 int QmsSolver::fields(int which, int axis, int index, double* host_out) {
     CK(cudaSetDevice(dev));
     const long long ncell = (long long)g.xs * g.ys * g.zs;

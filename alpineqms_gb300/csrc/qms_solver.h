@@ -188,6 +188,8 @@ struct QmsSolver {
     template <typename T> int inner_pcg(bool transient, int& iters);
     template <typename T> int inner_gmres(bool adv, bool transient, const double v[3], int& iters, int fixed_k);
     int clear_inner();
+    template <typename T> int apply_inner(int rows, bool transient, const double v[3], const double* dx,
+                                          const double* dw, double* dy);
     int residual_launch(bool adv, bool transient, const double v[3], bool exact = false);
     template <typename T> void gmres_begin();
     template <typename T> void gmres_steps(bool adv, bool transient, const double v[3], int j0, int j1);

@@ -217,6 +217,13 @@ int qms_assemble_csr(qms_handle* h, int transient, const double v[3], const doub
 /* y = M x with the matrix-free operator in FP64 (fp32 = 0) or FP32 (fp32 = 1);
  * d_x, d_y: n_dims elements of that type. */
 int qms_apply(qms_handle* h, int transient, const double v[3], int fp32, const void* d_x, void* d_y);
+/* The rows of the inner solver's operator, on its own vectors and in its own precision: verification path.
+ * QMS_ROWS_SCALED: y = D^-1 M x.  QMS_ROWS_COUPLE: the V rows of y = w - D^-1 M (x_A, 0).  QMS_ROWS_A:
+ * the A rows of y = M x for v = 0 and V = 0 (v is not read).  d_x, d_w, d_y: n_dims doubles, zero on the
+ * Dirichlet rows (d_w: QMS_ROWS_COUPLE alone); the other rows of y are zero.  Not inside a capture. */
+enum { QMS_ROWS_SCALED = 0, QMS_ROWS_COUPLE = 1, QMS_ROWS_A = 2 };
+int qms_apply_inner(qms_handle* h, int rows, int transient, const double v[3], const double* d_x, const double* d_w,
+                    double* d_y);
 /* CSR SpMV on the verification-path arrays (FP64). */
 int qms_csr_spmv(qms_handle* h, const int64_t* d_ia, const int32_t* d_ja, const double* d_a, const double* d_x,
                  double* d_y);

@@ -4,9 +4,9 @@
 
 struct QmsExcite { double B[3]; double G[9]; double v[3]; };
 
-// QOPH_VCOUPLE (padded-layout stencil only): y_V = w_V - D_V^-1 (M_VA x_A) on the V rows, the
-// A-to-V coupling of the operator applied to x's A blocks (x's V block is not read)
-enum QOpModeH { QOPH_APPLY = 0, QOPH_SCALED = 1, QOPH_RESID = 2, QOPH_VCOUPLE = 3, QOPH_APPLY_A = 4 };
+// modes of the reference-layout operator and of the padded-layout stencil (qms_launch_op_pl), each its own type
+enum QOpModeH { QOPH_APPLY = 0, QOPH_SCALED = 1, QOPH_RESID = 2 };
+enum QPlMode { QPL_SCALED = 0, QPL_VCOUPLE = 1, QPL_APPLY_A = 2 };
 
 // qms_exact.cu
 long long qms_launch_assemble(const QGrid& g, const uint8_t* ids, const QMatTable<double>* tab, const QmsExcite& ex,

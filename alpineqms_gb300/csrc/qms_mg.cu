@@ -1001,8 +1001,9 @@ static void mg0_prepare() {
 #define ATTR(K, Q) \
     cudaFuncSetAttribute(mg0_tiled<T, K, Q, U, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mg0_smem<T, K, Q>())
     ATTR(0, 0); ATTR(1, 0); ATTR(2, 0);
-    ATTR(0, 1); ATTR(1, 1); ATTR(2, 1); ATTR(3, 1);
-    ATTR(0, 2); ATTR(1, 2); ATTR(2, 2); ATTR(3, 2);
+    ATTR(0, 1); ATTR(1, 1); ATTR(2, 1);
+    ATTR(0, 2); ATTR(1, 2); ATTR(2, 2);
+        if constexpr (sizeof(T) == 4) { ATTR(3, 1); ATTR(3, 2); }
 #undef ATTR
     };
     using R1 = std::integral_constant<int, 1>;
@@ -1395,6 +1396,7 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     } while (0)
     // rows per thread: two on grids of many tiles (FP32)
     constexpr int ROWS2 = sizeof(T) == 4 ? 2 : 1;
+    constexpr bool FIRST2 = sizeof(T) == 4;      // (FP64 callers hand over no map of b)
     const bool two = (long long)g0grid.x * g0grid.y * g0grid.z >= QMS_CTA_TARGET;
     auto wgt = [&](int s, int nu) { return mg_weight<T>(omega, s, nu); };
     const bool cubic = P0.idx2 == P0.idy2 && P0.idx2 == P0.idz2;
@@ -1403,15 +1405,18 @@ int QmsMG<T>::vcycle_q(const T* b0, bool scaled, T* x0, const CUtensorMap& x0map
     Buf x{x0, &x0map}, t{t0, &t0map};
     if ((n1 + n2) % 2 == 0) std::swap(x, t);
     int s = 1;
-    if (b0map && scaled && QS != 0 && n1 >= 2) {
-        // the first two sweeps in one pass, from b's tiles (KIND 3), into the buffer the second
-        // sweep writes
-        Buf bb{const_cast<T*>(b0), b0map};
-        MG0(3, bb, t.p, nullptr, wgt(1, n1), wgt(0, n1));
-        std::swap(x, t);
-        launches++;
-        s = 2;
-    } else {
+    if constexpr (FIRST2 && QS != 0) {
+        if (b0map && scaled && n1 >= 2) {
+            // the first two sweeps in one pass, from b's tiles (KIND 3), into the buffer the second
+            // sweep writes
+            Buf bb{const_cast<T*>(b0), b0map};
+            MG0(3, bb, t.p, nullptr, wgt(1, n1), wgt(0, n1));
+            std::swap(x, t);
+            launches++;
+            s = 2;
+        }
+    }
+    if (s == 1) {
         MG0(0, x, x.p, nullptr, wgt(0, n1), T(0));
         launches++;
     }

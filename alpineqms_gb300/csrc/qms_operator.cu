@@ -233,11 +233,13 @@ static void qms_operator_prepare() {
     const int shm = (int)(sizeof(TileCoef<T>) + sizeof(XTile<T>));
     for (auto f : {qk_operator_t<T, 0, QOP_APPLY>, qk_operator_t<T, 0, QOP_SCALED>, qk_operator_t<T, 0, QOP_RESID>,
                    qk_operator_t<T, 7, QOP_APPLY>, qk_operator_t<T, 7, QOP_SCALED>, qk_operator_t<T, 7, QOP_RESID>,
-                   qk_operator_t<T, 1, QOP_RESID>, qk_operator_t<T, 2, QOP_RESID>, qk_operator_t<T, 4, QOP_RESID>,
-                   qk_operator_t<T, 0, QOP_RESID, QROW_TIME>, qk_operator_t<T, 1, QOP_RESID, QROW_TIME>,
-                   qk_operator_t<T, 2, QOP_RESID, QROW_TIME>, qk_operator_t<T, 4, QOP_RESID, QROW_TIME>,
-                   qk_operator_t<T, 7, QOP_RESID, QROW_TIME>})
+                   qk_operator_t<T, 1, QOP_RESID>, qk_operator_t<T, 2, QOP_RESID>, qk_operator_t<T, 4, QOP_RESID>})
         cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
+    if constexpr (sizeof(T) == 8)
+        for (auto f : {qk_operator_t<T, 0, QOP_RESID, QROW_TIME>, qk_operator_t<T, 1, QOP_RESID, QROW_TIME>,
+                       qk_operator_t<T, 2, QOP_RESID, QROW_TIME>, qk_operator_t<T, 4, QOP_RESID, QROW_TIME>,
+                       qk_operator_t<T, 7, QOP_RESID, QROW_TIME>})
+            cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
 
@@ -249,14 +251,18 @@ void qms_launch_operator(const QGrid& g, const QCoef<T>& c, const QStepPar<T>& P
     qms_operator_prepare<T>();
 #define L(VM, MODE) qk_operator_t<T, VM, MODE><<<gs, bs, shm, st>>>(g, c, P, x, b, y, w, partials, T(0))
     // the residual (the FP64 anchor of every solve) also has one instantiation per velocity axis, and those
-    // for cubic cells
-#define LR(VM)                                                                                                  \
-    do {                                                                                                        \
-        if (g.dx == g.dy && g.dx == g.dz)                                                                       \
-            qk_operator_t<T, VM, QOP_RESID, QROW_TIME><<<gs, bs, shm, st>>>(                                    \
-                g, c, qms_unit_par<T>(g, P, QROW_TIME), x, b, y, w, partials, P.idx2);                          \
-        else L(VM, QOP_RESID);                                                                                  \
-    } while (0)
+    // for cubic cells (FP64: nothing takes an FP32 one)
+    auto resid = [&](auto vm) {
+        constexpr int VM = decltype(vm)::value;
+        if constexpr (sizeof(T) == 8)
+            if (g.dx == g.dy && g.dx == g.dz) {
+                qk_operator_t<T, VM, QOP_RESID, QROW_TIME><<<gs, bs, shm, st>>>(
+                    g, c, qms_unit_par<T>(g, P, QROW_TIME), x, b, y, w, partials, P.idx2);
+                return;
+            }
+        L(VM, QOP_RESID);
+    };
+#define LR(VM) resid(std::integral_constant<int, VM>())
     const int m = (P.vx != T(0) ? 1 : 0) | (P.vy != T(0) ? 2 : 0) | (P.vz != T(0) ? 4 : 0);
     if (adv) {
         if (mode == QOP_APPLY) L(7, QOP_APPLY);

@@ -116,8 +116,9 @@ __device__ __forceinline__ T pl_div(T a, T d) {
     else return a / d;
 }
 
-// MODE: QOPH_APPLY_A (y_A = M_AA x_A; no velocity), QOPH_SCALED (y = D^-1 M x), QOPH_VCOUPLE (V rows only:
-// y = w - D^-1 M (x_A, 0)) or QOPH_RESID (T = qdf: y = (float) (w - D^-1 M x), the refinement
+#define QPL_RESID 3          // qms_launch_resid_df alone
+// MODE: QPL_APPLY_A (y_A = M_AA x_A; no velocity), QPL_SCALED (y = D^-1 M x), QPL_VCOUPLE (V rows only:
+// y = w - D^-1 M (x_A, 0)) or QPL_RESID (T = qdf: y = (float) (w - D^-1 M x), the refinement
 // residual in double-float arithmetic, with w the residual of the anchor and x the change of
 // the solution since then).  Partials (optional, FP64 across warps): APPLY_A / SCALED [0] += y . w
 // (w may be null), [1] += y . y; RESID |r_A|^2, |r_V|^2; none with VCOUPLE.
@@ -129,8 +130,8 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
          YT* y, const WT* w, double* partials, unsigned* err, WT* yfull, T unit) {
     // VCOUPLE reads only what the V rows' A couplings need: the three A blocks of x (xmap over
     // them) and the three conductivities (cmap over them)
-    constexpr bool VC = MODE == QOPH_VCOUPLE;
-    constexpr bool AO = MODE == QOPH_APPLY_A;      // the A blocks alone: conjugate gradients with V = 0
+    constexpr bool VC = MODE == QPL_VCOUPLE;
+    constexpr bool AO = MODE == QPL_APPLY_A;      // the A blocks alone: conjugate gradients with V = 0
     constexpr int C0 = VC ? 3 : 0;
     using TL = PLTiles<T, VC || AO ? 3 : 4, VC ? 3 : 6>;
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -185,7 +186,7 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
     using RT = float;
     RT red0 = 0, red1 = 0;
     auto emit = [&](long long row, T acc, T diag, bool is_a, T, bool fixed, T, T) {
-        if constexpr (MODE == QOPH_RESID) {
+        if constexpr (MODE == QPL_RESID) {
             const T out = w[row] - acc / diag;
             y[row] = out.h;
             if (yfull) yfull[row] = out;          // the residual in full, for the next solve's anchor
@@ -194,7 +195,7 @@ qk_op_pl(QGrid g, QStepPar<T> P, const __grid_constant__ CUtensorMap xmap, const
                 if (is_a) red0 += o * o;
                 else red1 += o * o;
             }
-        } else if constexpr (MODE == QOPH_VCOUPLE) {   // the A rows are not wanted (dead code)
+        } else if constexpr (MODE == QPL_VCOUPLE) {   // the A rows are not wanted (dead code)
             if (!is_a) y[row] = w[row] - pl_div(acc, diag);
         } else {
             if (AO && !is_a) return;                   // the V row is not wanted (dead code)
@@ -859,10 +860,10 @@ static void op_pl_attrs(int shm) {
     auto one = [&](auto uni) {
         constexpr bool U = decltype(uni)::value;
         if (VM == 0)
-            cudaFuncSetAttribute(qk_op_pl<T, 0, QOPH_APPLY_A, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(qk_op_pl<T, 0, QPL_APPLY_A, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)PLTiles<T, 3, 6>::SMEM);
-        cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_SCALED, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
-        cudaFuncSetAttribute(qk_op_pl<T, VM, QOPH_VCOUPLE, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(qk_op_pl<T, VM, QPL_SCALED, U>, cudaFuncAttributeMaxDynamicSharedMemorySize, shm);
+        cudaFuncSetAttribute(qk_op_pl<T, VM, QPL_VCOUPLE, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)PLTiles<T, 3, 3>::SMEM);
     };
     one(std::true_type());
@@ -884,11 +885,11 @@ static void op_pl_prepare() {
         op_pl_attrs<T, 2>(shm);
         op_pl_attrs<T, 4>(shm);
         const int shd = (int)PLTiles<qdf>::SMEM;
-        cudaFuncSetAttribute(qk_op_pl<qdf, 0, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-        cudaFuncSetAttribute(qk_op_pl<qdf, 1, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-        cudaFuncSetAttribute(qk_op_pl<qdf, 2, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-        cudaFuncSetAttribute(qk_op_pl<qdf, 4, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
-        cudaFuncSetAttribute(qk_op_pl<qdf, 7, QOPH_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 0, QPL_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 1, QPL_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 2, QPL_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 4, QPL_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
+        cudaFuncSetAttribute(qk_op_pl<qdf, 7, QPL_RESID, false, float, qdf>, cudaFuncAttributeMaxDynamicSharedMemorySize, shd);
     }
     done.fetch_or(bit, std::memory_order_acq_rel);
 }
@@ -902,7 +903,7 @@ long long qms_op_pl_num_blocks(const QGrid& g) {
 }
 
 template <typename T, int VM>
-static void op_pl_launch(dim3 gs, dim3 bs, size_t shm, cudaStream_t st, int mode, const QGrid& g,
+static void op_pl_launch(dim3 gs, dim3 bs, size_t shm, cudaStream_t st, QPlMode mode, const QGrid& g,
                          const QStepPar<T>& P, const CUtensorMap& xmap, const CUtensorMap& cmap, T* y, const T* w,
                          double* partials, unsigned* err) {
     if constexpr (sizeof(T) == 8 && VM != 0 && VM != 7) {
@@ -910,14 +911,14 @@ static void op_pl_launch(dim3 gs, dim3 bs, size_t shm, cudaStream_t st, int mode
     } else {
         auto go = [&](auto uni, const QStepPar<T>& Q) {
             constexpr bool U = decltype(uni)::value;
-            if (mode == QOPH_APPLY_A)             // (no velocity: VM is 0)
-                pdl_launch(qk_op_pl<T, 0, QOPH_APPLY_A, U>, gs, bs, PLTiles<T, 3, 6>::SMEM, st, 0, g, Q, xmap, cmap, y, w,
+            if (mode == QPL_APPLY_A)             // (no velocity: VM is 0)
+                pdl_launch(qk_op_pl<T, 0, QPL_APPLY_A, U>, gs, bs, PLTiles<T, 3, 6>::SMEM, st, 0, g, Q, xmap, cmap, y, w,
                            partials, err, nullptr, P.idx2);
-            else if (mode == QOPH_VCOUPLE)
-                pdl_launch(qk_op_pl<T, VM, QOPH_VCOUPLE, U>, gs, bs, PLTiles<T, 3, 3>::SMEM, st, 0, g, Q, xmap, cmap, y, w,
+            else if (mode == QPL_VCOUPLE)
+                pdl_launch(qk_op_pl<T, VM, QPL_VCOUPLE, U>, gs, bs, PLTiles<T, 3, 3>::SMEM, st, 0, g, Q, xmap, cmap, y, w,
                            partials, err, nullptr, P.idx2);
             else
-                pdl_launch(qk_op_pl<T, VM, QOPH_SCALED, U>, gs, bs, shm, st, 0, g, Q, xmap, cmap, y, w, partials, err,
+                pdl_launch(qk_op_pl<T, VM, QPL_SCALED, U>, gs, bs, shm, st, 0, g, Q, xmap, cmap, y, w, partials, err,
                            nullptr, P.idx2);
         };
         if (g.dx == g.dy && g.dx == g.dz) go(std::true_type(), qms_unit_par<T>(g, P));
@@ -927,7 +928,7 @@ static void op_pl_launch(dim3 gs, dim3 bs, size_t shm, cudaStream_t st, int mode
 
 template <typename T>
 void qms_launch_op_pl(const QGrid& g, const QStepPar<T>& P, const CUtensorMap& xmap, const CUtensorMap& cmap, bool adv,
-                      int mode, T* y, const T* w, double* partials, unsigned* err, cudaStream_t st) {
+                      QPlMode mode, T* y, const T* w, double* partials, unsigned* err, cudaStream_t st) {
     op_pl_prepare<T>();
     const dim3 bs(OTX, OTY, 1), gs = qms_pl_tiles(g);
     const size_t shm = PLTiles<T>::SMEM;
@@ -935,9 +936,9 @@ void qms_launch_op_pl(const QGrid& g, const QStepPar<T>& P, const CUtensorMap& x
     QMS_WITH_VM(vm, (op_pl_launch<T, VM>(gs, bs, shm, st, mode, g, P, xmap, cmap, y, w, partials, err)));
 }
 template void qms_launch_op_pl<float>(const QGrid&, const QStepPar<float>&, const CUtensorMap&, const CUtensorMap&,
-                                      bool, int, float*, const float*, double*, unsigned*, cudaStream_t);
+                                      bool, QPlMode, float*, const float*, double*, unsigned*, cudaStream_t);
 template void qms_launch_op_pl<double>(const QGrid&, const QStepPar<double>&, const CUtensorMap&, const CUtensorMap&,
-                                       bool, int, double*, const double*, double*, unsigned*, cudaStream_t);
+                                       bool, QPlMode, double*, const double*, double*, unsigned*, cudaStream_t);
 
 void qms_launch_resid_df(const QGrid& g, const QStepPar<qdf>& P, const CUtensorMap& xmap, const CUtensorMap& cmap,
                          bool adv, float* r, const qdf* b, double* partials, unsigned* err, cudaStream_t st,
@@ -946,7 +947,7 @@ void qms_launch_resid_df(const QGrid& g, const QStepPar<qdf>& P, const CUtensorM
     const dim3 bs(OTX, OTY, 1), gs = qms_pl_tiles(g);
     const size_t shm = PLTiles<qdf>::SMEM;
     const int vm = qms_vel_mask(P, adv, true);
-    QMS_WITH_VM(vm, (pdl_launch(qk_op_pl<qdf, VM, QOPH_RESID, false, float, qdf>, gs, bs, shm, st, 0, g, P, xmap, cmap, r, b,
+    QMS_WITH_VM(vm, (pdl_launch(qk_op_pl<qdf, VM, QPL_RESID, false, float, qdf>, gs, bs, shm, st, 0, g, P, xmap, cmap, r, b,
                                 partials, err, rfull, qdf(1))));
 }
 

@@ -17,13 +17,13 @@ dim3 qms_node_block();
 dim3 qms_pl_tiles(const QGrid& g);
 long long qms_op_pl_num_blocks(const QGrid& g);
 
-// y_A = M_AA x_A without velocity (mode QOPH_APPLY_A, the map of x's A blocks) or D^-1 M x (QOPH_SCALED) on
+// y_A = M_AA x_A without velocity (mode QPL_APPLY_A, the map of x's A blocks) or D^-1 M x (QPL_SCALED) on
 // padded vectors; x and the node
 // coefficients come through their tensor maps (qms_make_pl_map, 10 and 9 rows per box).
-// QOPH_VCOUPLE takes the maps of x's three A blocks and of the three conductivities.
+// QPL_VCOUPLE takes the maps of x's three A blocks and of the three conductivities.
 template <typename T>
 void qms_launch_op_pl(const QGrid& g, const QStepPar<T>& P, const CUtensorMap& xmap, const CUtensorMap& cmap, bool adv,
-                      int mode, T* y, const T* w, double* partials, unsigned* err, cudaStream_t st);
+                      QPlMode mode, T* y, const T* w, double* partials, unsigned* err, cudaStream_t st);
 
 // refinement residual in double-float from an anchor: r = (float) (r0 - D^-1 M dx) on padded
 // vectors, with r0 the anchor's scaled residual and dx (xmap) the change of x since the anchor,

@@ -576,42 +576,42 @@ static GmPtrs gm_shift(const GmPtrs& V, int off) {
 }
 // One resident wave of blocks (at most vb): each walks the vectors with the same stride, so blocks of a
 // second, partial wave would run while most SMs have nothing left
-static int gm_blocks(const void* kernel, std::atomic<int>& per, int vb) {
+static int gm_blocks(const void* kernel, std::atomic<int>& per, int vb, int nsm) {
     int p = per.load(std::memory_order_relaxed);
     if (p == 0) {
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&p, kernel, 256, 0);
         p = std::max(1, p);
         per.store(p, std::memory_order_relaxed);
     }
-    return std::min(vb, 152 * p);
+    return std::min(vb, nsm * p);
 }
 // return the kernel launches
 template <typename T>
 static int gm_dots(int nv, int vb, cudaStream_t st, long long n, const GmPtrs& V, const T* w, double* part, int row0,
-                   int j, int m, double* Hm, double* Gm, unsigned* counter) {
+                   int j, int m, double* Hm, double* Gm, unsigned* counter, int nsm) {
     const int now = std::min(nv, GM_PASS), final = now == nv ? 1 : 0;
     int nb = vb;                                // later passes: as many blocks (partials) as the first
     switch (now) {
 #define C(N) case N: { static std::atomic<int> per{0}; \
-        if (row0 == 0) nb = gm_blocks((const void*)qk_gm_dots<T, N>, per, vb); \
+        if (row0 == 0) nb = gm_blocks((const void*)qk_gm_dots<T, N>, per, vb, nsm); \
         pdl_launch(qk_gm_dots<T, N>, dim3(nb), dim3(256), 0, st, 0, n, V, w, part, row0, final, j, m, Hm, Gm, counter); } break;
         GM_CASES(C)
 #undef C
     }
-    return final ? 1 : 1 + gm_dots<T>(nv - now, nb, st, n, gm_shift(V, now), w, part, row0 + now, j, m, Hm, Gm, counter);
+    return final ? 1 : 1 + gm_dots<T>(nv - now, nb, st, n, gm_shift(V, now), w, part, row0 + now, j, m, Hm, Gm, counter, nsm);
 }
 template <typename T>
 static int gm_orth(int nv, int vb, cudaStream_t st, long long n, int j, int m, const GmPtrs& V, double* Hm, int row0,
-                   T* w, double* part, double* Gm, T* vout, unsigned* counter, unsigned* status) {
+                   T* w, double* part, double* Gm, T* vout, unsigned* counter, unsigned* status, int nsm) {
     const int now = std::min(nv, GM_PASS), final = now == nv ? 1 : 0;
     switch (now) {
 #define C(N) case N: { static std::atomic<int> per{0}; \
-        pdl_launch(qk_gm_orth<T, N>, dim3(gm_blocks((const void*)qk_gm_orth<T, N>, per, vb)), dim3(256), 0, st, 0, n, j, m, V, Hm, row0, w, part, Gm, vout, final, counter, status); } break;
+        pdl_launch(qk_gm_orth<T, N>, dim3(gm_blocks((const void*)qk_gm_orth<T, N>, per, vb, nsm)), dim3(256), 0, st, 0, n, j, m, V, Hm, row0, w, part, Gm, vout, final, counter, status); } break;
         GM_CASES(C)
 #undef C
     }
     return final ? 1 : 1 + gm_orth<T>(nv - now, vb, st, n, j, m, gm_shift(V, now), Hm, row0 + now, w, part, Gm, vout,
-                                      counter, status);
+                                      counter, status, nsm);
 }
 template <typename T>
 static int gm_update(int nv, cudaStream_t st, const QGrid& g, int m, const GmPtrs& Z, const double* Gm,
@@ -734,7 +734,6 @@ int QmsSolver::init(const qms_desc& d) {
     fp64_inner = d.precision == QMS_PREC_FP64;
     trace = std::getenv("QMS_TRACE") != nullptr;
     tsize = fp64_inner ? sizeof(double) : sizeof(float);
-    int nsm = 0;
     CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
     vec_blocks = (long long)nsm * 8;
     long long need = (npl + 255) / 256;
@@ -985,16 +984,16 @@ const CUtensorMap& QmsSolver::tmapq(const void* p, int qs) const {
 }
 
 template <typename T>
-void QmsSolver::op_pl(bool adv, int mode, const QStepPar<T>& P, const T* xin, T* y, const T* w, double* partials) {
+void QmsSolver::op_pl(bool adv, QPlMode mode, const QStepPar<T>& P, const T* xin, T* y, const T* w, double* partials) {
     const double ncell = (double)g.xs * g.ys * g.zs;
     OpEv* ev = prof_begin(sizeof(T) == 8 ? 1 : 0, (double)g.n * sizeof(T) * (2 + (w && w != xin ? 1 : 0)) + ncell);
-    qms_launch_op_pl<T>(g, P, mode == QOPH_APPLY_A ? tmapq(xin, 1) : tmap(xin), sizeof(T) == 8 ? cmap64 : cmap32, adv, mode,
+    qms_launch_op_pl<T>(g, P, mode == QPL_APPLY_A ? tmapq(xin, 1) : tmap(xin), sizeof(T) == 8 ? cmap64 : cmap32, adv, mode,
                         y, w, partials, status, st);
     nlaunch++;
     prof_end(ev);
 }
-template void QmsSolver::op_pl<float>(bool, int, const QStepPar<float>&, const float*, float*, const float*, double*);
-template void QmsSolver::op_pl<double>(bool, int, const QStepPar<double>&, const double*, double*, const double*,
+template void QmsSolver::op_pl<float>(bool, QPlMode, const QStepPar<float>&, const float*, float*, const float*, double*);
+template void QmsSolver::op_pl<double>(bool, QPlMode, const QStepPar<double>&, const double*, double*, const double*,
                                        double*);
 template void QmsSolver::op<double>(bool, int, const QStepPar<double>&, const double*, const double*, double*,
                                     const double*, double*);
@@ -1010,13 +1009,12 @@ QmsSolver::OpEv* QmsSolver::prof_begin(int kind, double bytes) {
     OpEv* ev = &evpool[evused++];
     ev->kind = kind;
     ev->bytes = bytes;
-    // inside a capture the record must become an event-record node of the graph
-    cudaEventRecordWithFlags(ev->a, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault);
+    cudaEventRecord(ev->a, st);                 // (a profiled solve captures nothing)
     return ev;
 }
 
 void QmsSolver::prof_end(OpEv* ev) {
-    if (ev) cudaEventRecordWithFlags(ev->b, st, capturing ? cudaEventRecordExternal : cudaEventRecordDefault);
+    if (ev) cudaEventRecord(ev->b, st);
 }
 
 bool QmsSolver::prof_accum(const OpEv& e) {
@@ -1089,7 +1087,7 @@ void QmsSolver::precond(const T* r, const float* bscale, T* z, bool mask_v, bool
             // the A correction leaves in the V rows (row-scaled like r)
             T* tv = (T*)mgtmp2;
             cycle(r, 1, cm);
-            qms_launch_op_pl<T>(g, *P, tmapq(z, 1), f32 ? cmapV32 : cmapV64, adv, QOPH_VCOUPLE, tv, r, nullptr,
+            qms_launch_op_pl<T>(g, *P, tmapq(z, 1), f32 ? cmapV32 : cmapV64, adv, QPL_VCOUPLE, tv, r, nullptr,
                                 status, st);
             cycle(tv, 2, f32 ? cmapV16 : cmapV64);
             nlaunch++;
@@ -1129,12 +1127,12 @@ int QmsSolver::inner_bicgstab(bool adv, bool transient, const double v[3], int& 
         qk_bicg_p<T><<<vb, 256, 0, st>>>(n, r, p, vv, S);
         nlaunch++;
         if (use_mg) precond<T>(p, dg, y, false, transient, false, &P, adv);
-        op_pl<T>(adv, QOPH_SCALED, P, y, vv, rh, part);
+        op_pl<T>(adv, QPL_SCALED, P, y, vv, rh, part);
         finalize(FIN_BICG_ALPHA, 1, nbpl);
         qk_bicg_s<T><<<vb, 256, 0, st>>>(n, r, vv, s, S);
         nlaunch++;
         if (use_mg) precond<T>(s, dg, z, false, transient, false, &P, adv);
-        op_pl<T>(adv, QOPH_SCALED, P, z, t, s, part);
+        op_pl<T>(adv, QPL_SCALED, P, z, t, s, part);
         finalize(FIN_BICG_OMEGA, 2, nbpl);
         qk_bicg_xr<T><<<vb, 256, 0, st>>>(n, y, z, s, t, rh, e, r, S, part);
         nlaunch++;
@@ -1184,10 +1182,10 @@ void QmsSolver::gmres_steps(bool adv, bool transient, const double v[3], int j0,
         T* vj = (T*)gmV[j];
         T* zj = use_mg ? (T*)gmZ[j] : vj;
         if (use_mg) precond<T>(vj, dg, zj, false, transient, false, &P, adv);
-        op_pl<T>(adv, QOPH_SCALED, P, zj, w, nullptr, nullptr);
-        nlaunch += gm_dots<T>(j + 1, vb, st, n, Vp, w, part, 0, j, m, gm_H, gm_scal, gm_count);
-        nlaunch += gm_orth<T>(j + 1, vb, st, n, j, m, Vp, gm_H, 0, w, part, gm_scal, (T*)gmV[j + 1], gm_count, status);
-        pdl_launch(qk_gm_scale<T>, dim3(std::min(vb, 152)), dim3(256), 0, st, 0, n, w, (T*)gmV[j + 1], gm_scal);
+        op_pl<T>(adv, QPL_SCALED, P, zj, w, nullptr, nullptr);
+        nlaunch += gm_dots<T>(j + 1, vb, st, n, Vp, w, part, 0, j, m, gm_H, gm_scal, gm_count, nsm);
+        nlaunch += gm_orth<T>(j + 1, vb, st, n, j, m, Vp, gm_H, 0, w, part, gm_scal, (T*)gmV[j + 1], gm_count, status, nsm);
+        pdl_launch(qk_gm_scale<T>, dim3(std::min(vb, nsm)), dim3(256), 0, st, 0, n, w, (T*)gmV[j + 1], gm_scal);
         nlaunch++;
     }
 }
@@ -1357,7 +1355,7 @@ int QmsSolver::inner_pcg(bool transient, int& iters) {
     const double tol2 = desc.inner_rtol * desc.inner_rtol;
     iters = 0;
     for (int it = 0; it < desc.max_inner; it++) {
-        op_pl<T>(false, QOPH_APPLY_A, P, p, q, p, part);
+        op_pl<T>(false, QPL_APPLY_A, P, p, q, p, part);
         finalize(FIN_CG_ALPHA, 1, nbpl);
         pdl_launch(qk_cg_axpy<T>, dim3(vb), dim3(256), 0, st, 0, nA, q, S, T(-1), r);
         nlaunch++;
@@ -1497,7 +1495,6 @@ int QmsSolver::step_graph(bool adv, const double v[3], const QStepStart& hs, boo
         int rc = 0;
         if (e == cudaSuccess) e = cudaStreamBeginCaptureToGraph(st, graph, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
-            capturing = true;
             cudaMemsetAsync(status, 0, 4, st);
             cudaMemcpyAsync(dptrs, hptrs, sizeof(QStepPtrs), cudaMemcpyHostToDevice, st);
             qms_launch_step_start(g, rfin, b, bprev, dinvdf, r0df, hs, rpl, part, nbpl, st, dptrs);
@@ -1540,7 +1537,6 @@ int QmsSolver::step_graph(bool adv, const double v[3], const QStepStart& hs, boo
                     if (e == cudaSuccess) e = e2;
                 }
             }
-            capturing = false;
         }
         nlaunch = n0;
         if (rc == 0 && e == cudaSuccess) e = cudaGraphInstantiate(&ng.exec, graph, 0);
@@ -1890,10 +1886,10 @@ int QmsSolver::apply_inner(int rows, bool transient, const double v[3], const do
     qms_launch_pl_from_ref<T>(g, dx, nullptr, xi, st);
     if (rows == QMS_ROWS_COUPLE) {
         qms_launch_pl_from_ref<T>(g, dw, nullptr, wi, st);
-        qms_launch_op_pl<T>(g, P, tmapq(xi, 1), sizeof(T) == 4 ? cmapV32 : cmapV64, adv, QOPH_VCOUPLE, yi, wi, nullptr,
+        qms_launch_op_pl<T>(g, P, tmapq(xi, 1), sizeof(T) == 4 ? cmapV32 : cmapV64, adv, QPL_VCOUPLE, yi, wi, nullptr,
                             status, st);
     } else {
-        op_pl<T>(adv, rows == QMS_ROWS_A ? QOPH_APPLY_A : QOPH_SCALED, P, xi, yi, nullptr, nullptr);
+        op_pl<T>(adv, rows == QMS_ROWS_A ? QPL_APPLY_A : QPL_SCALED, P, xi, yi, nullptr, nullptr);
     }
     CK(cudaMemsetAsync(dy, 0, g.n * sizeof(double), st));
     qms_launch_ref_add_pl<T>(g, yi, nullptr, dy, st);

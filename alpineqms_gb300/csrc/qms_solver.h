@@ -31,6 +31,7 @@ struct QmsSolver {
     bool fp64_inner = false;
     bool trace = false;         // QMS_TRACE set: one stderr line per refinement iteration
     size_t tsize = 4;
+    int nsm = 0;                // SMs of the device
     long long vec_blocks = 0;
     long long nbop = 0, nbpl = 0;   // CTAs of the reference-layout operator / over the padded vectors' tiles
 
@@ -133,7 +134,6 @@ struct QmsSolver {
     // added (profile events nest: the A-block sweeps inside a V-cycle's own event)
     std::deque<OpEv> evpool;
     size_t evused = 0;
-    bool capturing = false;                      // event records go into a graph being captured
     qms_profile profacc{};
     // the multigrid's timing hook (the A-block sweeps), forwarding to prof_begin / prof_end
     struct MgHook : MgProf {
@@ -147,7 +147,7 @@ struct QmsSolver {
     void op(bool adv, int mode, const QStepPar<T>& P, const T* x, const T* b, T* y, const T* w, double* partials);
     // the inner solver's operator on padded vectors (TMA-staged)
     template <typename T>
-    void op_pl(bool adv, int mode, const QStepPar<T>& P, const T* x, T* y, const T* w, double* partials);
+    void op_pl(bool adv, QPlMode mode, const QStepPar<T>& P, const T* x, T* y, const T* w, double* partials);
     long long npl = 0;                              // padded inner-vector length
     std::unordered_map<const void*, CUtensorMap> tmaps;   // tensor maps of the padded vectors
     CUtensorMap cmap32{}, cmap64{};                 // ... and of the node coefficients

@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(256) mg_prolong_smooth(MGLevelDev<T> L, const 
 // residual of the fine level summed over each aggregate -> coarse right-hand side.  A thread per fine
 // point (tiles of 32 x 4 x 2 points, even origins), the eight residuals of an aggregate added through a
 // shuffle and shared memory: a thread per coarse point left a chain of eight 7-point rows (10-16 us a
-// launch on levels of 25^3 to 129^3 points; ~MG_RESTRICT_US now).
+// launch on levels of 25^3 to 129^3 points; 65^3: 11 us then, 7 us now).
 #define MGR_X 32
 #define MGR_Y 4
 #define MGR_Z 2
@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
 // A stage of a march is x's plane k + 1 (all components, +-1 halo in i and j) and
 // the coefficients' plane k, two TMA copies on one mbarrier, issued two planes
 // ahead; b is fetched into registers one plane ahead.
-// The kernels are bound by instruction issue, not by bytes, so: on grids of 1216 tiles or more a thread has
+// The kernels were bound by instruction issue, not by bytes, so: on grids of 1216 tiles or more a thread has
 // two rows (ROWS; j and j + 1: their common coefficients and x are read once, address arithmetic and
 // the plane's barrier shared), on smaller ones, where the march's latency counts, one; what plane k - 1
 // contributes (x and three coefficients at the thread's own node) stays in
@@ -665,6 +665,8 @@ __global__ void __launch_bounds__(MGC_THREADS, 1) mg_sub(const __grid_constant__
 // two mbarriers per plane, one plane ahead), ms per run of steps: 96^3 202 -> 191, 128^3 244 -> 229,
 // moving plate 256^3 780 -> 717, 64^3 in FP64 411 -> 337.  Two rows per thread instead of one: 96^3 191 ->
 // 186, 128^3 228 -> 219, 256^3 717 -> 690, but 48^3 161 -> 169 and FP64 as before (one row there).
+// The A blocks' sweep at 192^3: 94.7 us and 87.7 M warp instructions before, 67.8 us and 47.1 M now, with issue
+// 62 % active and DRAM at 64 %: latency (staged planes, the plane's barrier) is what is left.
 // ---------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ T mg_rcp(T d) {
@@ -1343,11 +1345,8 @@ int QmsMG<T>::build(const QGrid& g, const QCoef<T>& c, const QStepPar<T>& P, T v
             }
             return smem(lt) <= MGC_SMEM;
         };
-        int lt = (int)v.size() - 1;
-        bool small = true;                       // the coarsest level is one CTA's
-        for (int b = 0; b < v[lt].nb; b++)
-            small = small && (long long)v[lt].blk[b].n1 * v[lt].blk[b].n2 * v[lt].blk[b].n3 <= MGC_LOCAL;
-        while (small && lt > 1 && (int)v.size() - (lt - 1) <= MGC_LEVELS && fits(lt - 1)) lt--;
+        int lt = (int)v.size() - 1;              // (the coarsest level, 5^3 points a block at most, always fits)
+        while (lt > 1 && (int)v.size() - (lt - 1) <= MGC_LEVELS && fits(lt - 1)) lt--;
         sub_first[qs] = lt;
         sub_smem[qs] = smem(lt);
     }

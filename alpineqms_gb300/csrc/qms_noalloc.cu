@@ -20,10 +20,10 @@
 #include <cmath>
 #include <mutex>
 
-// Scratch: at most QMS_NOALLOC_MAX_BLOCKS operator CTAs (tiles of 32 x 8 x 16
-// nodes; 512 x 512 x 256 cells needs 18,785), four partial sums each, plus one
-// material table.  Every GPU that loads the library holds these ~1.1 MB until
-// the process exits.
+// Scratch: at most QMS_NOALLOC_MAX_BLOCKS operator CTAs (tiles of 32 x 8 x g.okb
+// nodes, 16 planes on large grids and down to 2 on small ones; 512 x 512 x 256
+// cells needs 18,785), four partial sums each, plus one material table.  Every
+// GPU that loads the library holds these ~1.1 MB until the process exits.
 #define QMS_NOALLOC_MAX_BLOCKS 32768
 static __device__ __align__(256) double g_na_partials[4 * QMS_NOALLOC_MAX_BLOCKS];
 static __device__ __align__(256) QMatTable<double> g_na_table;

@@ -8,11 +8,11 @@
 //       stop when ||r|| <= tol * ||x||
 //       e ~= (D^-1 M)^-1 r / ||r||               inner Krylov in T (FP32 = mixed, FP64 = plain)
 //       x += ||r|| e                             FP64 accumulation
-// Inner Krylov: PCG (Jacobi) for the symmetric steady magnetostatic problem
-// (v = 0, V block identically zero), BiCGSTAB on the row-scaled operator for
-// every nonsymmetric system.  All Krylov scalars (alpha, beta, omega, rho)
-// live in device memory and are formed by one-block finalize kernels from
-// deterministic block partial sums, so the vector kernels never wait for the
+// Inner Krylov: PCG for the symmetric steady magnetostatic problem (v = 0, V
+// block identically zero), FGMRES (or BiCGSTAB) on the row-scaled operator for
+// every nonsymmetric system.  All Krylov scalars live in device memory and are
+// formed from deterministic block partial sums by one-block finalize kernels or
+// by the last block of a launch, so the vector kernels never wait for the
 // host; the host only reads the residual estimate to decide when to stop.
 #include "qms_internal.h"
 #include "qms_solver.h"
@@ -322,9 +322,6 @@ __global__ void __launch_bounds__(256) qk_cg_ep(long long n, const T* z, T* p, T
 #define GM_PASS 32
 struct GmPtrs { const void* p[GM_MAXM + 1]; };
 
-// block partials of V_i . w for i = 0..NV-1 (classical Gram-Schmidt projections).
-// NV is a compile-time count so every load of the unrolled loop is unconditional
-// and independent (memory-level parallelism over all basis vectors).
 // True in every thread of the block that arrives last (its threads then see what the others wrote
 // before); the counter is zero again for the next launch.
 __device__ __forceinline__ bool gm_last_block(unsigned* counter) {
@@ -340,6 +337,8 @@ __device__ __forceinline__ bool gm_last_block(unsigned* counter) {
     return last;
 }
 
+// Classical Gram-Schmidt projections.  NV is a compile-time count so every load of the unrolled loop is
+// unconditional and independent (memory-level parallelism over all basis vectors).
 // h_ij = V_i . w for i < NV, and w . w, as block partials (row i of `part`, rows of gridDim.x); in
 // the last pass over the basis (final) the last block adds them up in a fixed order into column j
 // of H and forms the norm of the orthogonalised w from Pythagoras, |w'|^2 = |w|^2 - sum_i h_ij^2:

@@ -6,8 +6,8 @@ step count -- everything ``inputs.txt`` + ``geom.bin`` carry for the reference
 program (3D/master.py:16-77).  The server
 
 * admits requests in arrival order while the HBM budget and the slot limit
-  allow, charging each its exact device footprint (``qms_device_bytes``:
-  solution, multigrid hierarchy, Krylov workspace);
+  allow, charging each its device footprint (``qms_device_bytes``: solution,
+  multigrid hierarchy, Krylov workspace);
 * keeps every admitted solve resident in HBM (its own qms_handle) and advances
   all resident solves concurrently: each runs on its own CUDA stream, driven
   by its own host thread (the ctypes calls release the GIL), so their kernels

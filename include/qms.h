@@ -80,7 +80,8 @@ typedef struct {
     double tol;              /* stop when ||D^-1 (b - M x)|| <= tol * ||x|| */
     int max_outer;           /* refinement iterations */
     int max_inner;           /* Krylov iterations per refinement iteration */
-    double inner_rtol;       /* relative reduction asked of each inner solve */
+    double inner_rtol;       /* relative reduction asked of each inner solve; with use_graphs the most that one
+                                FGMRES cycle aims at */
     int check_every;         /* inner iterations between host convergence checks */
     int device;              /* CUDA device ordinal */
     int precond;             /* QMS_PRECOND_MG (default) or QMS_PRECOND_JACOBI */
@@ -92,9 +93,9 @@ typedef struct {
                                 potential of isolated conductors) */
     int krylov;              /* nonsymmetric inner solver: QMS_KRYLOV_GMRES (default) or _BICGSTAB */
     int gmres_m;             /* FGMRES basis size per refinement iteration (<= 64) */
-    int use_graphs;          /* replay the FGMRES steps of a time step from CUDA graphs, and chained
-                                steps whole (1 = on); cycles then end by their residual estimate at
-                                equal shares of the reduction still wanted */
+    int use_graphs;          /* replay the FGMRES steps of a time step from CUDA graphs once they repeat, and
+                                chained steps whole (1 = on); cycles then end by their residual estimate
+                                at equal shares of the reduction still wanted */
     double mg_region_cut;    /* conductor-region coarse space of the potential block: eigenvalues of
                                 its region-stiffness-scaled Galerkin matrix at or below this are
                                 dropped (0 = automatic: 1e-9 with FP64 inner vectors, 1e-6 with FP32;
@@ -151,7 +152,10 @@ typedef struct qms_handle qms_handle;
 
 /* Fills `d` with the defaults for a grid (mixed precision, tol 2e-13). */
 void qms_default_desc(qms_desc* d, int xs, int ys, int zs, double dx, double dy, double dz, double dt);
-/* Device bytes a handle with this descriptor allocates (admission control). */
+/* Device bytes of the arrays that a handle with this descriptor allocates (admission control).  Not in it:
+ * the 2 MiB granules of the allocations (24x20x17 to 128^3: up to 12 MiB or 2 %) and the CUDA graphs of its
+ * runs (measured with a full cache of the longest ones: 24 to 38 MiB, most of it shared with the graphs of
+ * handles before). */
 size_t qms_device_bytes(const qms_desc* d);
 int64_t qms_n_dims(int xs, int ys, int zs);
 int64_t qms_csr_nnz(int xs, int ys, int zs);
@@ -204,7 +208,8 @@ int qms_get_rhs(qms_handle* h, double* b_out);            /* n_dims doubles: the
                                                              step with an unchanged field does not form it,
                                                              and this call then forms it from that step's
                                                              start state */
-int qms_set_state(qms_handle* h, const double* x_in);
+int qms_set_state(qms_handle* h, const double* x_in);    /* starts a run: its results do not depend on what the
+                                                             handle solved before */
 
 /* Verification path: CSR of the steady (transient = 0) or transient system and
  * its RHS, bit-identical to the reference's (F:448-1312 / F:1457-2191).

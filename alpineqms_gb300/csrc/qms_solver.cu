@@ -1837,7 +1837,9 @@ int QmsSolver::solve(bool transient, const double v[3], const double B[3], const
     auto count_for = [&](double steps) {
         const double r0 = stats.initial_residual, goal = desc.tol / 4.0;
         if (!(r0 > goal && rel > 0.0 && r0 > rel)) return 1;
-        return (int)std::ceil(std::log(r0 / goal) / (std::log(r0 / rel) / std::max(1.0, steps)));
+        // (r0 may be an ulp above rel: no reduction to speak of)
+        const double per = std::log(r0 / rel) / std::max(1.0, steps), all = std::log(r0 / goal);
+        return per * GM_MAXM > all ? (int)std::ceil(all / per) : GM_MAXM;
     };
     if (graph_cycles > 0 && rel <= desc.tol) {
         if (gm_ls_floor > 0 && ++gm_ls_floor_age > 4) { gm_ls_floor = 0; gm_ls_floor_age = 0; }

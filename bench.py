@@ -361,9 +361,9 @@ def run_gpu(args):
             run.step()
 
     # -- 3. kernel timings: K more steps with the profile on (CUDA events around every operator,
-    # V-cycle and level-0 A-block sweep, recorded into the replayed graphs; two untimed steps
-    # first capture the graphs that carry them).  The event records cost time of their own, so
-    # this pass is timed apart from the one above and its step time is reported beside it.
+    # V-cycle and level-0 A-block sweep; profiled steps launch every kernel directly, after two
+    # untimed ones).  The event records and launches cost time of their own, so this pass is
+    # timed apart from the one above and its step time is reported beside it.
     run.s.profile_enable(True)
     for _ in range(2):
         run.step()
@@ -372,8 +372,7 @@ def run_gpu(args):
     ext = torch.cuda.ExternalStream(run.s.stream_ptr())
     KP = args.profile_steps if args.profile_steps > 0 else K
     # (a profiler's per-kernel list can capture this range: kernels inside the conditional
-    # nodes of the whole-step graphs cannot be profiled one by one, and this pass runs the
-    # per-cycle graphs instead)
+    # nodes of the whole-step graphs cannot be profiled one by one, and this pass replays no graph)
     torch.cuda.nvtx.range_push("profiled_steps")
     prof_ms, _ = timed_steps(run, KP, ext)
     torch.cuda.nvtx.range_pop()
@@ -457,7 +456,9 @@ def run_gpu(args):
                 "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)"
                 if peak_kind == "measured" else "fallback 6800 GB/s",
-                "traffic": (tr * n_a if tr else None), "launches": klaunch,
+                "traffic": (tr * n_a if tr else None),
+                "traffic_def": "DRAM bytes per A unknown of an ncu capture at 192^3 (profiles/ncu_traffic.json) x n_A",
+                "launches": klaunch,
                 "avg_launch_us": 1e3 * kms / max(klaunch, 1),
                 "algorithmic_bytes_per_launch": kbytes / max(klaunch, 1),
                 "algorithmic_bytes_def": "3 p n_A + cells (x and b read, x written; one material byte per cell)",
